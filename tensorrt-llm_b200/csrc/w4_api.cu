@@ -196,11 +196,79 @@ int auto_regime(int m, int n, int k, int group_size, int weight_bits, int act_dt
     return f != W4_REGIME_AUTO ? f : w4_gemm_select_regime_typed(m, n, k, group_size, weight_bits, act_dtype);
 }
 
+// Where the decode regime ends. The regime decides what workspace a caller has to bring, so for a given
+// problem it does not move with every change of a kernel: the model is that of decode passes (16 rows while
+// more than 8 are left, then one for up to 8: 4.2 us plus the weight bytes at 3.4 TB/s; 16 rows 6.3 us plus
+// the bytes at 2.7 TB/s for int4, 3.5 us at 3.2 TB/s for int8, 5.0 us at 3.1 TB/s for int8 under bf16)
+// against tensor-core tiles of 128 columns, 7 us plus waves times the step costs. Which kernel runs inside
+// the regime is decided by decode_takes_tensor_cores() below.
+double regime_decode_us(int m, int n, int k, int weight_bits, int act_dtype)
+{
+    double const weight_mb = double(n) * double(k) * weight_bits / 8.0 / 1.0e6;
+    int passes16 = 0, left = m;
+    while (left > 8)
+    {
+        ++passes16;
+        left -= left < 16 ? left : 16;
+    }
+    double const pass16_us = weight_bits == 8 ? (act_dtype == W4_DTYPE_BF16 ? weight_mb / 3.1 + 5.0 : weight_mb / 3.2 + 3.5)
+                                              : weight_mb / 2.7 + 6.3;
+    return passes16 * pass16_us + (left > 0 ? weight_mb / 3.4 + 4.2 : 0.0);
+}
+
+double regime_prefill_us(int m, int n, int k, int num_sms, int weight_bits)
+{
+    bool const w8 = weight_bits == 8;
+    auto step_us = [&](int bm) { return w8 ? (bm <= 64 ? 0.56 : bm <= 128 ? 0.70 : bm == 192 ? 1.11 : 1.9)
+                                           : (bm <= 128 ? 0.57 : bm == 192 ? 0.70 : 1.05); };
+    auto tiles = [&](int bm) { return long((n + 127) / 128) * long((m + bm - 1) / bm); };
+    auto waves = [&](int bm, long splits) { return double((tiles(bm) * splits + num_sms - 1) / num_sms); };
+    int bm = m <= 64 ? 64 : (m <= 128 ? 128 : 192);
+    if (m > 192 || (w8 && m > 128))
+    {
+        bm = 128;
+        for (int const c : {192, 256})
+            if (waves(c, 1) * step_us(c) < waves(bm, 1) * step_us(bm))
+                bm = c;
+    }
+    long const steps = (k + 127) / 128;
+    long splits = 1;
+    if (tiles(bm) * 2 <= num_sms && m <= 256)
+    {
+        splits = num_sms / tiles(bm);
+        splits = splits > steps / 4 ? steps / 4 : splits;
+        splits = splits > 16 ? 16 : (splits < 1 ? 1 : splits);
+    }
+    return 7.0 + (splits > 1 ? 3.0 : 0.0) + waves(bm, splits) * step_us(bm) * double((steps + splits - 1) / splits);
+}
+
+// An automatic launch in the decode regime with more than 8 rows: the tensor-core kernel in the forms that
+// need no workspace, where its estimate is clearly below that of the 16-row passes (4096 x 14336 int4 at 16
+// rows: 12.4 against 17.2 us; at 4096 x 4096 int8 the two are as fast and the decode kernel launches faster).
+bool decode_takes_tensor_cores(W4GemmParams const& p)
+{
+    if (p.m <= 8 || p.act_scale)
+        return false;
+    w4::DeviceInfo const& dev = w4::current_device_info();
+    return dev.num_sms > 0
+        && w4::gemm_tc_plan(p.m, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 1.5
+        < regime_decode_us(p.m, p.n, p.k, p.weight_bits, p.act_dtype);
+}
+
 int resolve_regime(W4GemmParams const& p)
 {
     if (p.regime == W4_REGIME_GEMV || p.regime == W4_REGIME_GEMM)
         return p.regime;
     return auto_regime(p.m, p.n, p.k, p.group_size, p.weight_bits, p.act_dtype);
+}
+
+// Whether the launch runs the decode kernel.
+bool takes_decode_kernel(W4GemmParams const& p)
+{
+    if (resolve_regime(p) != W4_REGIME_GEMV)
+        return false;
+    bool const chosen = p.regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO;
+    return !(chosen && decode_takes_tensor_cores(p));
 }
 
 void log_refusal(char const* entry, W4GemmParams const* p, int rc)
@@ -291,32 +359,11 @@ extern "C"
         (void) group_size;
         if (m <= 8)
             return W4_REGIME_GEMV; // one pass over the weights
-        // Cost model fitted to measurements on B200 (microseconds). The decode kernel passes over the
-        // packed weights once per 16 rows while more than 8 rows are left, then once for up to 8:
-        // an 8-row pass costs 4.2 us plus the weight bytes at 3.4 TB/s (config 2: 12.1 us; 4096 x 4096
-        // int4: 6.6 us), a 16-row pass 6.3 us plus the bytes at 2.7 TB/s for int4 (config 2: 17.2 us;
-        // 4096 x 1024: 6.8 us) and 3.5 us plus the bytes at 3.2 TB/s for int8, whose narrower units let
-        // a 16-row tile cover as much k as an 8-row one (4096 x 4096: 7.8 us; 4096 x 14336: 20-23 us);
-        // bf16 activations with int8 weights need two mma planes per byte: 5.0 us plus the bytes at
-        // 3.1 TB/s (4096 x 1024: 6.4 us; 4096 x 4096: 9.6 us; 4096 x 14336: 23.6 us).
-        // The tensor-core kernel's
-        // estimate comes from its own per-step costs. The SM count is the current device's (148 when
-        // no device is present).
         w4::DeviceInfo const& dev = w4::current_device_info();
-        int const sms = dev.num_sms > 0 ? dev.num_sms : 148;
-        double const weight_mb = double(n) * double(k) * weight_bits / 8.0 / 1.0e6;
-        int passes16 = 0, left = m;
-        while (left > 8)
-        {
-            ++passes16;
-            left -= left < 16 ? left : 16;
-        }
-        double const pass16_us = weight_bits == 8
-            ? (act_dtype == W4_DTYPE_BF16 ? weight_mb / 3.1 + 5.0 : weight_mb / 3.2 + 3.5)
-            : weight_mb / 2.7 + 6.3;
-        double const gemv_us = passes16 * pass16_us + (left > 0 ? weight_mb / 3.4 + 4.2 : 0.0);
-        double const gemm_us = w4::gemm_tc_estimate_us(m, n, k, sms, weight_bits);
-        return gemv_us <= gemm_us ? W4_REGIME_GEMV : W4_REGIME_GEMM;
+        int const sms = dev.num_sms > 0 ? dev.num_sms : 148; // 148 when no device is present
+        return regime_decode_us(m, n, k, weight_bits, act_dtype) <= regime_prefill_us(m, n, k, sms, weight_bits)
+            ? W4_REGIME_GEMV
+            : W4_REGIME_GEMM;
     }
 
     size_t w4_gemm_workspace_bytes(int m, int n, int k, int group_size, int weight_bits, int act_dtype,
@@ -329,7 +376,7 @@ extern "C"
             r = auto_regime(m, n, k, group_size, weight_bits, act_dtype);
         if (r == W4_REGIME_GEMV)
             return 0;
-        return w4::gemm_tc_workspace_bytes(m, n, k, has_act_scale, weight_bits);
+        return w4::gemm_tc_workspace_bytes(m, n, k, has_act_scale, weight_bits, act_dtype);
     }
 
     size_t w4_gemm_workspace_bytes_max(int max_m, int n, int k, int group_size, int weight_bits, int act_dtype,
@@ -373,7 +420,7 @@ extern "C"
         if (p->m == 0)
             return W4_OK;
         cudaStream_t const s = static_cast<cudaStream_t>(stream);
-        bool const gemv = resolve_regime(*p) == W4_REGIME_GEMV;
+        bool const gemv = takes_decode_kernel(*p);
         if (log_level() <= W4_LOG_DEBUG)
             log_line(W4_LOG_DEBUG, "w4_gemm_launch m=%d n=%d k=%d bits=%d group=%d zeros=%d bias=%d act_scale=%d alpha=%g %s%s",
                 p->m, p->n, p->k, p->weight_bits, p->group_size, p->zeros != nullptr, p->bias != nullptr,
@@ -509,7 +556,7 @@ extern "C"
         W4GemmParams q = *p;
         if (out_dev)
             q.out = out_dev;
-        int const lrc = resolve_regime(q) == W4_REGIME_GEMV ? w4::launch_gemv(q, s) : w4::launch_gemm_tc(q, s);
+        int const lrc = takes_decode_kernel(q) ? w4::launch_gemv(q, s) : w4::launch_gemm_tc(q, s);
         if (lrc != W4_OK)
             return lrc;
         if (!out_dev && cudaMemcpyAsync(host_out, p->out, out_bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)

@@ -197,6 +197,10 @@ struct Pair<__half>
     {
         return __half_as_ushort(__float2half_rn(f));
     }
+    static __device__ __forceinline__ uint32_t pack2(float lo, float hi)
+    {
+        return bits(__floats2half2_rn(lo, hi));
+    }
     // Both halves of a packed pair as floats (low half first).
     static __device__ __forceinline__ void unpack2(uint32_t v, float& lo, float& hi)
     {
@@ -250,6 +254,10 @@ struct Pair<__nv_bfloat16>
     static __device__ __forceinline__ uint16_t from_float(float f)
     {
         return __bfloat16_as_ushort(__float2bfloat16_rn(f));
+    }
+    static __device__ __forceinline__ uint32_t pack2(float lo, float hi)
+    {
+        return bits(__floats2bfloat162_rn(lo, hi));
     }
     // Both halves of a packed pair as floats (low half first): two integer ops.
     static __device__ __forceinline__ void unpack2(uint32_t v, float& lo, float& hi)

@@ -9,29 +9,34 @@
 //
 // Orientation. The output tile is computed transposed: D[n, m] = sum_k W[n, k] * A[m, k]. The
 // dequantised weights are the MMA's "A" operand and live in tensor memory (one TMEM lane per
-// output column n, 128 per tile), written there straight from registers by the conversion warps,
-// so they never travel through shared memory; the activations are the "B" operand, brought by TMA
-// into 128-byte-swizzled shared memory and consumed by the MMA unmodified. One tile is 128 columns
-// of W times 64..256 rows of the activation matrix; a pipeline step covers 128 k (two 64-wide
-// swizzled halves, eight tcgen05.mma of K = 16).
+// output column n), written there straight from registers by the conversion warps, so they never
+// travel through shared memory; the activations are the "B" operand, brought by TMA into
+// 128-byte-swizzled shared memory and consumed by the MMA unmodified.
 //
-// Warp roles (320 threads, one CTA per SM, persistent over tiles, n-fastest tile order):
-//   warp 0      TMA producer: two activation half-tiles [BM x 64] + the packed weight lines per step
-//   warp 1      allocates TMEM, issues tcgen05.mma and tcgen05.commit (whole warp, warp-uniform
-//               operands, one elected lane per instruction)
-//   warps 2..9  conversion, two warps per TMEM lane quadrant taking alternate k steps: shared memory
-//               -> registers -> exact int->T conversion, scale/zero -> tcgen05.st into the TMEM ring
-//               of A stages; after the last k step the same warps run the epilogue (tcgen05.ld,
-//               alpha/bias, convert, store), each on its share of the accumulator columns.
-// Hand-offs: `full` (TMA -> conversion), per-warp step counters polled with acquire loads
-// (conversion -> MMA), `done` (tcgen05.commit -> producer and conversion: the shared-memory stage
-// and the TMEM stage of a step are released together), `d_full` / `d_empty` (accumulator).
-// What was measured while tuning (B200): the pipeline has a cost per k step of roughly 900-1100
-// cycles that does not depend on the row tile, so the step is made as fat as shared memory allows
-// (128 k); issuing tcgen05.mma from a divergent single lane costs ~70 cycles per instruction
-// against ~40 from a converged warp; scale/zero loads need several groups of lookahead because a
-// step is shorter than an L2 round trip.
-// All waits are bounded; a timeout sets the device status word and the CTA drains and exits.
+// A CTA pair (cluster of two, cta_group::2) owns a tile of 256 weight columns x BM activation rows,
+// BM a multiple of 32 up to 256 chosen per problem: each CTA converts its own 128 columns and holds
+// half of the activation rows, which the pair's MMAs read from both shared memories. That halves the
+// activation bytes a CTA has to pull out of L2 (at 256 rows 20 KB of operands per 64 k and 512
+// tensor cycles instead of 36 KB, which alone would exceed what L2 delivers to all SMs) and leaves
+// room for deep rings.
+//
+// Warp roles (one CTA pair per two SMs, persistent over tiles, n-fastest tile order):
+//   warps 0..3            epilogue: tcgen05.ld, alpha/bias, convert, store; the accumulator is double
+//                         buffered up to 128 rows
+//   warps 4..4+4G-1       conversion, G groups of four warps (one per TMEM lane quadrant) that take
+//                         alternate steps: shared memory -> registers -> exact int->T
+//                         conversion, scale/zero -> tcgen05.st into the TMEM ring
+//   next                  weight producer: packed weights and their scale/zero rows, one TMA box each
+//                         per step, a ring of its own that runs far ahead (its latency is
+//                         HBM's) and, with static weights, ahead of the preceding kernel
+//   next                  activation producer: two boxes of 64 k x BM/2 rows per step
+//   last                  MMA issuer (first CTA of the pair) and TMEM alloc/free (both)
+// A step is 128 k (eight tcgen05.mma of K = 16). Hand-offs, all mbarriers: `w_full` / `w_empty` (weight
+// ring, local), `full` (first CTA: both CTAs' halves of the step's activations landed and the eight
+// conversion warps of both CTAs stored their part of the step's weights), `empty` (tcgen05.commit,
+// multicast to both CTAs: the step's activation stage and TMEM stage are free), `d_full` /
+// `d_empty` (accumulator).
+// All waits are bounded; a timeout sets the device status word and the CTAs drain and exit.
 #include <mutex>
 #include <type_traits>
 
@@ -44,77 +49,132 @@ namespace w4
 namespace tc
 {
 
-constexpr int BN = 128;       // weight columns per tile (MMA M, TMEM lanes)
-constexpr int BK = 128;       // k per pipeline step: two 64-wide halves (one 128-byte swizzle span of T each)
-constexpr int kHalves = BK / 64;
-constexpr int kMaxAStages = 4; // TMEM ring of converted-weight stages (64 columns each): columns 256..511
-constexpr int kACol0 = 256;   // first TMEM column of that ring; the accumulator uses [0, 256)
+constexpr int BN = 128;            // weight columns per CTA (TMEM lanes)
+constexpr int kPairN = 2 * BN;     // weight columns per CTA pair
+constexpr int kMaxBM = 256;        // activation rows per tile at most
 constexpr int kTmemCols = 512;
-constexpr int kConvGroups = 2;   // groups of 4 conversion warps; group g converts k steps with ks % 2 == g
-constexpr int kThreads = 64 + 128 * kConvGroups;
-constexpr int kMaxStages = kMaxAStages; // one ring index for the shared-memory stage and its TMEM stage
+constexpr int kStageCols = 64;     // TMEM columns of one converted 128-k stage
+constexpr int kConvGroups = 3;
+constexpr int kEpiWarps = 4;
+constexpr int kConvWarp0 = kEpiWarps;
+constexpr int kWProdWarp = kConvWarp0 + 4 * kConvGroups;
+constexpr int kActWarp = kWProdWarp + 1;
+constexpr int kMmaWarp = kWProdWarp + 2;
+constexpr int kThreads = 32 * (kWProdWarp + 4);
+constexpr int kMaxStages = 8;      // activation / TMEM ring
+constexpr int kMaxWStages = 12;    // weight ring
 
 struct Args
 {
-    void const* scales;
-    void const* zeros;
     void const* bias;
     void* out;
     float alpha;
     int m, n, k;
     int group_shift; // log2(group size), 31 = per-channel
+    int bm;          // activation rows per tile
     int tiles_n, tiles_m;
-    int num_stages;
-    // Split-k: an output tile's k range is cut into `splits` work items that run on different SMs;
-    // each stores its fp32 partial tile and a second small kernel adds them in split order.
+    int num_stages, num_wstages;
+    int d_bufs;      // accumulators in TMEM: 2 up to 128 rows, else 1
+    int weights_static;
+    // Split-k: an output tile's k range is cut into `splits` work items that run on different CTA pairs.
     int splits;       // 1 = off
-    int ksteps_split; // k steps per work item
-    float* partial;   // [splits, m, n] fp32 (workspace)
+    int steps_split;  // 128-wide k steps per work item
+    float* partial;   // [splits, m, n] fp32 (SPLIT_WORKSPACE)
 };
+
+// Where the fp32 partial tiles of a split tile meet. CLUSTER: the splits' CTA pairs form one cluster of
+// 2 * splits CTAs, every CTA leaves its partial tile in its own shared memory and adds a share of the rows
+// over all of them through distributed shared memory. WORKSPACE: partial tiles in the caller's workspace,
+// added by a second kernel; for more splits than a cluster can hold, and where the device cannot
+// co-schedule such clusters. Both add in split order (deterministic).
+enum SplitMode
+{
+    SPLIT_NONE,
+    SPLIT_CLUSTER,
+    SPLIT_WORKSPACE
+};
+constexpr int kMaxClusterSplits = 8; // clusters of 16 CTAs
 
 struct __align__(16) Barriers
 {
-    // TMA landed (tx bytes), one barrier per (conversion group, stage): the copy of a k step signals the
-    // barrier of the group that converts that step. A group therefore sees every phase of every
-    // barrier it waits on, whatever the number of stages and of k steps per tile (with one barrier
-    // per stage a group would meet a subset of the phases and could take a lagging copy of the other
-    // group's step for its own).
-    uint64_t full[kConvGroups][kMaxStages];
-    uint64_t done[kMaxStages];    // the MMAs of the step completed: smem stage and TMEM stage are free
-    uint64_t d_full;              // accumulator complete
-    uint64_t d_empty;             // the epilogue warps drained the accumulator
-    // Steps each conversion warp has finished storing into TMEM, [group][quadrant]. The MMA warp
-    // polls these with plain acquire loads: an mbarrier test issued by the MMA warp right after its
-    // tcgen05.commit is held back until the committed MMAs finish, which costs a full step.
-    alignas(16) uint32_t ready[kConvGroups][4];
+    uint64_t full[kMaxStages];    // first CTA: activations of both CTAs landed, 8 conversion warps stored
+    uint64_t empty[kMaxStages];   // the MMAs of the step completed: activation stage and TMEM stage are free
+    // Weights of a step landed, one barrier per (conversion group, stage): copies land out of order, and a
+    // group that met only some of a stage's phases could take the parity of an older phase for its own.
+    // (The `empty` phases come from commits, which complete in order.)
+    uint64_t w_full[kConvGroups][kMaxWStages];
+    uint64_t w_empty[kMaxWStages];
+    uint64_t d_full[2];           // accumulator complete
+    uint64_t d_empty[2];          // first CTA: the epilogue warps of both CTAs drained the accumulator
     uint32_t tmem_base;
     int abort_flag;
 };
 
-
-__device__ __forceinline__ bool wait_flag(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
+// Bounded wait on an mbarrier phase, executed by a converged warp (every lane polls the same word).
+// CLUSTER: the phase was completed by the other CTA's arrivals as well.
+template <bool CLUSTER>
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity)
 {
-    // Spin on the non-blocking test: the blocking try_wait form parks the thread for a
-    // hardware-defined interval, which costs about a microsecond per hand-off in this pipeline.
-    for (uint32_t i = 0; i < kMaxSpinPolls; ++i)
-    {
-        if (mbar_test_wait(bar, parity))
-            return true;
-        if ((i & 1023u) == 1023u && *abort_flag)
-            return false;
-    }
-    *abort_flag = 1;
-    atomicExch(&g_device_status, kDeviceTimeout);
-    return false;
+    uint32_t ok;
+    if (CLUSTER)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    return __all_sync(0xffffffffu, ok) != 0; // warp-uniform: the code behind a wait is executed converged
 }
 
-// Warp-wide wait: one lane polls, the result is broadcast (keeps 31 lanes off the barrier word).
-__device__ __forceinline__ bool wait_flag_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int lane)
+template <bool CLUSTER>
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
-    int ok = 1;
-    if (lane == 0)
-        ok = wait_flag(bar, parity, abort_flag) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    for (uint32_t polls = 1; !mbar_poll<CLUSTER>(bar, parity); ++polls)
+    {
+        if ((polls & 1023u) == 0 && (*abort_flag || polls >= kMaxWaitPolls))
+        {
+            *abort_flag = 1;
+            atomicExch(&g_device_status, kDeviceTimeout);
+            return false;
+        }
+    }
+    return true;
+}
+
+// Address of this CTA's shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void cluster_sync_all()
+{
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before()
@@ -127,27 +187,10 @@ __device__ __forceinline__ void tc_fence_after()
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-__device__ __forceinline__ bool mbar_test_wait_addr(uint32_t bar_addr, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar_addr), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-
 // The following are executed by a whole (converged) warp; one elected lane performs the operation.
 // Keeping the surrounding control flow warp-uniform lets the compiler hold addresses and
 // descriptors in uniform registers, which is what the tensor-core and TMA instructions consume;
-// issued from inside a divergent `if (lane == 0)` every operand has to be moved across first and
-// one tcgen05.mma costs ~70 cycles to issue.
+// issued from inside a divergent `if (lane == 0)` every operand has to be moved across first.
 __device__ __forceinline__ void tc_mma_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc)
 {
     asm volatile(
@@ -155,69 +198,76 @@ __device__ __forceinline__ void tc_mma_ts_elect(uint32_t d_tmem, uint32_t a_tmem
         ".reg .pred p, pe;\n"
         "elect.sync _|pe, 0xffffffff;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
         "}\n" ::"r"(d_tmem),
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
         : "memory");
 }
 
-__device__ __forceinline__ void tc_commit_elect(uint32_t bar_addr)
+// Arrives on the barrier at this offset in both CTAs of the pair (`mask`: their ranks in the cluster) once
+// all MMAs issued so far have completed.
+__device__ __forceinline__ void tc_commit_pair_elect(uint32_t bar_addr, uint16_t mask)
 {
     asm volatile(
         "{\n"
         ".reg .pred pe;\n"
         "elect.sync _|pe, 0xffffffff;\n"
-        "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-        "}\n" ::"r"(bar_addr)
+        "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+        "}\n" ::"r"(bar_addr),
+        "h"(mask)
         : "memory");
 }
 
-// Warp-uniform bounded spin on an mbarrier phase (every lane polls the same word).
-__device__ __forceinline__ bool spin_wait(uint32_t bar_addr, uint32_t parity, volatile int* abort_flag)
-{
-    uint32_t polls = 0;
-    while (!mbar_test_wait_addr(bar_addr, parity))
-    {
-        if ((++polls & 0xffffu) == 0 && (*abort_flag || polls >= kMaxSpinPolls))
-        {
-            *abort_flag = 1;
-            atomicExch(&g_device_status, kDeviceTimeout);
-            return false;
-        }
-    }
-    return true;
-}
-
-// Spins until all four conversion warps of a group have published at least `needed` steps.
-__device__ __forceinline__ bool spin_ready(uint32_t addr, uint32_t needed, volatile int* abort_flag)
-{
-    uint32_t polls = 0;
-    for (;;)
-    {
-        uint32_t a, b, c, d;
-        asm volatile("ld.acquire.cta.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
-                     : "r"(addr)
-                     : "memory");
-        // counters only grow and stay within a few steps of each other: compare as signed distance
-        if (int(a - needed) >= 0 && int(b - needed) >= 0 && int(c - needed) >= 0 && int(d - needed) >= 0)
-            return true;
-        if ((++polls & 0xffffu) == 0 && (*abort_flag || polls >= kMaxSpinPolls))
-        {
-            *abort_flag = 1;
-            atomicExch(&g_device_status, kDeviceTimeout);
-            return false;
-        }
-    }
-}
-
-__device__ __forceinline__ void tc_st16(uint32_t taddr, uint32_t const (&v)[16])
+// 2-D tile load of this CTA's half of an activation step; completion is counted on `bar_addr`, which
+// is the first CTA's barrier for both.
+__device__ __forceinline__ void elect_tma_load_2d_pair(uint32_t dst, void const* tensor_map, int c0, int c1, uint32_t bar_addr)
 {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
-            taddr),
+        "{\n"
+        ".reg .pred pe;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "@pe cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+        "}\n" ::"r"(dst),
+        "l"(tensor_map), "r"(c0), "r"(c1), "r"(bar_addr)
+        : "memory");
+}
+
+__device__ __forceinline__ void elect_tma_load_3d(uint32_t dst, void const* tensor_map, int c0, int c1, int c2, uint32_t bar_addr)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred pe;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "@pe cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
+        "}\n" ::"r"(dst),
+        "l"(tensor_map), "r"(c0), "r"(c1), "r"(c2), "r"(bar_addr)
+        : "memory");
+}
+
+__device__ __forceinline__ void arrive_local(uint32_t bar_addr)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
+}
+
+// Publishes tensor-memory accesses (ordered by tcgen05.wait and tcgen05.fence::before_thread_sync in
+// front of it) to the first CTA's MMA warp. Relaxed: with release semantics every arrival waits for a
+// cluster-scope fence, about half a microsecond that the conversion warp spends idle (the kernel took
+// 0.33 us per 64 k instead of 0.17).
+__device__ __forceinline__ void arrive_cluster_relaxed(uint32_t addr)
+{
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+__device__ __forceinline__ void tc_st32(uint32_t taddr, uint32_t const (&v)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
+        "%30,%31,%32};" ::"r"(taddr),
         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
 }
 
@@ -247,439 +297,510 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr)
     return d;
 }
 
-template <typename T, int BITS, int BM, bool HAS_ZERO, bool SPLITK>
+
+template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
-    gemm_kernel(Args const a, __grid_constant__ CUtensorMap const tm_act, __grid_constant__ CUtensorMap const tm_w)
+    gemm_kernel(Args const a, __grid_constant__ CUtensorMap const tm_act, __grid_constant__ CUtensorMap const tm_w,
+        __grid_constant__ CUtensorMap const tm_s, __grid_constant__ CUtensorMap const tm_z)
 {
     using P = Pair<T>;
     constexpr int IL = BITS == 4 ? 4 : 2;
-    constexpr int ACT_HALF = BM * 128;                      // BM rows x 64 k of T (one swizzled tile)
-    constexpr int ACT_BYTES = kHalves * ACT_HALF;
-    constexpr int W_BYTES = (BN / IL) * 128 * kHalves;      // interleaved rows x two adjacent 128-byte lines
-    constexpr int STAGE_BYTES = ACT_BYTES + W_BYTES;
-    constexpr int SEG = 128 / IL;                // bytes of one column inside a line
+    constexpr int SEG_CHUNKS = 8 / IL;               // 16-byte chunks of one column inside a 128-byte line (64 k)
+    constexpr int LINE_TILE = (BN / IL) * 128;       // this CTA's interleaved rows x one line
+    constexpr int W_BYTES = 2 * LINE_TILE;           // a step: two lines per row
+    constexpr int W_STAGE = W_BYTES + 1024;          // + up to two rows of 128 scales, and of zeros
     constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u; // 0 = fp16, 1 = bf16
-    constexpr uint32_t kIdesc = (1u << 4)                                   // fp32 accumulator
-        | (kFmt << 7)                                                       // A type
-        | (kFmt << 10)                                                      // B type (both K-major)
-        | (uint32_t(BM >> 3) << 17)                                         // MMA N = activation rows
-        | (uint32_t(BN >> 4) << 24);                                        // MMA M = weight columns
 
     // The 128-byte swizzle of the TMA copies and of the MMA descriptors is a function of the
-    // shared-memory address: the ring starts on a 1024-byte boundary (declared, and checked below).
+    // shared-memory address: the rings start on a 1024-byte boundary (declared, and checked below).
     extern __shared__ __align__(1024) uint8_t smem[];
-    if ((smem_u32(smem) & 1023u) != 0) // never seen; nothing has been allocated or initialised yet
-    {
-        if (threadIdx.x == 0)
-            atomicExch(&g_device_status, kDeviceTimeout);
-        return;
-    }
-    Barriers* bars = reinterpret_cast<Barriers*>(smem + size_t(a.num_stages) * STAGE_BYTES);
+    uint32_t const smem_base = smem_u32(smem);
+    int const act_half = a.bm * 64;       // bm / 2 rows of 128 bytes: 64 k
+    int const act_stage = 2 * act_half;
+    uint32_t const w_ring = smem_base + uint32_t(a.num_stages) * act_stage;
+    Barriers* bars = reinterpret_cast<Barriers*>(smem + size_t(a.num_stages) * act_stage + size_t(a.num_wstages) * W_STAGE);
     volatile int* abort_flag = &bars->abort_flag;
 
-    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int const num_tiles = a.tiles_n * a.tiles_m * (SPLITK ? a.splits : 1); // work items: (tile, split), splits adjacent
-    int const ksteps_all = (a.k + BK - 1) / BK; // a trailing 64-wide half reads as zeros (TMA fill)
+    int const warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    uint32_t cta_rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
+    uint32_t const rank = cta_rank & 1u, lead_rank = cta_rank & ~1u; // in the pair; the pair's first CTA
+    // Work items: (tile, split), splits adjacent. With SPLIT_CLUSTER a pair has exactly one: the grid is one
+    // cluster per tile and a pair's rank in it is its split.
+    int const pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+    int const num_items = a.tiles_n * a.tiles_m * (SPLIT != SPLIT_NONE ? a.splits : 1);
+    int const steps_all = (a.k + 127) >> 7; // the second half of the last step may lie past k: zeros, not multiplied
 
+    bool const aligned = (smem_base & 1023u) == 0; // never false; the check keeps a wrong layout from being read
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < a.num_stages; ++s)
         {
-            for (int g = 0; g < kConvGroups; ++g)
-                mbar_init(&bars->full[g][s], 1);
-            mbar_init(&bars->done[s], 1);
+            mbar_init(&bars->full[s], 1 + 8); // expect_tx of the first CTA + four conversion warps of each CTA
+            mbar_init(&bars->empty[s], 1);
         }
-        mbar_init(&bars->d_full, 1);
-        mbar_init(&bars->d_empty, 4 * kConvGroups);
-        bars->abort_flag = 0;
-        for (int i = 0; i < kConvGroups * 4; ++i)
-            (&bars->ready[0][0])[i] = 0;
+        for (int s = 0; s < a.num_wstages; ++s)
+        {
+            for (int g = 0; g < kConvGroups; ++g)
+                mbar_init(&bars->w_full[g][s], 1);
+            mbar_init(&bars->w_empty[s], 4);
+        }
+        for (int b = 0; b < 2; ++b)
+        {
+            mbar_init(&bars->d_full[b], 1);
+            mbar_init(&bars->d_empty[b], 2 * kEpiWarps);
+        }
+        bars->abort_flag = aligned ? 0 : 1;
+        if (!aligned)
+            atomicExch(&g_device_status, kDeviceTimeout);
         mbar_fence_init();
     }
-    if (warp == 1)
+    if (warp == kMmaWarp)
     {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&bars->tmem_base)),
                      "r"(uint32_t(kTmemCols))
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync_all(); // the barriers of both CTAs are initialised before either arrives on the other's
     tc_fence_after();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t const tmem = bars->tmem_base;
+    uint32_t const a_ring = tmem + uint32_t(a.d_bufs * a.bm); // TMEM ring of converted weights, behind the accumulators
 
-    if (warp == 0)
+    uint32_t const full0 = smem_u32(&bars->full[0]), empty0 = smem_u32(&bars->empty[0]);
+    uint32_t const w_full0 = smem_u32(&bars->w_full[0][0]), w_empty0 = smem_u32(&bars->w_empty[0]);
+
+    // k range of a work item, in steps
+    auto item_range = [&](int item, int& tile, int& split, int& st0, int& st1)
     {
-        // ------------------------------------------------------------------ TMA producer
-        // (whole warp, warp-uniform; an elected lane issues the copies)
+        tile = SPLIT != SPLIT_NONE ? item / a.splits : item;
+        split = SPLIT != SPLIT_NONE ? item - tile * a.splits : 0;
+        st0 = split * a.steps_split;
+        st1 = SPLIT != SPLIT_NONE ? min(steps_all, st0 + a.steps_split) : steps_all;
+    };
+
+    if (!aligned)
+    {
+        // nothing: fall through to the teardown
+    }
+    else if (warp == kWProdWarp)
+    {
+        // ------------------------------------------------------------------ weight producer
         if (lane == 0)
         {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_act) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_s) : "memory");
+            if (HAS_ZERO)
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_z) : "memory");
         }
         __syncwarp();
+        // Weights that the preceding kernel may still be writing must not be fetched early.
+        if (!a.weights_static)
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t const scale_bytes = a.group_shift == 6 ? 512u : 256u;
+        uint32_t const tx = W_BYTES + scale_bytes * (HAS_ZERO ? 2 : 1);
+        int s = 0, turn = 0; // turn: the group that converts the step
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int item = pair; item < num_items && ok; item += num_pairs)
         {
+            int tile, split, st0, st1;
+            item_range(item, tile, split, st0, st1);
+            int const n0 = (tile % a.tiles_n) * kPairN + int(rank) * BN;
+            for (int st = st0; st < st1; ++st)
+            {
+                ok = wait_bar<false>(w_empty0 + 8 * s, ph ^ 1, abort_flag);
+                if (!ok)
+                    break;
+                uint32_t const dst = w_ring + uint32_t(s) * W_STAGE, bar = w_full0 + 8 * (turn * kMaxWStages + s);
+                int const g = a.group_shift >= 31 ? 0 : (st << 7) >> a.group_shift;
+                elect_expect_tx(bar, tx);
+                elect_tma_load_3d(dst, &tm_w, 0, n0 / IL, 2 * st, bar);
+                elect_tma_load_2d(dst + W_BYTES, &tm_s, n0, g, bar);
+                if (HAS_ZERO)
+                    elect_tma_load_2d(dst + W_BYTES + 512, &tm_z, n0, g, bar);
+                turn = turn + 1 == kConvGroups ? 0 : turn + 1;
+                if (++s == a.num_wstages)
+                {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+    }
+    else if (warp == kActWarp)
+    {
+        // ------------------------------------------------------------------ activation producer
+        if (lane == 0)
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_act) : "memory");
+        __syncwarp();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t const lead_full0 = cluster_addr(full0, lead_rank);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int item = pair; item < num_items && ok; item += num_pairs)
+        {
+            int tile, split, st0, st1;
+            item_range(item, tile, split, st0, st1);
+            int const row0 = (tile / a.tiles_n) * a.bm + int(rank) * (a.bm >> 1);
+            for (int st = st0; st < st1; ++st)
+            {
+                ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
+                if (!ok)
+                    break;
+                uint32_t const dst = smem_base + uint32_t(s) * act_stage, bar = lead_full0 + 8 * s;
+                if (rank == 0)
+                    elect_expect_tx(full0 + 8 * s, uint32_t(a.bm) * 256u); // both CTAs' rows
+                elect_tma_load_2d_pair(dst, &tm_act, st * 128, row0, bar);
+                elect_tma_load_2d_pair(dst + act_half, &tm_act, st * 128 + 64, row0, bar);
+                if (++s == a.num_stages)
+                {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        // the last commits arrive on this CTA's barriers from the first CTA: stay until they have
+        for (int i = 0; i < a.num_stages && ok; ++i)
+        {
+            ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
+            if (++s == a.num_stages)
+            {
+                s = 0;
+                ph ^= 1;
+            }
+        }
+    }
+    else if (warp == kMmaWarp)
+    {
+        // ------------------------------------------------------------------ MMA issuer
+        if (rank == 0)
+        {
+            uint32_t const idesc = (1u << 4)             // fp32 accumulator
+                | (kFmt << 7) | (kFmt << 10)             // A and B types (both K-major)
+                | (uint32_t(a.bm >> 3) << 17)            // MMA N = activation rows
+                | (uint32_t(kPairN >> 4) << 24);         // MMA M = weight columns of the pair
+            uint64_t const desc0 = smem_desc_sw128(smem_base);
+            uint64_t const desc_stage = uint64_t(act_stage >> 4), desc_half = uint64_t(act_half >> 4); // 16-byte units
+            uint32_t const d_empty0 = smem_u32(&bars->d_empty[0]), d_full0 = smem_u32(&bars->d_full[0]);
+            uint16_t const both = uint16_t(3u << lead_rank);
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            uint32_t const smem_base = smem_u32(smem);
-            uint32_t const full0 = smem_u32(&bars->full[0][0]), done0 = smem_u32(&bars->done[0]);
-            for (int item = blockIdx.x; item < num_tiles && ok; item += gridDim.x)
+            uint32_t dph = 0; // bit b: parity of accumulator b's next drain
+            int db = 0, it = 0;
+            for (int item = pair; item < num_items && ok; item += num_pairs, ++it)
             {
-                int const tile = SPLITK ? item / a.splits : item, split = SPLITK ? item - tile * a.splits : 0;
-                int const tn = tile % a.tiles_n, tm = tile / a.tiles_n;
-                int const ks0 = SPLITK ? split * a.ksteps_split : 0, ks1 = SPLITK ? min(ksteps_all, ks0 + a.ksteps_split) : ksteps_all;
-                for (int ks = ks0; ks < ks1; ++ks)
+                int tile, split, st0, st1;
+                item_range(item, tile, split, st0, st1);
+                if (it >= a.d_bufs)
                 {
-                    ok = spin_wait(done0 + 8 * s, ph ^ 1, abort_flag);
+                    ok = wait_bar<true>(d_empty0 + 8 * db, (dph >> db) & 1u, abort_flag);
                     if (!ok)
                         break;
-                    uint32_t const stage = smem_base + uint32_t(s) * STAGE_BYTES;
-                    uint32_t const full = full0 + 8 * ((uint32_t(ks) % kConvGroups) * kMaxStages + s);
-                    elect_expect_tx(full, STAGE_BYTES);
-                    elect_tma_load_2d(stage, &tm_act, ks * BK, tm * BM, full);
-                    elect_tma_load_2d(stage + ACT_HALF, &tm_act, ks * BK + 64, tm * BM, full);
-                    elect_tma_load_2d(stage + ACT_BYTES, &tm_w, ks * 128 * kHalves, tn * (BN / IL), full);
-                    if (++s == a.num_stages)
-                    {
-                        s = 0;
-                        ph ^= 1;
-                    }
-                }
-            }
-        }
-    }
-    else if (warp == 1)
-    {
-        // ------------------------------------------------------------------ MMA issuer
-        // One thread feeds the tensor core; its queue is only about one instruction deep, so this
-        // loop has to come back with the next MMA within ~100 cycles: descriptors and addresses are
-        // advanced incrementally, there is one wait and one commit per k step, and the wait spins
-        // on the non-blocking test.
-        {
-            uint64_t const desc0 = smem_desc_sw128(smem_u32(smem));
-            constexpr uint64_t kDescStage = uint64_t(STAGE_BYTES >> 4); // address field is in 16-byte units
-            uint32_t const done0 = smem_u32(&bars->done[0]);
-            uint32_t const d_empty = smem_u32(&bars->d_empty), d_full = smem_u32(&bars->d_full);
-            uint64_t desc = desc0;
-            uint32_t a_col = tmem + kACol0;
-            uint32_t done = done0;
-            uint32_t const ready0 = smem_u32(&bars->ready[0][0]);
-            uint32_t issued[kConvGroups] = {}; // k steps issued so far per conversion group, over all tiles
-            int s = 0;
-            uint32_t ph = 0, dph = 0;
-            bool ok = true;
-            for (int item = blockIdx.x, it = 0; item < num_tiles && ok; item += gridDim.x, ++it)
-            {
-                int const tile = SPLITK ? item / a.splits : item, split = SPLITK ? item - tile * a.splits : 0;
-                int const ks0 = SPLITK ? split * a.ksteps_split : 0, ks1 = SPLITK ? min(ksteps_all, ks0 + a.ksteps_split) : ksteps_all;
-                if (it > 0)
-                {
-                    ok = spin_wait(d_empty, dph, abort_flag);
-                    if (!ok)
-                        break;
-                    dph ^= 1;
+                    dph ^= 1u << db;
                     tc_fence_after();
                 }
+                uint32_t const d_tmem = tmem + uint32_t(db * a.bm);
                 uint32_t accumulate = 0;
-                for (int ks = ks0; ks < ks1; ++ks)
+                for (int st = st0; st < st1; ++st)
                 {
-                    // The conversion warps publish a step only after they have seen the stage's TMA
-                    // barrier, so it covers the activations as well.
-                    uint32_t const grp = uint32_t(ks) % kConvGroups; // the group that converts this step
-                    uint32_t const needed = ++issued[grp];
-                    ok = spin_ready(ready0 + 16 * grp, needed, abort_flag);
+                    ok = wait_bar<true>(full0 + 8 * s, ph, abort_flag);
                     if (!ok)
                         break;
                     tc_fence_after();
-                    tc_mma_ts_elect(tmem, a_col, desc, kIdesc, accumulate);
-                    tc_mma_ts_elect(tmem, a_col + 8, desc + 2, kIdesc, 1u);
-                    tc_mma_ts_elect(tmem, a_col + 16, desc + 4, kIdesc, 1u);
-                    tc_mma_ts_elect(tmem, a_col + 24, desc + 6, kIdesc, 1u);
-                    constexpr uint64_t kDescHalf = uint64_t(ACT_HALF >> 4); // second 64-wide half of the step
-                    tc_mma_ts_elect(tmem, a_col + 32, desc + kDescHalf, kIdesc, 1u);
-                    tc_mma_ts_elect(tmem, a_col + 40, desc + kDescHalf + 2, kIdesc, 1u);
-                    tc_mma_ts_elect(tmem, a_col + 48, desc + kDescHalf + 4, kIdesc, 1u);
-                    tc_mma_ts_elect(tmem, a_col + 56, desc + kDescHalf + 6, kIdesc, 1u);
+                    uint64_t const desc = desc0 + uint64_t(s) * desc_stage;
+                    uint32_t const a_col = a_ring + uint32_t(s) * kStageCols;
+                    tc_mma_ts_elect(d_tmem, a_col, desc, idesc, accumulate);
+                    tc_mma_ts_elect(d_tmem, a_col + 8, desc + 2, idesc, 1u);
+                    tc_mma_ts_elect(d_tmem, a_col + 16, desc + 4, idesc, 1u);
+                    tc_mma_ts_elect(d_tmem, a_col + 24, desc + 6, idesc, 1u);
+                    if (st * 128 + 64 < a.k)
+                    {
+                        tc_mma_ts_elect(d_tmem, a_col + 32, desc + desc_half, idesc, 1u);
+                        tc_mma_ts_elect(d_tmem, a_col + 40, desc + desc_half + 2, idesc, 1u);
+                        tc_mma_ts_elect(d_tmem, a_col + 48, desc + desc_half + 4, idesc, 1u);
+                        tc_mma_ts_elect(d_tmem, a_col + 56, desc + desc_half + 6, idesc, 1u);
+                    }
                     accumulate = 1u;
-                    tc_commit_elect(done); // frees the shared-memory stage and the TMEM stage
-                    desc += kDescStage;
-                    a_col += 32 * kHalves;
-                    done += 8;
+                    tc_commit_pair_elect(empty0 + 8 * s, both); // frees the activation stage and the TMEM stage
                     if (++s == a.num_stages)
                     {
                         s = 0;
                         ph ^= 1;
-                        desc = desc0;
-                        a_col = tmem + kACol0;
-                        done = done0;
                     }
                 }
                 if (ok)
-                    tc_commit_elect(d_full);
+                    tc_commit_pair_elect(d_full0 + 8 * db, both);
+                db = db + 1 == a.d_bufs ? 0 : db + 1;
+            }
+            // stay until the other CTA's last arrivals have landed
+            for (int i = 0; i < a.d_bufs && i < it && ok; ++i)
+            {
+                db = db == 0 ? a.d_bufs - 1 : db - 1;
+                ok = wait_bar<true>(d_empty0 + 8 * db, (dph >> db) & 1u, abort_flag);
             }
         }
     }
-    else
+    else if (warp >= kConvWarp0 && warp < kWProdWarp)
     {
-        // ------------------------------------------------------------------ conversion + epilogue
-        int const quad = warp & 3;             // TMEM lane quadrant this warp may touch
-        int const cgroup = (warp - 2) >> 2;    // which k steps this warp converts
-        int const n_local = quad * 32 + lane;  // weight column inside the tile = TMEM lane
-        uint32_t const lane_addr = tmem + (uint32_t(quad * 32) << 16);
-        uint16_t const* scales = static_cast<uint16_t const*>(a.scales);
-        uint16_t const* zeros = static_cast<uint16_t const*>(a.zeros);
-        uint16_t const* bias = static_cast<uint16_t const*>(a.bias);
-        uint16_t* out = static_cast<uint16_t*>(a.out);
-        int const gsh = a.group_shift >= 31 ? 30 : a.group_shift - 6; // log2(64-wide halves per scale group)
-        // Column segment of this thread inside the first of a stage's two weight lines.
-        int const w_off = (n_local / IL) * (128 * kHalves) + (n_local % IL) * SEG;
+        // ------------------------------------------------------------------ conversion
+        int const quad = warp & 3;                     // TMEM lane quadrant this warp may touch
+        int const cgroup = (warp - kConvWarp0) >> 2;   // which k blocks this warp converts
+        int const n_local = quad * 32 + lane;          // weight column inside the CTA's tile = TMEM lane
+        uint32_t const lane_ring = a_ring + (uint32_t(quad * 32) << 16);
+        uint32_t const lead_full0 = cluster_addr(full0, lead_rank);
+        // This thread's 16-byte chunk c of a line sits at w_off ^ (c << 4): the TMA's 128-byte swizzle
+        // exchanges chunk index and row modulo 8, which makes the reads conflict-free.
+        int const w_row = n_local / IL;
+        uint32_t const w_off = uint32_t(w_row * 128 + ((((n_local % IL) * SEG_CHUNKS) ^ (w_row & 7)) << 4));
 
-        int s_item = 0;          // ring position of the current work item's first k step
-        uint32_t ph_item = 0, dph = 0;
-        uint32_t my_steps = 0; // steps this warp has stored into TMEM (published by lane 0)
-        uint32_t full_seen = 0; // bit s: phases of full[cgroup][s] this group has consumed, mod 2
+        int s = 0, ws = 0;
+        uint32_t ph = 0;
+        uint32_t w_seen = 0; // bit ws: parity of this group's next phase on w_full[cgroup][ws]
+        int turn = 0; // which group converts the next step
         bool ok = true;
-        for (int item = blockIdx.x; item < num_tiles && ok; item += gridDim.x)
+        for (int item = pair; item < num_items && ok; item += num_pairs)
         {
-            int const tile = SPLITK ? item / a.splits : item, split = SPLITK ? item - tile * a.splits : 0;
-            int const tn = tile % a.tiles_n, tm = tile / a.tiles_n;
-            int const ks0 = SPLITK ? split * a.ksteps_split : 0, ks1 = SPLITK ? min(ksteps_all, ks0 + a.ksteps_split) : ksteps_all;
-            int const n = tn * BN + n_local;
-            bool const n_ok = n < a.n;
-            // Scale / zero of this thread's column for the steps THIS group converts (every
-            // kConvGroups-th k step), one pair per 64-k half. They come from global memory (L2 at
-            // best, ~1 us under load, longer than a k step), so the pairs of a step are loaded two of
-            // the group's own steps ahead, into one of two register sets that the twice-unrolled loop
-            // below addresses statically. (A shift queue does not work here: shifting it reads the
-            // newest entry one scale group after its load was issued, and with 64-wide groups that
-            // is half a k step - the warp ends up waiting for every load.)
-            int const num_groups = a.group_shift >= 31 ? 1 : (a.k >> a.group_shift);
-            auto load_pairs = [&](int ks, uint32_t(&sp)[kHalves], uint32_t(&zp)[kHalves])
+            int tile, split, st0, st1;
+            item_range(item, tile, split, st0, st1);
+            for (int st = st0; st < st1; ++st)
             {
-#pragma unroll
-                for (int h = 0; h < kHalves; ++h)
+                if (turn == cgroup)
                 {
-                    int const g = (ks * kHalves + h) >> gsh;
-                    uint32_t sv = 0, zv = 0;
-                    if (n_ok && ks < ks1 && g < num_groups)
-                    {
-                        sv = scales[size_t(g) * a.n + n];
-                        if (HAS_ZERO)
-                            zv = zeros[size_t(g) * a.n + n];
-                    }
-                    sp[h] = sv | (sv << 16);
-                    zp[h] = zv | (zv << 16);
-                }
-            };
-            // position of the item's first step in the ring; own steps are reached from it
-            int const first_own = ks0 + ((cgroup - ks0 % kConvGroups + kConvGroups) % kConvGroups);
-            int s = s_item;
-            uint32_t ph = ph_item;
-            auto advance = [&](int steps)
-            {
-                s += steps;
-                while (s >= a.num_stages)
-                {
-                    s -= a.num_stages;
-                    ph ^= 1;
-                }
-            };
-            advance(first_own - ks0);
-            uint32_t sset[2][kHalves], zset[2][kHalves];
-            load_pairs(first_own, sset[0], zset[0]);
-            load_pairs(first_own + kConvGroups, sset[1], zset[1]);
-
-            // One own step: wait for its weights, convert, store into the TMEM stage, publish.
-            auto convert_step = [&](int ks, uint32_t const(&s2h)[kHalves], uint32_t const(&z2h)[kHalves]) -> bool
-            {
-                (void) ks;
-                {
-                    // parity of this group's next phase on the stage's barrier: one bit per stage
-                    uint32_t const fph = (full_seen >> s) & 1u;
-                    full_seen ^= 1u << s;
-                    ok = wait_flag_warp(&bars->full[cgroup][s], fph, abort_flag, lane);
+                    ok = wait_bar<false>(w_full0 + 8 * (cgroup * kMaxWStages + ws), (w_seen >> ws) & 1u, abort_flag);
                     if (!ok)
-                        return false;
-                    uint8_t const* wsm = smem + size_t(s) * STAGE_BYTES + ACT_BYTES + w_off;
-                    constexpr int CHUNKS = SEG / 16; // 16-byte chunks per half: 2 (int4) or 4 (int8)
-                    uint4 raw[kHalves][CHUNKS];
+                        break;
+                    w_seen ^= 1u << ws;
+                    uint8_t const* wst = smem + (w_ring - smem_base) + size_t(ws) * W_STAGE;
+                    uint16_t const* sc = reinterpret_cast<uint16_t const*>(wst + W_BYTES) + n_local;
+                    uint4 raw[2][SEG_CHUNKS];
+                    uint32_t s2[2], z2[2];
 #pragma unroll
-                    for (int h = 0; h < kHalves; ++h)
-#pragma unroll
-                        for (int c = 0; c < CHUNKS; ++c)
-                            raw[h][c] = *reinterpret_cast<uint4 const*>(wsm + h * 128 + c * 16);
-                    // Convert into registers first; only the stores have to wait for the TMEM stage.
-                    // v[2h + x] holds TMEM columns 32h + 16x .. +15 (k = 64h + 32x .. +31).
-                    uint32_t v[2 * kHalves][16];
-#pragma unroll
-                    for (int h = 0; h < kHalves; ++h)
+                    for (int h = 0; h < 2; ++h)
                     {
-                        uint32_t const s2 = s2h[h], z2 = z2h[h];
-                        if (BITS == 4)
+                        int const grow = h && a.group_shift == 6 ? 128 : 0;
+                        s2[h] = sc[grow];
+                        s2[h] = prmt(s2[h], s2[h], 0x1010u);
+                        if (HAS_ZERO)
                         {
+                            z2[h] = sc[grow + 256];
+                            z2[h] = prmt(z2[h], z2[h], 0x1010u);
+                        }
 #pragma unroll
-                            for (int c = 0; c < 2; ++c)
+                        for (int c = 0; c < SEG_CHUNKS; ++c)
+                            raw[h][c] = *reinterpret_cast<uint4 const*>(wst + h * LINE_TILE + (w_off ^ uint32_t(c << 4)));
+                    }
+                    __syncwarp();
+                    if (lane == 0)
+                        arrive_local(w_empty0 + 8 * ws);
+                    uint32_t const a_col = lane_ring + uint32_t(s) * kStageCols;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                    {
+                        uint32_t v[32]; // TMEM columns of the half step: k = 2 * column (+1)
+#pragma unroll
+                        for (int c = 0; c < SEG_CHUNKS; ++c)
+                        {
+                            uint32_t const r[4] = {raw[h][c].x, raw[h][c].y, raw[h][c].z, raw[h][c].w};
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
                             {
-                                uint32_t const r[4] = {raw[h][c].x, raw[h][c].y, raw[h][c].z, raw[h][c].w};
-#pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                {
-                                    uint32_t q[4];
+                                // pair p of register j holds k = 32c + 2j + 8p (+1) (int4), 16c + 2j + 8p (+1) (int8)
+                                constexpr int PAIRS = BITS == 4 ? 4 : 2;
+                                uint32_t q[PAIRS];
+                                if constexpr (BITS == 4)
                                     cvt_int4x8<T>(r[j], q);
+                                else
+                                    cvt_int8x4<T>(r[j], q);
 #pragma unroll
-                                    for (int p = 0; p < 4; ++p) // pair p of register j holds k = 32c + 2j + 8p (+1)
-                                        v[2 * h + c][j + 4 * p] = HAS_ZERO ? P::fma(q[p], s2, z2) : P::mul(q[p], s2);
-                                }
+                                for (int p = 0; p < PAIRS; ++p)
+                                    v[4 * PAIRS * c + j + 4 * p] = HAS_ZERO ? P::fma(q[p], s2[h], z2[h]) : P::mul(q[p], s2[h]);
                             }
                         }
-                        else
+                        if (h == 0)
                         {
-#pragma unroll
-                            for (int x = 0; x < 2; ++x)
-#pragma unroll
-                                for (int cc = 0; cc < 2; ++cc)
-                                {
-                                    uint4 const w = raw[h][(2 * x + cc) % CHUNKS];
-                                    uint32_t const r[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                                    for (int j = 0; j < 4; ++j)
-                                    {
-                                        uint32_t q[2];
-                                        cvt_int8x4<T>(r[j], q);
-#pragma unroll
-                                        for (int p = 0; p < 2; ++p) // pair p of register j holds k = 16(2x+cc) + 2j + 8p (+1)
-                                            v[2 * h + x][8 * cc + j + 4 * p]
-                                                = HAS_ZERO ? P::fma(q[p], s2, z2) : P::mul(q[p], s2);
-                                    }
-                                }
+                            ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
+                            if (!ok)
+                                break;
+                            tc_fence_after();
                         }
+                        tc_st32(a_col + 32 * h, v);
                     }
-                    ok = wait_flag_warp(&bars->done[s], ph ^ 1, abort_flag, lane);
                     if (!ok)
-                        return false;
-                    tc_fence_after();
-                    uint32_t const a_addr = lane_addr + kACol0 + s * (32 * kHalves); // warp-uniform column address
-#pragma unroll
-                    for (int x = 0; x < 2 * kHalves; ++x)
-                        tc_st16(a_addr + 16 * x, v[x]);
+                        break;
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0)
-                    {
-                        ++my_steps;
-                        asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(&bars->ready[cgroup][quad])),
-                                     "r"(my_steps)
-                                     : "memory");
-                    }
+                        arrive_cluster_relaxed(lead_full0 + 8 * s);
                 }
-                return true;
-            };
-
-            for (int ks = first_own; ks < ks1 && ok; ks += 2 * kConvGroups)
-            {
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
+                turn = turn + 1 == kConvGroups ? 0 : turn + 1;
+                ws = ws + 1 == a.num_wstages ? 0 : ws + 1;
+                if (++s == a.num_stages)
                 {
-                    int const kk = ks + u * kConvGroups;
-                    if (kk < ks1 && ok)
-                    {
-                        uint32_t s2h[kHalves], z2h[kHalves];
-#pragma unroll
-                        for (int h = 0; h < kHalves; ++h)
-                        {
-                            s2h[h] = sset[u][h];
-                            z2h[h] = zset[u][h];
-                        }
-                        load_pairs(kk + 2 * kConvGroups, sset[u], zset[u]);
-                        if (convert_step(kk, s2h, z2h))
-                            advance(kConvGroups);
-                    }
+                    s = 0;
+                    ph ^= 1;
                 }
-            }
-            // the next item starts where this one's k range ends
-            s = s_item;
-            ph = ph_item;
-            advance(ks1 - ks0);
-            s_item = s;
-            ph_item = ph;
-            if (!ok)
-                break;
-
-            // ---- epilogue: this thread owns output column n for all BM rows of the tile
-            ok = wait_flag_warp(&bars->d_full, dph, abort_flag, lane);
-            if (!ok)
-                break;
-            dph ^= 1;
-            tc_fence_after();
-            float const bias_f = (bias && n_ok) ? P::to_float(bias[n]) : 0.f;
-            int const m0 = tm * BM;
-            if (!SPLITK)
-            {
-#pragma unroll 1
-                for (int c0 = cgroup * 32; c0 < BM; c0 += 32 * kConvGroups)
-                {
-                    if (m0 + c0 >= a.m)
-                        break; // warp-uniform
-                    uint32_t v[32];
-                    tc_ld32(lane_addr + c0, v);
-                    if (n_ok)
-                    {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                        {
-                            int const mrow = m0 + c0 + j;
-                            if (mrow < a.m)
-                                out[size_t(mrow) * a.n + n]
-                                    = P::from_float(fmaf(a.alpha, __uint_as_float(v[j]), bias_f));
-                        }
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(&bars->d_empty);
-            }
-            else
-            {
-                // Split-k: store the fp32 partial tile; splitk_reduce_kernel, next on the stream,
-                // adds the partial tiles in split order (deterministic) and writes the output.
-                float* part = a.partial + size_t(split) * a.m * a.n;
-#pragma unroll 1
-                for (int c0 = cgroup * 32; c0 < BM; c0 += 32 * kConvGroups)
-                {
-                    if (m0 + c0 >= a.m)
-                        break;
-                    uint32_t v[32];
-                    tc_ld32(lane_addr + c0, v);
-                    if (n_ok)
-                    {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                        {
-                            int const mrow = m0 + c0 + j;
-                            if (mrow < a.m)
-                                __stcg(part + size_t(mrow) * a.n + n, __uint_as_float(v[j]));
-                        }
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(&bars->d_empty);
             }
         }
     }
+    else if (warp < kEpiWarps)
+    {
+        // ------------------------------------------------------------------ epilogue
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t const lane_addr = tmem + (uint32_t(warp * 32) << 16);
+        uint16_t const* bias = static_cast<uint16_t const*>(a.bias);
+        uint32_t const d_full0 = smem_u32(&bars->d_full[0]), lead_d_empty0 = cluster_addr(smem_u32(&bars->d_empty[0]), lead_rank);
+        uint32_t dph = 0;
+        int db = 0;
+        bool ok = true;
+        for (int item = pair; item < num_items && ok; item += num_pairs)
+        {
+            int tile, split, st0, st1;
+            item_range(item, tile, split, st0, st1);
+            int const n = (tile % a.tiles_n) * kPairN + int(rank) * BN + warp * 32 + lane;
+            bool const n_ok = n < a.n; // n is a multiple of 32: uniform over the warp
+            int const m0 = (tile / a.tiles_n) * a.bm;
+            float const bias_f = (SPLIT == SPLIT_NONE && bias && n_ok) ? P::to_float(bias[n]) : 0.f;
+            ok = wait_bar<false>(d_full0 + 8 * db, (dph >> db) & 1u, abort_flag);
+            if (!ok)
+                break;
+            dph ^= 1u << db;
+            tc_fence_after();
+            float* part = SPLIT == SPLIT_WORKSPACE ? a.partial + size_t(split) * a.m * a.n + n : nullptr;
+            // two rows at a time: neighbouring lanes exchange halves, so that the even lane stores columns
+            // n, n + 1 of the first row and the odd lane columns n - 1, n of the second
+            uint16_t* out = static_cast<uint16_t*>(a.out) + (n & ~1);
+            uint32_t const sel = lane & 1 ? 0x3276u : 0x5410u;
+            int const c_end = min(a.bm, a.m - m0);
+#pragma unroll 1
+            for (int c0 = 0; c0 < c_end; c0 += 32)
+            {
+                uint32_t v[32];
+                tc_ld32(lane_addr + uint32_t(db * a.bm + c0), v);
+                if (c0 + 32 >= c_end)
+                {
+                    // everything is in registers: the accumulator may be overwritten
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        arrive_cluster_relaxed(lead_d_empty0 + 8 * db);
+                }
+                if (SPLIT == SPLIT_CLUSTER)
+                {
+                    // [row][128 columns] in the activation ring, which no copy or MMA uses any more
+                    float* dst = reinterpret_cast<float*>(smem) + c0 * BN + warp * 32 + lane;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        dst[j * BN] = __uint_as_float(v[j]);
+                    continue;
+                }
+                if (!n_ok)
+                    continue;
+                if (SPLIT == SPLIT_WORKSPACE)
+                {
+                    // fp32 partial tile; splitk_reduce_kernel, next on the stream, adds the partial tiles in
+                    // split order (deterministic) and writes the output
+                    float* dst = part + size_t(m0 + c0) * a.n;
+                    int const rows = a.m - m0 - c0;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j, dst += a.n)
+                        if (j < rows)
+                            __stcg(dst, __uint_as_float(v[j]));
+                }
+                else
+                {
+                    // (row pointers are advanced, not computed from the row: with an address product per
+                    // row and a bounds test in front of every store a chunk took twice as long)
+                    uint32_t o[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        o[j] = P::pack2(fmaf(a.alpha, __uint_as_float(v[2 * j]), bias_f),
+                            fmaf(a.alpha, __uint_as_float(v[2 * j + 1]), bias_f));
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        o[j] = prmt(o[j], __shfl_xor_sync(0xffffffffu, o[j], 1), sel);
+                    int const mrow = m0 + c0 + (lane & 1), rows = a.m - mrow; // this lane's rows: mrow, mrow + 2, ..
+                    uint16_t* dst = out + size_t(mrow) * a.n;
+                    size_t const two_rows = size_t(a.n) * 2;
+                    if (m0 + c0 + 32 <= a.m)
+                    {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j, dst += two_rows)
+                            *reinterpret_cast<uint32_t*>(dst) = o[j];
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j, dst += two_rows)
+                            if (2 * j < rows)
+                                *reinterpret_cast<uint32_t*>(dst) = o[j];
+                    }
+                }
+            }
+            db = db + 1 == a.d_bufs ? 0 : db + 1;
+        }
+    }
 
-    // Teardown: everyone meets here (also after a timeout), then the allocating warp frees TMEM.
+    // Teardown: both CTAs meet here (also after a timeout), then the allocating warps free TMEM.
     tc_fence_before();
     __syncthreads();
-    if (warp == 1)
+    if (*abort_flag)
+        for (int i = 0; i < 64; ++i)
+            __nanosleep(10000); // copies and MMAs that are still in flight end before the memory is given back
+    cluster_sync_all();
+    if (SPLIT == SPLIT_CLUSTER)
+    {
+        // Every CTA adds the rows row % splits == its split of its 128 columns: a warp per row, four columns
+        // per lane, the other splits' values from their shared memory.
+        int const tile = pair / a.splits, split = pair - tile * a.splits;
+        int const m0 = (tile / a.tiles_n) * a.bm, rows = min(a.bm, a.m - m0);
+        int const n = (tile % a.tiles_n) * kPairN + int(rank) * BN + 4 * lane;
+        if (n < a.n) // n is a multiple of 32
+        {
+            float b[4] = {0.f, 0.f, 0.f, 0.f};
+            if (a.bias)
+            {
+                uint2 const bw = *reinterpret_cast<uint2 const*>(static_cast<uint16_t const*>(a.bias) + n);
+                P::unpack2(bw.x, b[0], b[1]);
+                P::unpack2(bw.y, b[2], b[3]);
+            }
+            for (int row = split + a.splits * warp; row < rows; row += a.splits * (kThreads / 32))
+            {
+                uint32_t const local = smem_base + uint32_t(row * BN + 4 * lane) * 4u;
+                float4 x[kMaxClusterSplits];
+#pragma unroll
+                for (int q = 0; q < kMaxClusterSplits; ++q)
+                    if (q < a.splits)
+                        x[q] = ld_cluster_f4(cluster_addr(local, 2 * q + rank));
+                float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int q = 0; q < kMaxClusterSplits; ++q)
+                    if (q < a.splits)
+                    {
+                        sum.x += x[q].x;
+                        sum.y += x[q].y;
+                        sum.z += x[q].z;
+                        sum.w += x[q].w;
+                    }
+                uint2 o;
+                o.x = P::pack2(fmaf(a.alpha, sum.x, b[0]), fmaf(a.alpha, sum.y, b[1]));
+                o.y = P::pack2(fmaf(a.alpha, sum.z, b[2]), fmaf(a.alpha, sum.w, b[3]));
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.out) + size_t(m0 + row) * a.n + n) = o;
+            }
+        }
+        cluster_sync_all(); // nobody leaves while its shared memory is being read
+    }
+    if (warp == kMmaWarp)
     {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(kTmemCols))
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(kTmemCols))
                      : "memory");
     }
 }
@@ -704,6 +825,9 @@ __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(T* out, float const* partial, T const* bias, float alpha, size_t mn_vec, int n_vec, int splits)
 {
     using P = Pair<T>;
+    // programmatic dependent of the GEMM: its launch overlaps the GEMM's tail
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     size_t const i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= mn_vec)
         return;
@@ -746,16 +870,36 @@ __global__ void __launch_bounds__(256)
     *reinterpret_cast<uint2*>(out + i * 4) = o;
 }
 
-template <typename T, int BITS, int BM, bool HAS_ZERO, bool SPLITK>
-static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream, int splits)
+// Launches a kernel as a programmatic dependent of whatever precedes it in the stream (every kernel
+// here orders itself with griddepcontrol.wait before it touches what its predecessors may write).
+template <typename... KArgs, typename... Args_>
+static int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t smem, int cluster, cudaStream_t stream,
+    Args_ const&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = unsigned(cluster);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
+}
+
+template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
+static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream, TcPlan const& plan)
 {
     constexpr int IL = BITS == 4 ? 4 : 2;
-    constexpr int STAGE_BYTES = kHalves * (BM * 128 + (BN / IL) * 128);
-    auto kernel = gemm_kernel<T, BITS, BM, HAS_ZERO, SPLITK>;
+    constexpr int W_STAGE = 2 * (BN / IL) * 128 + 1024;
+    auto kernel = gemm_kernel<T, BITS, HAS_ZERO, SPLIT>;
 
     Args a{};
-    a.scales = p.scales;
-    a.zeros = p.zeros;
     a.bias = p.bias;
     a.out = p.out;
     a.alpha = p.alpha;
@@ -763,35 +907,52 @@ static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& 
     a.n = p.n;
     a.k = p.k;
     a.group_shift = p.group_size == 64 ? 6 : (p.group_size == 128 ? 7 : 31);
-    a.tiles_n = (p.n + BN - 1) / BN;
-    a.tiles_m = (p.m + BM - 1) / BM;
+    a.bm = plan.bm;
+    a.tiles_n = (p.n + kPairN - 1) / kPairN;
+    a.tiles_m = (p.m + plan.bm - 1) / plan.bm;
+    a.weights_static = (p.flags & W4_GEMM_WEIGHTS_STATIC) ? 1 : 0;
+    a.splits = plan.splits;
+    a.steps_split = plan.steps_split;
+    if (SPLIT == SPLIT_WORKSPACE)
     {
-        // Split-k (chosen by the caller of this function): partial tiles go to the workspace, behind
-        // the scaled copy of the activations if there is one.
-        int const ksteps = (p.k + BK - 1) / BK;
+        // partial tiles go to the workspace, behind the scaled copy of the activations if there is one
         size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
-        a.ksteps_split = (ksteps + splits - 1) / splits;
-        a.splits = (ksteps + a.ksteps_split - 1) / a.ksteps_split; // no empty work items
-        if (SPLITK)
-            a.partial = reinterpret_cast<float*>(static_cast<char*>(p.workspace) + act_copy);
+        a.partial = reinterpret_cast<float*>(static_cast<char*>(p.workspace) + act_copy);
     }
-    size_t const fixed = sizeof(Barriers) + 1024; // + slack to align the ring to 1024 bytes
-    int stages = int((size_t(dev.max_smem_optin) - fixed) / STAGE_BYTES);
-    if (stages < 2)
+    // Rings: as many 128-k steps as fit TMEM next to the accumulators (4 at 256 and at 128 rows, more in
+    // between and below), the rest of shared memory for weight blocks.
+    a.d_bufs = plan.bm <= 128 ? 2 : 1;
+    int const stages = (kTmemCols - a.d_bufs * plan.bm) / kStageCols;
+    a.num_stages = stages < kMaxStages ? stages : kMaxStages;
+    size_t const fixed = sizeof(Barriers) + 16;
+    size_t const act_bytes = size_t(a.num_stages) * plan.bm * 128;
+    if (size_t(dev.max_smem_optin) < fixed + act_bytes + 3 * W_STAGE)
         return W4_ERR_CUDA;
-    a.num_stages = stages > kMaxStages ? kMaxStages : stages;
-    size_t const smem = size_t(a.num_stages) * STAGE_BYTES + fixed;
+    size_t const wstages = (size_t(dev.max_smem_optin) - fixed - act_bytes) / W_STAGE;
+    a.num_wstages = wstages < size_t(kMaxWStages) ? int(wstages) : kMaxWStages;
+    size_t const smem = act_bytes + size_t(a.num_wstages) * W_STAGE + fixed;
 
-    // Activations [m, k] of T, boxes of 64 k x BM rows, 128-byte swizzle (rows past m read as 0).
-    // Weights as bytes: [n / IL interleaved rows, 2k bytes], boxes of one 128-byte line x BN/IL rows.
-    CUtensorMap tm_act, tm_w;
+    // Activations [m, k] of T, boxes of 64 k x bm / 2 rows, 128-byte swizzle (rows past m read as 0).
+    // Weights as bytes [k / 64 lines, n / IL interleaved rows, 128], boxes of two lines x 128 / IL rows.
+    // Scales / zeros [groups, n], boxes of the rows of a 128-wide k step x 128 columns.
+    CUtensorMap tm_act, tm_w, tm_s, tm_z;
     CUtensorMapDataType const dt
         = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    if (!make_tensor_map_2d(&tm_act, dt, act, uint64_t(p.k), uint64_t(p.m), uint64_t(p.k) * 2, 64, BM,
+    if (!make_tensor_map_2d(&tm_act, dt, act, uint64_t(p.k), uint64_t(p.m), uint64_t(p.k) * 2, 64, uint32_t(plan.bm / 2),
             CU_TENSOR_MAP_SWIZZLE_128B))
         return W4_ERR_CUDA;
-    if (!make_tensor_map_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.weight, uint64_t(p.k) * 2, uint64_t(p.n / IL),
-            uint64_t(p.k) * 2, 128 * kHalves, BN / IL, CU_TENSOR_MAP_SWIZZLE_NONE))
+    if (!make_tensor_map_3d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.weight, 128, uint64_t(p.n / IL), uint64_t(p.k / 64),
+            uint64_t(p.k) * 2, 128, 128, BN / IL, 2, CU_TENSOR_MAP_SWIZZLE_128B))
+        return W4_ERR_CUDA;
+    uint64_t const groups = p.group_size ? uint64_t(p.k / p.group_size) : 1;
+    uint32_t const box_rows = p.group_size == 64 ? 2 : 1;
+    if (!make_tensor_map_2d(&tm_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.scales, uint64_t(p.n), groups, uint64_t(p.n) * 2, BN,
+            box_rows, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return W4_ERR_CUDA;
+    tm_z = tm_s;
+    if (HAS_ZERO
+        && !make_tensor_map_2d(&tm_z, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.zeros, uint64_t(p.n), groups, uint64_t(p.n) * 2, BN,
+            box_rows, CU_TENSOR_MAP_SWIZZLE_NONE))
         return W4_ERR_CUDA;
 
     {
@@ -802,54 +963,41 @@ static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& 
         if (dev.device < 0 || dev.device >= 64 || !configured[dev.device])
         {
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin)
-                != cudaSuccess)
+                    != cudaSuccess
+                || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
                 return W4_ERR_CUDA;
             if (dev.device >= 0 && dev.device < 64)
                 configured[dev.device] = true;
         }
     }
-    int const tiles = a.tiles_n * a.tiles_m * (SPLITK ? a.splits : 1);
-    int const grid = tiles < dev.num_sms ? tiles : dev.num_sms;
-    kernel<<<grid, kThreads, smem, stream>>>(a, tm_act, tm_w);
-    if (SPLITK)
+    int const items = a.tiles_n * a.tiles_m * a.splits;
+    int const pairs = SPLIT == SPLIT_CLUSTER || items < dev.num_sms / 2 ? items : dev.num_sms / 2;
+    int rc = launch_pdl(kernel, 2 * pairs, kThreads, smem, SPLIT == SPLIT_CLUSTER ? 2 * a.splits : 2, stream, a, tm_act, tm_w,
+        tm_s, tm_z);
+    if (rc == W4_OK && SPLIT == SPLIT_WORKSPACE)
     {
         size_t const mn_vec = size_t(p.m) * p.n / 4; // n is a multiple of 32
-        splitk_reduce_kernel<T><<<unsigned((mn_vec + 255) / 256), 256, 0, stream>>>(static_cast<T*>(p.out), a.partial,
-            static_cast<T const*>(p.bias), p.alpha, mn_vec, p.n / 4, a.splits);
+        rc = launch_pdl(splitk_reduce_kernel<T>, int((mn_vec + 255) / 256), 256, 0, 1, stream, static_cast<T*>(p.out),
+            static_cast<float const*>(a.partial), static_cast<T const*>(p.bias), p.alpha, mn_vec, p.n / 4, a.splits);
     }
-    return cudaGetLastError() == cudaSuccess ? W4_OK : W4_ERR_CUDA;
+    return rc;
 }
 
 template <typename T, int BITS, bool HAS_ZERO>
-static int dispatch_bm(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream)
+static int dispatch_split(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream)
 {
-    int const bm = gemm_tc_row_tile(p.m, p.n, dev.num_sms, p.weight_bits);
-    // Split-k when the tiles alone would leave most SMs idle and the caller's workspace has room
-    // for the partial tiles; the unsplit kernel is a separate instantiation without any of it.
-    int splits = gemm_tc_splits(p.m, p.n, p.k, dev.num_sms, p.weight_bits);
-    if (splits > 1)
+    TcPlan plan = gemm_tc_plan(p.m, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, true);
+    if (plan.splits > 1 && plan.cluster)
+        return launch_one<T, BITS, HAS_ZERO, SPLIT_CLUSTER>(p, act, dev, stream, plan);
+    if (plan.splits > 1)
     {
+        // this form of split-k needs room for the partial tiles in the caller's workspace
         size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
-        if (!p.workspace || p.workspace_bytes < act_copy + split_bytes(p.m, p.n, splits))
-            splits = 1;
+        if (p.workspace && p.workspace_bytes >= act_copy + split_bytes(p.m, p.n, plan.splits))
+            return launch_one<T, BITS, HAS_ZERO, SPLIT_WORKSPACE>(p, act, dev, stream, plan);
+        plan = gemm_tc_plan(p.m, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false);
     }
-    if (splits > 1)
-    {
-        if (bm == 64)
-            return launch_one<T, BITS, 64, HAS_ZERO, true>(p, act, dev, stream, splits);
-        if (bm == 128)
-            return launch_one<T, BITS, 128, HAS_ZERO, true>(p, act, dev, stream, splits);
-        if (bm == 192)
-            return launch_one<T, BITS, 192, HAS_ZERO, true>(p, act, dev, stream, splits);
-        return launch_one<T, BITS, 256, HAS_ZERO, true>(p, act, dev, stream, splits);
-    }
-    if (bm == 64)
-        return launch_one<T, BITS, 64, HAS_ZERO, false>(p, act, dev, stream, 1);
-    if (bm == 128)
-        return launch_one<T, BITS, 128, HAS_ZERO, false>(p, act, dev, stream, 1);
-    if (bm == 192)
-        return launch_one<T, BITS, 192, HAS_ZERO, false>(p, act, dev, stream, 1);
-    return launch_one<T, BITS, 256, HAS_ZERO, false>(p, act, dev, stream, 1);
+    return launch_one<T, BITS, HAS_ZERO, SPLIT_NONE>(p, act, dev, stream, plan);
 }
 
 template <typename T>
@@ -857,79 +1005,111 @@ static int dispatch(W4GemmParams const& p, void const* act, DeviceInfo const& de
 {
     bool const z = p.zeros != nullptr;
     if (p.weight_bits == 4)
-        return z ? dispatch_bm<T, 4, true>(p, act, dev, stream) : dispatch_bm<T, 4, false>(p, act, dev, stream);
-    return z ? dispatch_bm<T, 8, true>(p, act, dev, stream) : dispatch_bm<T, 8, false>(p, act, dev, stream);
+        return z ? dispatch_split<T, 4, true>(p, act, dev, stream) : dispatch_split<T, 4, false>(p, act, dev, stream);
+    return z ? dispatch_split<T, 8, true>(p, act, dev, stream) : dispatch_split<T, 8, false>(p, act, dev, stream);
+}
+
+// Clusters of 2 * splits CTAs the current device runs side by side: fixed by how its SMs are grouped.
+// Without a device, the numbers of a B200 with all 148 SMs.
+static int max_clusters(int splits)
+{
+    struct Limits
+    {
+        bool known = false;
+        int clusters[kMaxClusterSplits + 1] = {0, 74, 33, 22, 15, 11, 7, 7, 7};
+    };
+    static std::mutex mu;
+    static Limits devices[64], none;
+    DeviceInfo const& dev = current_device_info();
+    std::lock_guard<std::mutex> lock(mu);
+    Limits& l = dev.num_sms > 0 ? devices[dev.device] : none;
+    if (dev.num_sms > 0 && !l.known)
+    {
+        auto kernel = gemm_kernel<__nv_bfloat16, 4, true, SPLIT_CLUSTER>;
+        bool const ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin) == cudaSuccess
+            && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        for (int s = 1; s <= kMaxClusterSplits; ++s)
+        {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(unsigned(2 * s));
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = size_t(dev.max_smem_optin);
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = unsigned(2 * s);
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            l.clusters[s] = ok && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
+        }
+        (void) cudaGetLastError(); // a cluster size the device refuses is no error of the caller's
+        l.known = true;
+    }
+    return l.clusters[splits];
 }
 
 } // namespace tc
 
-
-// Microseconds one CTA spends per 128-wide k step, by row tile (measured on B200, bf16, group 128).
-// int4: up to 192 rows the step is bound by the conversion / hand-off pipeline, not by its tensor
-// work; 256 rows leave shared memory for three stages only and the step turns latency-bound. int8
-// stages carry 16 KB of weights instead of 8: four of them fit up to 128 rows, three at 192 rows
-// (4096 x 14336 x 4096: 546 us with 128-row tiles against 623 us with 192), two at 256; with 64-row
-// tiles the int8 step is shorter (4096 x 14336 at 32 and 64 rows: 25 us for 32 steps).
-static double step_us(int bm, int bits)
+// Microseconds per 128-wide k step of a CTA pair (measured on B200): up to 96 rows the conversion's, which
+// takes most of the issue slots and, for int8 to bf16, more instructions per weight; above, the MMAs'
+// (1024 tensor cycles at 256 rows).
+static double step_us(int bm, int bits, int act_dtype)
 {
-    if (bits == 8)
-        return bm <= 64 ? 0.56 : (bm <= 128 ? 0.70 : (bm == 192 ? 1.11 : 1.9));
-    return bm <= 128 ? 0.57 : (bm == 192 ? 0.70 : 1.05);
+    double const conv = bits == 8 && act_dtype == W4_DTYPE_BF16 ? 0.35 : 0.27, mma = bm * (0.57 / 256);
+    return conv > mma ? conv : mma;
 }
 
-// Split-k factor: used when the output tiles would occupy less than half of the SMs; every work
-// item keeps at least four k steps; only for m <= 256, where the fp32 partial tiles stay small.
-int gemm_tc_splits(int m, int n, int k, int num_sms, int bits)
+// The plan with the shortest estimated time: row tiles in steps of 32 and, where the tiles leave pairs idle
+// (and only up to 256 rows, where the fp32 partial tiles stay small), split factors. A launch costs 2 us plus
+// the waves of its work items; an item's epilogue 0.3 us per 32 rows, of which the double-buffered
+// accumulators hide all but the last. Splits that share a cluster add the exchange of the partial tiles
+// (clusters of 4 and 8 CTAs about 1 us; 6 and more than 8 wait longer for enough free SMs side by side), splits
+// through the workspace a second kernel and their traffic. Fitted to 4096 and 8192 x 1024..14336 at 16 to
+// 777 rows: within 1 us of the best plan found by trying all at 14 of 16 points.
+TcPlan gemm_tc_plan(int m, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace)
 {
-    int const bm = gemm_tc_row_tile(m, n, num_sms, bits);
-    long const tiles = long((n + tc::BN - 1) / tc::BN) * long((m + bm - 1) / bm);
-    int const ksteps = (k + tc::BK - 1) / tc::BK;
-    if (tiles * 2 > num_sms || m > 256)
-        return 1;
-    long s = num_sms / tiles;
-    if (s > ksteps / 4)
-        s = ksteps / 4;
-    if (s > 16)
-        s = 16;
-    return s < 1 ? 1 : int(s);
-}
-
-static double waves(int m, int n, int bm, int num_sms, int splits = 1)
-{
-    long const tiles = long((n + tc::BN - 1) / tc::BN) * long((m + bm - 1) / bm) * splits;
-    return double((tiles + num_sms - 1) / num_sms);
-}
-
-int gemm_tc_row_tile(int m, int n, int num_sms, int bits)
-{
-    if (m <= 64)
-        return 64;
-    if (m <= 128)
-        return 128;
-    if (m <= 192 && bits != 8) // int8 keeps only three stages at 192 rows: let the costs decide
-        return 192;
-    int const cand[3] = {128, 192, 256};
-    int bm = 0;
-    double best = 0;
-    for (int i = 0; i < 3; ++i)
+    int const pairs = num_sms > 1 ? num_sms / 2 : 1;
+    int const steps = (k + 127) / 128;
+    long const tiles_n = (n + tc::kPairN - 1) / tc::kPairN;
+    TcPlan best{};
+    int const most = m >= tc::kMaxBM ? tc::kMaxBM : (m + 31) & ~31;
+    for (int bm = 32; bm <= most; bm += 32)
     {
-        double const cost = waves(m, n, cand[i], num_sms) * step_us(cand[i], bits);
-        if (!bm || cost < best)
+        long const tiles = tiles_n * ((m + bm - 1) / bm);
+        double const step = step_us(bm, bits, act_dtype), drain = 0.01 * bm;
+        int splits_max = m <= 256 && tiles < pairs ? int(pairs / tiles) : 1;
+        splits_max = splits_max > 16 ? 16 : splits_max;
+        for (int s = 1; s <= splits_max; ++s)
         {
-            bm = cand[i];
-            best = cost;
+            int const per = (steps + s - 1) / s;
+            if ((steps + per - 1) / per != s || (s > 1 && per < 2))
+                continue; // an empty work item, or too little in each
+            bool const cluster = s > 1 && s <= tc::kMaxClusterSplits && tiles <= tc::max_clusters(s);
+            if (s > 1 && !cluster && !may_use_workspace)
+                continue;
+            double const waves = double((tiles * s + pairs - 1) / pairs);
+            double us = 2.0 + drain + waves * per * step + (waves - 1) * (bm <= 128 ? 0.1 : drain + 0.3);
+            if (cluster)
+                us += (s == 2 || s == 4 ? 1.0 : 3.0) + 0.008 * bm;
+            else if (s > 1)
+                us += 2.5 + double(s) * m * n * 8.0 / 6.0e6;
+            if (!best.bm || us < best.us)
+            {
+                best.bm = bm;
+                best.splits = s;
+                best.steps_split = per;
+                best.cluster = cluster;
+                best.us = us;
+            }
         }
     }
-    return bm;
+    return best;
 }
 
-double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits)
+double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits, int act_dtype)
 {
-    int const bm = gemm_tc_row_tile(m, n, num_sms, bits);
-    int const splits = gemm_tc_splits(m, n, k, num_sms, bits);
-    int const ksteps = (k + tc::BK - 1) / tc::BK;
-    int const per = (ksteps + splits - 1) / splits;
-    return 7.0 + (splits > 1 ? 3.0 : 0.0) + waves(m, n, bm, num_sms, splits) * step_us(bm, bits) * double(per);
+    return gemm_tc_plan(m, n, k, num_sms, bits, act_dtype, true).us;
 }
 
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale)
@@ -939,12 +1119,13 @@ size_t gemm_tc_workspace_min(int m, int k, int has_act_scale)
     return has_act_scale ? size_t(m) * k * 2 : 0;
 }
 
-size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits)
+size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits, int act_dtype)
 {
-    // what lets the kernel use split-k as well; with less (but at least the minimum) it runs unsplit
+    // what lets the kernel use every form of split-k; with less (but at least the minimum) it runs with the
+    // forms that need none
     DeviceInfo const& dev = current_device_info();
     int const sms = dev.num_sms > 0 ? dev.num_sms : 148;
-    int const splits = gemm_tc_splits(m, n, k, sms, bits);
+    int const splits = gemm_tc_plan(m, n, k, sms, bits, act_dtype, true).splits;
     size_t bytes = gemm_tc_workspace_min(m, k, has_act_scale);
     if (splits > 1)
         bytes = tc::split_align(bytes) + tc::split_bytes(m, n, splits);

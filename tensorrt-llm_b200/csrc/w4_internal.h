@@ -46,12 +46,20 @@ bool allreduce_push_target(W4AllReduceParams const& r, PushTarget* t);
 int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream);
 // Workspace: the minimum the kernel needs (scaled activation copy), and what also allows split-k.
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale);
-size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits);
-int gemm_tc_splits(int m, int n, int k, int num_sms, int bits);
-// Activation-row tile the tensor-core kernel uses for this problem, and its estimated duration
-// (microseconds, measured per-step costs); shared by the launcher and the regime heuristic.
-int gemm_tc_row_tile(int m, int n, int num_sms, int bits);
-double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits);
+size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits, int act_dtype);
+// How the tensor-core kernel runs a problem: activation rows per tile, split-k factor and 128-wide k
+// steps per work item, and the estimated duration (microseconds, from measured step costs); shared by the
+// launcher, the workspace size and the regime heuristic.
+struct TcPlan
+{
+    int bm = 0;
+    int splits = 1;
+    int steps_split = 0;
+    bool cluster = false; // the splits of a tile are one cluster (otherwise they meet in the workspace)
+    double us = 0;
+};
+TcPlan gemm_tc_plan(int m, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace);
+double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits, int act_dtype);
 
 // out[m, k] = act[m, k] * scale[k], rounded to the element type (the reference's
 // apply_per_channel_scale, cpp/tensorrt_llm/kernels/preQuantScaleKernel.cu:43-95).

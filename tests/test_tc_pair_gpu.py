@@ -1,0 +1,45 @@
+"""The CTA-pair tensor-core kernel at the sizes where its tiles, rings and splits can go wrong (needs a B200)."""
+import pytest
+import torch
+
+import tensorrt_llm_b200 as pkg
+from oracle import woq_oracle as oracle
+from _cases import make_problem, max_err, oracle_out, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k,bits,group,dtype", [
+    (31, 64, 64, 4, 64, torch.bfloat16),      # one half-filled step; the pair's second CTA has no columns
+    (33, 320, 128, 4, 128, torch.float16),    # the second pair tile has half of one CTA's columns
+    (257, 192, 192, 8, 64, torch.bfloat16),   # two row tiles, odd number of 64-k halves
+    (160, 8192, 1152, 8, 0, torch.bfloat16),  # seven weight stages, nine steps, three conversion groups
+    (224, 16640, 832, 4, 64, torch.float16),  # single accumulator, rings that wrap at different places
+    (96, 19200, 640, 8, 128, torch.float16),  # two accumulators, more tiles than pairs
+    (64, 1280, 2048, 4, 128, torch.bfloat16),  # splits that share a cluster
+    (17, 96, 8192, 8, 0, torch.float16),      # one tile, the largest cluster
+    (250, 512, 4096, 4, 64, torch.bfloat16),  # cluster splits of a 256-row tile
+    (40, 256, 4224, 4, 128, torch.bfloat16),  # 33 steps: the last split is shorter
+])
+def test_tile_ring_and_split_edges(m, n, k, bits, group, dtype):
+    full = group != 0
+    p = make_problem(m, n, k, bits, group, dtype, zero=full, bias=full, seed=m + n)
+    alpha = 0.5 if full else 1.0
+    rows = sorted({0, m - 1, *range(0, m, 29)})
+    for _ in range(3):  # back to back: the next launch's weights are fetched while the previous one drains
+        out = run_gpu(p, regime=pkg.W4_REGIME_GEMM, alpha=alpha)
+    ref = oracle_out(dict(p, act=p["act"][rows].contiguous(), m=len(rows)), alpha=alpha)
+    assert max_err(out[rows], ref) <= oracle.tolerance(ref)
+    assert torch.equal(out, run_gpu(p, regime=pkg.W4_REGIME_GEMM, alpha=alpha))  # sums in a fixed order
+    assert pkg._lib.lib().w4_gemm_device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,bits", [(9, 14336, 1024, 4), (16, 4096, 4096, 4), (12, 8192, 2048, 8)])
+def test_decode_regime_through_the_tensor_cores(m, n, k, bits):
+    """9 to 16 rows in the decode regime: whichever kernel the launch takes needs no workspace and agrees
+    with the decode kernel to rounding."""
+    p = make_problem(m, n, k, bits, 128, torch.bfloat16, zero=True, bias=True, seed=m)
+    assert pkg.ops.workspace_bytes(m, n, k, 128, bits, torch.bfloat16, False) == 0
+    auto, decode = run_gpu(p), run_gpu(p, regime=pkg.W4_REGIME_GEMV)
+    ref = oracle_out(p)
+    assert max_err(auto, ref) <= oracle.tolerance(ref) and max_err(auto, decode) <= oracle.tolerance(ref)
