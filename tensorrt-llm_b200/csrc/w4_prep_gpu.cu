@@ -11,9 +11,12 @@
 // adjacent columns - the closed form of the four reference passes (row permutation inside 16/32-row
 // blocks, sub-byte transpose, column interleave in 64-k tiles, bias + in-register shuffle).
 #include <algorithm>
+#include <mutex>
+#include <type_traits>
 
 #include "w4_common.cuh"
 #include "w4_internal.h"
+#include "w4_tma.h"
 
 namespace w4
 {
@@ -367,6 +370,437 @@ __global__ void __launch_bounds__(kThreads)
     emit_tile<BITS>(out, tile, k_tile, n0, cols, K);
 }
 
+// ------------------------------------------------------------------------------------------------
+// Quantisation in one pass over the weights. A cluster of CTAs owns a strip of columns (128 or 64
+// bytes of each row) and all of K: every CTA brings its rows of the strip into shared
+// memory by TMA, finds their column maxima as the 64-row boxes land, the cluster combines the maxima through
+// distributed shared memory, and the weights are quantised and laid out straight from shared memory.
+// HBM-bound: each weight is read from memory once (the two passes of the kernels below read it twice, and
+// scales were a memset, an atomic merge and a launch in between). 4096 x 14336 bf16 -> int4: 98 -> QUS us
+// per call. A thread turns one block of 32 (int4) / 16 (int8) rows x 8 columns - what four adjacent output
+// registers of each column hold - so all its stores are 16 bytes and a warp writes whole 32-byte sectors.
+// Several CTAs share an SM, so that one's arithmetic covers another's loads.
+// ------------------------------------------------------------------------------------------------
+constexpr int kMaxStripThreads = 256;
+constexpr int kMaxStripTiles = 56;        // 64-row boxes of a CTA at most
+constexpr int kMaxStripSmem = 224 * 1024; // shared memory for them
+
+struct StripArgs
+{
+    uint32_t* out;
+    uint8_t* unprocessed;
+    float* scales;
+    void* scales_t;
+    int scales_dtype;
+    int K, N;
+    int tiles_cta; // 64-row tiles per CTA, the last one may have fewer (or none)
+};
+
+// max(|a|, |b|) of eight weights as they lie in memory: kept packed.
+template <typename W>
+struct StripMax
+{
+    using W2 = typename std::conditional<std::is_same<W, __half>::value, __half2, __nv_bfloat162>::type;
+    W2 m[4];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint32_t*>(&m[i]) = 0u;
+    }
+    __device__ __forceinline__ void add(uint4 v)
+    {
+        uint32_t const w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            m[i] = __hmax2(m[i], __habs2(*reinterpret_cast<W2 const*>(&w[i])));
+    }
+    __device__ __forceinline__ void get(float (&x)[8]) const
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            Pair<W>::unpack2(*reinterpret_cast<uint32_t const*>(&m[i]), x[2 * i], x[2 * i + 1]);
+    }
+};
+
+// Eight consecutive weights of a staged row; `flip` exchanges the order in which the two halves of an fp32
+// vector are read (bank conflicts).
+template <typename W>
+__device__ __forceinline__ void strip_load8(uint8_t const* row, int c, bool flip, float (&x)[8])
+{
+    if constexpr (std::is_same<W, float>::value)
+    {
+        float4 const* p = reinterpret_cast<float4 const*>(row) + 2 * c;
+        float4 const a = p[flip ? 1 : 0], b = p[flip ? 0 : 1];
+        float4 const lo = flip ? b : a, hi = flip ? a : b;
+        x[0] = lo.x, x[1] = lo.y, x[2] = lo.z, x[3] = lo.w, x[4] = hi.x, x[5] = hi.y, x[6] = hi.z, x[7] = hi.w;
+    }
+    else
+    {
+        uint4 const v = reinterpret_cast<uint4 const*>(row)[c];
+        Pair<W>::unpack2(v.x, x[0], x[1]);
+        Pair<W>::unpack2(v.y, x[2], x[3]);
+        Pair<W>::unpack2(v.z, x[4], x[5]);
+        Pair<W>::unpack2(v.w, x[6], x[7]);
+    }
+}
+
+// Packs eight q + 2^(BITS - 1) in column order. Float arithmetic up to the packed integers, which has twice
+// the integer pipe's rate: sums of q * 16^e (or 256^e) below 2^16 are exact.
+template <int BITS>
+__device__ __forceinline__ void pack_q(float const (&q)[8], uint32_t (&word)[BITS / 4])
+{
+    constexpr float kStep = BITS == 8 ? 256.f : 16.f;
+    constexpr float kBias = BITS == 8 ? 128.f * 257.f : 8.f * 4369.f;
+    constexpr int PER = 16 / BITS;
+    uint32_t half[BITS / 2]; // 2^23 + 16 bits of the result each
+#pragma unroll
+    for (int h = 0; h < BITS / 2; ++h)
+    {
+        float v = q[h * PER + PER - 1];
+#pragma unroll
+        for (int e = PER - 2; e >= 0; --e)
+            v = fmaf(v, kStep, q[h * PER + e]);
+        half[h] = __float_as_uint(v + (8388608.f + kBias));
+    }
+#pragma unroll
+    for (int w = 0; w < BITS / 4; ++w)
+        word[w] = prmt(half[2 * w], half[2 * w + 1], 0x5410u);
+}
+
+// clamp(round-half-away(fl(x / s))), fl = the rounding of the reference's fp32 division.
+template <int BITS>
+__device__ __noinline__ float quantize_exact(float x, float s)
+{
+    int const q = s != 0.f ? int(roundf(__fdiv_rn(x, s))) : 0;
+    return float(max(-(1 << (BITS - 1)), min((1 << (BITS - 1)) - 1, q)));
+}
+
+// Scales of a thread's eight columns and what the arithmetic needs of them.
+struct StripScales
+{
+    float s[8], inv[8], half[8]; // half: s / 2, or 1 for a zero column
+    bool extreme;                // some scale is near underflow or overflow: divide
+    __device__ __forceinline__ void load(float const* scale)
+    {
+        extreme = false;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+        {
+            s[e] = scale[e];
+            extreme |= s[e] != 0.f && !(s[e] > 1e-30f && s[e] < 1e30f);
+            inv[e] = s[e] != 0.f ? __fdiv_rn(1.f, s[e]) : 0.f;
+            half[e] = s[e] != 0.f ? 0.5f * s[e] : 1.f;
+        }
+    }
+};
+
+// round-half-away(fl(x / s)) by comparing |x| with the boundary instead of dividing (a product with the
+// reciprocal is not enough: a 16-bit weight in a thousand sits exactly on a boundary). m = the integer in
+// front of the boundary B = m + 1/2 next to |x / s|, from the rounded product with 1 / s - 1/2 (an error next
+// to an integer picks a neighbour's boundary, which gives the same result). The answer is m + 1 where
+// fl(|x| / s) >= B, that is where |x| / s >= B - u / 2 with u the spacing of the floats below B (the midpoint
+// rounds to B, whose mantissa is even). |x| - m s is exact near the boundary, elsewhere its size decides.
+// 16-bit weights: s is the largest times a power of two, so |x| - B s is zero or at least 2^-20 s and u / 2
+// plays no part. Eight instructions a weight, five of them on the float pipe.
+template <typename W, int BITS>
+__device__ __forceinline__ float quantize1(float x, float s, float inv, float half)
+{
+    constexpr float kRound = 12582912.f; // 1.5 * 2^23: adding it rounds to an integer
+    float const a = fabsf(x), m = (fmaf(a, inv, -0.5f) + kRound) - kRound;
+    float const t = fmaf(-m, s, a);
+    bool up = t >= half;
+    if constexpr (std::is_same<W, float>::value)
+    {
+        float const half_u = __uint_as_float((__float_as_uint(m + 0.5f) - 1u) & 0x7f800000u) * 0x1p-24f;
+        up = t - half >= -half_u * s;
+    }
+    float const q = m + (up ? 1.f : 0.f);
+    return fminf(copysignf(q, x), BITS == 8 ? 127.f : 7.f);
+}
+
+template <typename W, int BITS>
+__device__ __forceinline__ void quantize8(float const (&x)[8], StripScales const& c, uint32_t (&word)[BITS / 4])
+{
+    float q[8];
+    if (!c.extreme)
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            q[e] = quantize1<W, BITS>(x[e], c.s[e], c.inv[e], c.half[e]);
+    else
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            q[e] = quantize_exact<BITS>(x[e], c.s[e]);
+    pack_q<BITS>(q, word);
+}
+
+template <typename W, int BITS, int kStripBytes>
+__global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripArgs const a, __grid_constant__ CUtensorMap const tm)
+{
+    constexpr int E = 32 / BITS;                    // elements per output register
+    constexpr int VT = 64 / E;                      // registers per 64-k tile of one column
+    constexpr int IL = BITS == 8 ? 2 : 4;           // interleaved columns
+    constexpr int GP = 4 * E;                       // rows of a block: four registers
+    constexpr int S = kStripBytes / int(sizeof(W)); // columns of the strip
+    constexpr int NV = S / 8;                       // vectors of eight columns
+    constexpr int TILE_BYTES = 64 * kStripBytes;
+    extern __shared__ __align__(128) uint8_t slab[];
+    __shared__ float part[kMaxStripThreads / 32][S];
+    __shared__ float amax[S];
+    __shared__ float scale_s[S];
+    __shared__ __align__(8) uint64_t full[kMaxStripTiles];
+    __shared__ int failed;
+
+    uint32_t rank, ranks;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    int const n0 = int(blockIdx.x / ranks) * S;
+    int const t0 = int(rank) * a.tiles_cta, tiles = min(a.tiles_cta, a.K / 64 - t0); // <= 0: nothing here
+    int const tid = threadIdx.x, lane = tid & 31, cv = tid % NV;
+    if (tid == 0)
+    {
+        failed = 0;
+        for (int i = 0; i < tiles; ++i)
+            mbar_init(&full[i], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory"); // the weights, and what the outputs held before
+    if (tid == 0)
+        for (int i = 0; i < tiles; ++i)
+        {
+            mbar_expect_tx(&full[i], TILE_BYTES);
+            tma_load_2d(slab + i * TILE_BYTES, &tm, n0, (t0 + i) * 64, &full[i]);
+        }
+
+    // ---- column maxima: a thread walks one vector of columns
+    float m[8];
+    bool ok = true;
+    if constexpr (std::is_same<W, float>::value)
+    {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            m[e] = 0.f;
+        for (int i = 0; i < tiles && ok; ++i)
+        {
+            ok = mbar_wait(&full[i], 0);
+            for (int r = tid / NV; r < 64 && ok; r += int(blockDim.x) / NV)
+            {
+                float x[8];
+                strip_load8<W>(slab + i * TILE_BYTES + r * kStripBytes, cv, (tid / NV) & 1, x);
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    m[e] = fmaxf(m[e], fabsf(x[e]));
+            }
+        }
+    }
+    else
+    {
+        StripMax<W> pm;
+        pm.clear();
+        for (int i = 0; i < tiles && ok; ++i)
+        {
+            ok = mbar_wait(&full[i], 0);
+            for (int r = tid / NV; r < 64 && ok; r += int(blockDim.x) / NV)
+                pm.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
+        }
+        pm.get(m);
+    }
+    if (!ok)
+        failed = 1;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int x = NV; x < 32; x *= 2)
+            m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], x));
+    if (lane < NV)
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            part[tid >> 5][lane * 8 + e] = m[e];
+    __syncthreads();
+    if (tid < S)
+    {
+        float v = part[0][tid];
+        for (int w = 1; w < int(blockDim.x) / 32; ++w)
+            v = fmaxf(v, part[w][tid]);
+        amax[tid] = v;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < S)
+    {
+        float v = 0.f;
+        for (uint32_t q = 0; q < ranks; ++q)
+        {
+            uint32_t addr;
+            float other;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&amax[tid])), "r"(q));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(addr) : "memory");
+            v = fmaxf(v, other);
+        }
+        float const s = v * (1.f / float(1 << (BITS - 1)));
+        scale_s[tid] = s;
+        int const c = n0 + tid;
+        if (rank == 0 && c < a.N)
+        {
+            a.scales[c] = s;
+            if (a.scales_t)
+            {
+                if (a.scales_dtype == W4_DTYPE_FP16)
+                    static_cast<__half*>(a.scales_t)[c] = __float2half_rn(s);
+                else
+                    static_cast<__nv_bfloat16*>(a.scales_t)[c] = __float2bfloat16_rn(s);
+            }
+        }
+    }
+    // (the barrier is also the CTA's; nobody leaves while its maxima are being read)
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (failed)
+        return;
+
+    // ---- quantise: a thread takes the E rows behind one output register of eight columns and leaves the eight
+    // finished registers in the place of the first two rows of its own input
+    int const c0 = n0 + cv * 8;
+    bool const inside = c0 < a.N; // n is a multiple of 32: a thread's eight columns are all inside or all outside
+    size_t const row_bytes = size_t(a.N) * BITS / 8;
+    constexpr uint32_t kSigned = BITS == 8 ? 0x80808080u : 0x88888888u;
+    // 16-byte place of registers 4h .. 4h + 3 of block b, register r4, column vector v
+    auto place = [&](int b, int r4, int v, int h)
+    {
+        uint8_t* row = slab + (b * GP + 2 * r4) * kStripBytes;
+        return reinterpret_cast<uint4*>(sizeof(W) == 4 ? row + v * 32 + h * 16 : row + h * kStripBytes + v * 16);
+    };
+    int const blocks = tiles * (64 / GP);
+    if (inside)
+    {
+        StripScales sc;
+        sc.load(scale_s + cv * 8);
+#pragma unroll 1
+        for (int u = tid / NV; u < blocks * 4; u += int(blockDim.x) / NV)
+        {
+            int const b = u >> 2, r4 = u & 3;
+            uint8_t const* block = slab + (b * GP + 2 * r4) * kStripBytes;
+            uint32_t w[BITS / 4][E];
+#pragma unroll
+            for (int d = 0; d < E; ++d)
+            {
+                // the row behind position d of the register, as in emit_tile
+                int const p = BITS == 4 ? (d < 4 ? 2 * d : 2 * (d - 4) + 1) : (d == 1 ? 2 : (d == 2 ? 1 : d));
+                int const row = 8 * (p >> 1) + (p & 1);
+                float x[8];
+                strip_load8<W>(block + row * kStripBytes, cv, (tid / NV) & 1, x);
+                uint32_t word[BITS / 4];
+                quantize8<W, BITS>(x, sc, word);
+#pragma unroll
+                for (int h = 0; h < BITS / 4; ++h)
+                {
+                    w[h][d] = word[h];
+                    if (a.unprocessed)
+                        *reinterpret_cast<uint32_t*>(a.unprocessed + (size_t(t0) * 64 + b * GP + 2 * r4 + row) * row_bytes
+                            + size_t(c0) * BITS / 8 + 4 * h)
+                            = word[h] ^ kSigned;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < BITS / 4; ++h)
+                if constexpr (BITS == 4)
+                    transpose_nibbles(w[h]);
+                else
+                    transpose_bytes(w[h]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *place(b, r4, cv, h) = make_uint4(w[4 * h / E][4 * h % E], w[4 * h / E][4 * h % E + 1], w[4 * h / E][4 * h % E + 2],
+                    w[4 * h / E][4 * h % E + 3]);
+        }
+    }
+    __syncthreads();
+    // ---- store: a thread takes the four registers of a block of four columns; neighbouring blocks in one warp
+    // make whole 32-byte sectors
+    if (inside)
+    {
+        size_t const regs_per_irow = size_t(a.K / E) * IL;
+        for (int u = tid / NV; u < blocks * 2; u += int(blockDim.x) / NV)
+        {
+            int const b = (u & 1) | ((u >> 2) << 1), h = (u >> 1) & 1; // (a 64-row tile has an even number of blocks)
+            uint4 r[4];
+#pragma unroll
+            for (int r4 = 0; r4 < 4; ++r4)
+                r[r4] = *place(b, r4, cv, h);
+            int const col = c0 + 4 * h, k_tile = t0 + b / (64 / GP), vr = 4 * (b % (64 / GP));
+            uint32_t* dst = a.out + size_t(col / IL) * regs_per_irow + size_t(k_tile) * 32 + vr;
+            *reinterpret_cast<uint4*>(dst) = make_uint4(r[0].x, r[1].x, r[2].x, r[3].x);
+            *reinterpret_cast<uint4*>(dst + VT) = make_uint4(r[0].y, r[1].y, r[2].y, r[3].y);
+            dst += BITS == 4 ? 2 * VT : regs_per_irow; // int8: columns 2 and 3 are the next interleaved row
+            *reinterpret_cast<uint4*>(dst) = make_uint4(r[0].z, r[1].z, r[2].z, r[3].z);
+            *reinterpret_cast<uint4*>(dst + VT) = make_uint4(r[0].w, r[1].w, r[2].w, r[3].w);
+        }
+    }
+}
+
+// How a strip is cut: CTAs of its cluster, and bytes of a row. The slab of a CTA should stay below 72 KB, so
+// that three share an SM: 128-byte rows and eight CTAs to 4608 rows, half as wide strips to 9216, sixteen
+// CTAs beyond (only 112 SMs can form such clusters). cluster 0: K is too long for shared memory.
+struct StripShape
+{
+    int cluster, bytes;
+};
+
+StripShape strip_shape(int k)
+{
+    int const tiles = k / 64;
+    int c = 8;
+    while (c > 1 && c > tiles)
+        c /= 2;
+    if (tiles <= 8 * 9)
+        return {c, 128};
+    if (tiles <= 8 * 18)
+        return {8, 64};
+    return {tiles <= 16 * kMaxStripTiles ? 16 : 0, 64};
+}
+
+template <typename W, int BITS, int kStripBytes>
+int launch_strips(StripArgs a, W const* w, int cluster, cudaStream_t stream)
+{
+    constexpr int S = kStripBytes / int(sizeof(W)), NV = S / 8, GP = 128 / BITS;
+    DeviceInfo const& dev = current_device_info();
+    CUtensorMap tm;
+    CUtensorMapDataType const dt = sizeof(W) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16;
+    if (!make_tensor_map_2d(&tm, dt, w, uint64_t(a.N), uint64_t(a.K), uint64_t(a.N) * sizeof(W), S, 64, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return W4_ERR_CUDA;
+    auto kernel = strip_quantize_kernel<W, BITS, kStripBytes>;
+    {
+        static std::mutex mu;
+        static bool configured[64] = {};
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev.device < 0 || dev.device >= 64 || !configured[dev.device])
+        {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStripSmem)
+                    != cudaSuccess
+                || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+                return W4_ERR_CUDA;
+            if (dev.device >= 0 && dev.device < 64)
+                configured[dev.device] = true;
+        }
+    }
+    a.tiles_cta = (a.K / 64 + cluster - 1) / cluster;
+    int const units = a.tiles_cta * (64 / GP) * 4 * NV;
+    int const threads = std::max(64, std::min(units, kMaxStripThreads)); // units: a multiple of 64
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned((a.N + S - 1) / S * cluster));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = size_t(a.tiles_cta) * 64 * kStripBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = unsigned(cluster);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, a, tm) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
+}
+
 bool shape_ok(long k, long n, int bits)
 {
     return k > 0 && n > 0 && k % 64 == 0 && (n * bits / 8) % 32 == 0 && (k * bits / 8) % 32 == 0
@@ -377,6 +811,16 @@ template <typename W>
 int quantize_typed(void* processed, void* unprocessed, float* scales, void* scales_t, int scales_dtype, W const* w,
     int k, int n, int bits, cudaStream_t stream)
 {
+    StripShape const shape = strip_shape(k);
+    if (shape.cluster)
+    {
+        StripArgs const a{static_cast<uint32_t*>(processed), static_cast<uint8_t*>(unprocessed), scales, scales_t,
+            scales_dtype, k, n, 0};
+        if (shape.bytes == 128)
+            return bits == 4 ? launch_strips<W, 4, 128>(a, w, shape.cluster, stream) : launch_strips<W, 8, 128>(a, w, shape.cluster, stream);
+        return bits == 4 ? launch_strips<W, 4, 64>(a, w, shape.cluster, stream) : launch_strips<W, 8, 64>(a, w, shape.cluster, stream);
+    }
+    // more rows than a cluster's shared memory holds: maxima first, then quantise
     if (cudaMemsetAsync(scales, 0, size_t(n) * sizeof(float), stream) != cudaSuccess)
         return W4_ERR_CUDA;
     dim3 const ga((n + kAmaxVecs * 8 - 1) / (kAmaxVecs * 8), (k + kAmaxRows - 1) / kAmaxRows);
