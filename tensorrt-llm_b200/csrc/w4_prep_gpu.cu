@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kThreads)
 // memory by TMA, finds their column maxima as the 64-row boxes land, the cluster combines the maxima through
 // distributed shared memory, and the weights are quantised and laid out straight from shared memory.
 // HBM-bound: each weight is read from memory once (the two passes of the kernels below read it twice, and
-// scales were a memset, an atomic merge and a launch in between). 4096 x 14336 bf16 -> int4: 98 -> QUS us
+// scales were a memset, an atomic merge and a launch in between). 4096 x 14336 bf16 -> int4: 98 -> 56 us
 // per call. A thread turns one block of 32 (int4) / 16 (int8) rows x 8 columns - what four adjacent output
 // registers of each column hold - so all its stores are 16 bytes and a warp writes whole 32-byte sectors.
 // Several CTAs share an SM, so that one's arithmetic covers another's loads.
@@ -477,10 +477,11 @@ __device__ __noinline__ float quantize_exact(float x, float s)
 }
 
 // Scales of a thread's eight columns and what the arithmetic needs of them.
+template <typename W>
 struct StripScales
 {
-    float s[8], inv[8], half[8]; // half: s / 2, or 1 for a zero column
-    bool extreme;                // some scale is near underflow or overflow: divide
+    float s[8], inv[8];
+    bool extreme; // some scale is near underflow or overflow: divide
     __device__ __forceinline__ void load(float const* scale)
     {
         extreme = false;
@@ -489,48 +490,70 @@ struct StripScales
         {
             s[e] = scale[e];
             extreme |= s[e] != 0.f && !(s[e] > 1e-30f && s[e] < 1e30f);
-            inv[e] = s[e] != 0.f ? __fdiv_rn(1.f, s[e]) : 0.f;
-            half[e] = s[e] != 0.f ? 0.5f * s[e] : 1.f;
+            inv[e] = s[e] != 0.f ? __fdiv_rn(1.f, s[e]) : 0.f; // 0 for a zero column: every q is 0 there
+            if constexpr (!std::is_same<W, float>::value)
+                inv[e] *= 1.f + 0x1p-21f; // (see quantize8)
         }
     }
 };
 
-// round-half-away(fl(x / s)) by comparing |x| with the boundary instead of dividing (a product with the
-// reciprocal is not enough: a 16-bit weight in a thousand sits exactly on a boundary). m = the integer in
+// round-half-away(fl(x / s)) by comparing |x| with the boundary instead of dividing. m = the integer in
 // front of the boundary B = m + 1/2 next to |x / s|, from the rounded product with 1 / s - 1/2 (an error next
 // to an integer picks a neighbour's boundary, which gives the same result). The answer is m + 1 where
 // fl(|x| / s) >= B, that is where |x| / s >= B - u / 2 with u the spacing of the floats below B (the midpoint
-// rounds to B, whose mantissa is even). |x| - m s is exact near the boundary, elsewhere its size decides.
-// 16-bit weights: s is the largest times a power of two, so |x| - B s is zero or at least 2^-20 s and u / 2
-// plays no part. Eight instructions a weight, five of them on the float pipe.
-template <typename W, int BITS>
-__device__ __forceinline__ float quantize1(float x, float s, float inv, float half)
+// rounds to B, whose mantissa is even). |x| - B s is exact near the boundary, elsewhere its size decides.
+template <int BITS>
+__device__ __forceinline__ float quantize_boundary(float x, float s, float inv)
 {
     constexpr float kRound = 12582912.f; // 1.5 * 2^23: adding it rounds to an integer
     float const a = fabsf(x), m = (fmaf(a, inv, -0.5f) + kRound) - kRound;
-    float const t = fmaf(-m, s, a);
-    bool up = t >= half;
-    if constexpr (std::is_same<W, float>::value)
-    {
-        float const half_u = __uint_as_float((__float_as_uint(m + 0.5f) - 1u) & 0x7f800000u) * 0x1p-24f;
-        up = t - half >= -half_u * s;
-    }
-    float const q = m + (up ? 1.f : 0.f);
-    return fminf(copysignf(q, x), BITS == 8 ? 127.f : 7.f);
+    float const half_u = __uint_as_float((__float_as_uint(m + 0.5f) - 1u) & 0x7f800000u) * 0x1p-24f;
+    bool const up = fmaf(-m, s, a) - 0.5f * s >= -half_u * s && a > 0.f;
+    return fminf(copysignf(m + (up ? 1.f : 0.f), x), BITS == 8 ? 127.f : 7.f);
 }
 
+// Eight weights of a row: q = clamp(round-half-away(fl(x / s))).
+// 16-bit weights: s is the column's largest weight times a power of two, so x / s is either exactly a
+// half-integer or at least 2^-19 of its size away from one (the product of the odd integer 2B < 2^8 and an
+// 11-bit significand has 19 bits). A reciprocal that is 2^-21 too large puts the exact ones on the far side
+// and leaves the others, its own error and the product's below 2^-22, where they are: three instructions a
+// weight (dividing near the boundaries took as long as everything else, one 16-bit weight in a thousand
+// is on one).
+// fp32 weights: the product with the reciprocal decides wherever it is not within 1e-4 of a half-integer
+// (its error is 2.3e-5 at most; NaNs are not away from one), else the comparison above.
 template <typename W, int BITS>
-__device__ __forceinline__ void quantize8(float const (&x)[8], StripScales const& c, uint32_t (&word)[BITS / 4])
+__device__ __forceinline__ void quantize8(float const (&x)[8], StripScales<W> const& c, uint32_t (&word)[BITS / 4])
 {
+    constexpr float kRound = 12582912.f;
+    constexpr float kHi = BITS == 8 ? 127.f : 7.f;
     float q[8];
-    if (!c.extreme)
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            q[e] = quantize1<W, BITS>(x[e], c.s[e], c.inv[e], c.half[e]);
-    else
+    if (c.extreme)
+    {
 #pragma unroll
         for (int e = 0; e < 8; ++e)
             q[e] = quantize_exact<BITS>(x[e], c.s[e]);
+    }
+    else if constexpr (std::is_same<W, float>::value)
+    {
+        bool sure = true;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+        {
+            float const r = x[e] * c.inv[e], i = (r + kRound) - kRound;
+            sure &= fabsf(r - i) <= 0.4999f;
+            q[e] = fminf(i, kHi);
+        }
+        if (!sure)
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                q[e] = quantize_boundary<BITS>(x[e], c.s[e], c.inv[e]);
+    }
+    else
+    {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            q[e] = fminf(fmaf(x[e], c.inv[e], kRound), kRound + kHi) - kRound;
+    }
     pack_q<BITS>(q, word);
 }
 
@@ -673,7 +696,7 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     int const blocks = tiles * (64 / GP);
     if (inside)
     {
-        StripScales sc;
+        StripScales<W> sc;
         sc.load(scale_s + cv * 8);
 #pragma unroll 1
         for (int u = tid / NV; u < blocks * 4; u += int(blockDim.x) / NV)
@@ -739,13 +762,14 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
 
 // How a strip is cut: CTAs of its cluster, and bytes of a row. The slab of a CTA should stay below 72 KB, so
 // that three share an SM: 128-byte rows and eight CTAs to 4608 rows, half as wide strips to 9216, sixteen
-// CTAs beyond (only 112 SMs can form such clusters). cluster 0: K is too long for shared memory.
+// CTAs beyond. Only 112 SMs can form such clusters: 16-bit weights still gain (14336 x 4096 to int4 99 ->
+// 66 us), fp32 ones lose (to int8 116 -> 139 us). cluster 0: two passes.
 struct StripShape
 {
     int cluster, bytes;
 };
 
-StripShape strip_shape(int k)
+StripShape strip_shape(int k, int bytes_per_weight)
 {
     int const tiles = k / 64;
     int c = 8;
@@ -755,7 +779,7 @@ StripShape strip_shape(int k)
         return {c, 128};
     if (tiles <= 8 * 18)
         return {8, 64};
-    return {tiles <= 16 * kMaxStripTiles ? 16 : 0, 64};
+    return {bytes_per_weight == 2 && tiles <= 16 * kMaxStripTiles ? 16 : 0, 64};
 }
 
 template <typename W, int BITS, int kStripBytes>
@@ -811,7 +835,7 @@ template <typename W>
 int quantize_typed(void* processed, void* unprocessed, float* scales, void* scales_t, int scales_dtype, W const* w,
     int k, int n, int bits, cudaStream_t stream)
 {
-    StripShape const shape = strip_shape(k);
+    StripShape const shape = strip_shape(k, int(sizeof(W)));
     if (shape.cluster)
     {
         StripArgs const a{static_cast<uint32_t*>(processed), static_cast<uint8_t*>(unprocessed), scales, scales_t,
@@ -820,7 +844,7 @@ int quantize_typed(void* processed, void* unprocessed, float* scales, void* scal
             return bits == 4 ? launch_strips<W, 4, 128>(a, w, shape.cluster, stream) : launch_strips<W, 8, 128>(a, w, shape.cluster, stream);
         return bits == 4 ? launch_strips<W, 4, 64>(a, w, shape.cluster, stream) : launch_strips<W, 8, 64>(a, w, shape.cluster, stream);
     }
-    // more rows than a cluster's shared memory holds: maxima first, then quantise
+    // maxima first, then quantise
     if (cudaMemsetAsync(scales, 0, size_t(n) * sizeof(float), stream) != cudaSuccess)
         return W4_ERR_CUDA;
     dim3 const ga((n + kAmaxVecs * 8 - 1) / (kAmaxVecs * 8), (k + kAmaxRows - 1) / kAmaxRows);

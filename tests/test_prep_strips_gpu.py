@@ -1,0 +1,33 @@
+"""The one-pass device quantiser where its strips, clusters and rounding can go wrong (needs a B200)."""
+import pytest
+import torch
+
+from oracle import woq_oracle as o
+from tensorrt_llm_b200 import quantize as Q
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("k,n,dtype,bits", [
+    (64, 32, torch.float16, 8),        # one tile: a cluster of one; half a strip
+    (448, 96, torch.bfloat16, 8),      # seven tiles: a cluster of four, the last CTA short
+    (576, 64, torch.float32, 4),       # nine tiles on eight CTAs: some have none
+    (4672, 192, torch.bfloat16, 4),    # narrow strips
+    (4672, 96, torch.float32, 8),
+    (9280, 64, torch.float16, 8),      # clusters of sixteen
+    (9280, 64, torch.float32, 4),      # two passes
+])
+def test_strip_shapes(k, n, dtype, bits):
+    torch.manual_seed(k + n)
+    w = (torch.randn(k, n) * 0.02).to(dtype)
+    w[:, 5] = 0          # a zero column
+    w[:, 9] *= 1e-4      # (subnormal float16)
+    if dtype != torch.float16:
+        w[:, 11] *= 1e-33  # a scale too small for its reciprocal
+    w[k // 2, 13] = -4 * w[:, 13].abs().max()
+    u_ref, p_ref, s_ref = o.symmetric_quantize(w, bits)
+    u, p, s = Q.symmetric_quantize_last_axis_of_batched_matrix_cuda(
+        w.cuda(), torch.int8 if bits == 8 else torch.quint4x2, return_unprocessed=True)
+    assert torch.equal(s.cpu().float(), s_ref.float())
+    assert torch.equal(u.cpu(), u_ref)
+    assert torch.equal(p.cpu(), p_ref)
