@@ -191,16 +191,22 @@ __device__ __forceinline__ void tc_fence_after()
 // Keeping the surrounding control flow warp-uniform lets the compiler hold addresses and
 // descriptors in uniform registers, which is what the tensor-core and TMA instructions consume;
 // issued from inside a divergent `if (lane == 0)` every operand has to be moved across first.
-__device__ __forceinline__ void tc_mma_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc)
+__device__ __forceinline__ void tc_mma4_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc)
 {
+    // the four K = 16 instructions of 64 k: one election for all
     asm volatile(
         "{\n"
-        ".reg .pred p, pe;\n"
+        ".reg .pred p, pt, pe;\n"
         "elect.sync _|pe, 0xffffffff;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "setp.ne.b32 p, %10, 0;\n"
+        "setp.eq.b32 pt, 0, 0;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %5, %9, p;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%2], %6, %9, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%3], %7, %9, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%4], %8, %9, pt;\n"
         "}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
+        "r"(a_tmem), "r"(a_tmem + 8), "r"(a_tmem + 16), "r"(a_tmem + 24), "l"(b_desc), "l"(b_desc + 2), "l"(b_desc + 4),
+        "l"(b_desc + 6), "r"(idesc), "r"(acc)
         : "memory");
 }
 
@@ -516,17 +522,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     tc_fence_after();
                     uint64_t const desc = desc0 + uint64_t(s) * desc_stage;
                     uint32_t const a_col = a_ring + uint32_t(s) * kStageCols;
-                    tc_mma_ts_elect(d_tmem, a_col, desc, idesc, accumulate);
-                    tc_mma_ts_elect(d_tmem, a_col + 8, desc + 2, idesc, 1u);
-                    tc_mma_ts_elect(d_tmem, a_col + 16, desc + 4, idesc, 1u);
-                    tc_mma_ts_elect(d_tmem, a_col + 24, desc + 6, idesc, 1u);
+                    tc_mma4_ts_elect(d_tmem, a_col, desc, idesc, accumulate);
                     if (st * 128 + 64 < a.k)
-                    {
-                        tc_mma_ts_elect(d_tmem, a_col + 32, desc + desc_half, idesc, 1u);
-                        tc_mma_ts_elect(d_tmem, a_col + 40, desc + desc_half + 2, idesc, 1u);
-                        tc_mma_ts_elect(d_tmem, a_col + 48, desc + desc_half + 4, idesc, 1u);
-                        tc_mma_ts_elect(d_tmem, a_col + 56, desc + desc_half + 6, idesc, 1u);
-                    }
+                        tc_mma4_ts_elect(d_tmem, a_col + 32, desc + desc_half, idesc, 1u);
                     accumulate = 1u;
                     tc_commit_pair_elect(empty0 + 8 * s, both); // frees the activation stage and the TMEM stage
                     if (++s == a.num_stages)
@@ -560,94 +558,95 @@ __global__ void __launch_bounds__(kThreads, 1)
         int const w_row = n_local / IL;
         uint32_t const w_off = uint32_t(w_row * 128 + ((((n_local % IL) * SEG_CHUNKS) ^ (w_row & 7)) << 4));
 
-        int s = 0, ws = 0;
+        // Own steps are every kConvGroups-th, counted over all items; the rings run on from item to item.
+        int s = cgroup, ws = cgroup;
         uint32_t ph = 0;
         uint32_t w_seen = 0; // bit ws: parity of this group's next phase on w_full[cgroup][ws]
-        int turn = 0; // which group converts the next step
+        int skip = cgroup;   // steps from the start of the item to the next own step
         bool ok = true;
         for (int item = pair; item < num_items && ok; item += num_pairs)
         {
             int tile, split, st0, st1;
             item_range(item, tile, split, st0, st1);
-            for (int st = st0; st < st1; ++st)
+            int st = st0 + skip;
+            for (; st < st1; st += kConvGroups)
             {
-                if (turn == cgroup)
+                ok = wait_bar<false>(w_full0 + 8 * (cgroup * kMaxWStages + ws), (w_seen >> ws) & 1u, abort_flag);
+                if (!ok)
+                    break;
+                w_seen ^= 1u << ws;
+                uint8_t const* wst = smem + (w_ring - smem_base) + size_t(ws) * W_STAGE;
+                uint16_t const* sc = reinterpret_cast<uint16_t const*>(wst + W_BYTES) + n_local;
+                uint4 raw[2][SEG_CHUNKS];
+                uint32_t s2[2], z2[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
                 {
-                    ok = wait_bar<false>(w_full0 + 8 * (cgroup * kMaxWStages + ws), (w_seen >> ws) & 1u, abort_flag);
-                    if (!ok)
-                        break;
-                    w_seen ^= 1u << ws;
-                    uint8_t const* wst = smem + (w_ring - smem_base) + size_t(ws) * W_STAGE;
-                    uint16_t const* sc = reinterpret_cast<uint16_t const*>(wst + W_BYTES) + n_local;
-                    uint4 raw[2][SEG_CHUNKS];
-                    uint32_t s2[2], z2[2];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
+                    int const grow = h && a.group_shift == 6 ? 128 : 0;
+                    s2[h] = sc[grow];
+                    s2[h] = prmt(s2[h], s2[h], 0x1010u);
+                    if (HAS_ZERO)
                     {
-                        int const grow = h && a.group_shift == 6 ? 128 : 0;
-                        s2[h] = sc[grow];
-                        s2[h] = prmt(s2[h], s2[h], 0x1010u);
-                        if (HAS_ZERO)
-                        {
-                            z2[h] = sc[grow + 256];
-                            z2[h] = prmt(z2[h], z2[h], 0x1010u);
-                        }
-#pragma unroll
-                        for (int c = 0; c < SEG_CHUNKS; ++c)
-                            raw[h][c] = *reinterpret_cast<uint4 const*>(wst + h * LINE_TILE + (w_off ^ uint32_t(c << 4)));
+                        z2[h] = sc[grow + 256];
+                        z2[h] = prmt(z2[h], z2[h], 0x1010u);
                     }
-                    __syncwarp();
-                    if (lane == 0)
-                        arrive_local(w_empty0 + 8 * ws);
-                    uint32_t const a_col = lane_ring + uint32_t(s) * kStageCols;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                    {
-                        uint32_t v[32]; // TMEM columns of the half step: k = 2 * column (+1)
-#pragma unroll
-                        for (int c = 0; c < SEG_CHUNKS; ++c)
-                        {
-                            uint32_t const r[4] = {raw[h][c].x, raw[h][c].y, raw[h][c].z, raw[h][c].w};
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                            {
-                                // pair p of register j holds k = 32c + 2j + 8p (+1) (int4), 16c + 2j + 8p (+1) (int8)
-                                constexpr int PAIRS = BITS == 4 ? 4 : 2;
-                                uint32_t q[PAIRS];
-                                if constexpr (BITS == 4)
-                                    cvt_int4x8<T>(r[j], q);
-                                else
-                                    cvt_int8x4<T>(r[j], q);
-#pragma unroll
-                                for (int p = 0; p < PAIRS; ++p)
-                                    v[4 * PAIRS * c + j + 4 * p] = HAS_ZERO ? P::fma(q[p], s2[h], z2[h]) : P::mul(q[p], s2[h]);
-                            }
-                        }
-                        if (h == 0)
-                        {
-                            ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
-                            if (!ok)
-                                break;
-                            tc_fence_after();
-                        }
-                        tc_st32(a_col + 32 * h, v);
-                    }
-                    if (!ok)
-                        break;
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0)
-                        arrive_cluster_relaxed(lead_full0 + 8 * s);
+                    for (int c = 0; c < SEG_CHUNKS; ++c)
+                        raw[h][c] = *reinterpret_cast<uint4 const*>(wst + h * LINE_TILE + (w_off ^ uint32_t(c << 4)));
                 }
-                turn = turn + 1 == kConvGroups ? 0 : turn + 1;
-                ws = ws + 1 == a.num_wstages ? 0 : ws + 1;
-                if (++s == a.num_stages)
+                __syncwarp();
+                if (lane == 0)
+                    arrive_local(w_empty0 + 8 * ws);
+                uint32_t const a_col = lane_ring + uint32_t(s) * kStageCols;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
                 {
-                    s = 0;
+                    uint32_t v[32]; // TMEM columns of the half step: k = 2 * column (+1)
+#pragma unroll
+                    for (int c = 0; c < SEG_CHUNKS; ++c)
+                    {
+                        uint32_t const r[4] = {raw[h][c].x, raw[h][c].y, raw[h][c].z, raw[h][c].w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                        {
+                            // pair p of register j holds k = 32c + 2j + 8p (+1) (int4), 16c + 2j + 8p (+1) (int8)
+                            constexpr int PAIRS = BITS == 4 ? 4 : 2;
+                            uint32_t q[PAIRS];
+                            if constexpr (BITS == 4)
+                                cvt_int4x8<T>(r[j], q);
+                            else
+                                cvt_int8x4<T>(r[j], q);
+#pragma unroll
+                            for (int p = 0; p < PAIRS; ++p)
+                                v[4 * PAIRS * c + j + 4 * p] = HAS_ZERO ? P::fma(q[p], s2[h], z2[h]) : P::mul(q[p], s2[h]);
+                        }
+                    }
+                    if (h == 0)
+                    {
+                        ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
+                        if (!ok)
+                            break;
+                        tc_fence_after();
+                    }
+                    tc_st32(a_col + 32 * h, v);
+                }
+                if (!ok)
+                    break;
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    arrive_cluster_relaxed(lead_full0 + 8 * s);
+                ws += kConvGroups;
+                ws -= ws >= a.num_wstages ? a.num_wstages : 0;
+                s += kConvGroups;
+                if (s >= a.num_stages)
+                {
+                    s -= a.num_stages;
                     ph ^= 1;
                 }
             }
+            skip = st - st1;
         }
     }
     else if (warp < kEpiWarps)
