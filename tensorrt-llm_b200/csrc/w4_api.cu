@@ -251,7 +251,7 @@ bool decode_takes_tensor_cores(W4GemmParams const& p)
         return false;
     w4::DeviceInfo const& dev = w4::current_device_info();
     return dev.num_sms > 0
-        && w4::gemm_tc_plan(p.m, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 1.5
+        && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 1.5
         < regime_decode_us(p.m, p.n, p.k, p.weight_bits, p.act_dtype);
 }
 
@@ -502,6 +502,28 @@ extern "C"
         size_t const weight_bytes = size_t(p->k) * p->n * p->weight_bits / 8;
         auto at = [](const void* base, size_t bytes) -> const void*
         { return base ? static_cast<const char*>(base) + bytes : nullptr; };
+        // Two or more experts with rows and nothing to do in front: all in one launch of the tensor-core kernel,
+        // whose work items then fill the chip together (eight experts of 4096 x 14336 int4 with 4 to 19 rows:
+        // one after another 100 us, together 72 us). One expert, or a pre-quant scale: expert by expert.
+        int used = 0;
+        for (int e = 0; e < num_experts; ++e)
+            used += expert_first_row[e + 1] > expert_first_row[e];
+        if (used > 1 && !p->act_scale && p->regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO)
+        {
+            W4GemmParams q = *p;
+            q.m = expert_first_row[num_experts];
+            q.regime = W4_REGIME_GEMM;
+            int const rc = w4_gemm_validate(&q);
+            if (rc != W4_OK)
+            {
+                log_refusal("w4_gemm_launch_experts", p, rc);
+                return rc;
+            }
+            if (log_level() <= W4_LOG_DEBUG)
+                log_line(W4_LOG_DEBUG, "w4_gemm_launch_experts m=%d n=%d k=%d bits=%d group=%d experts=%d tensor-core kernel (chosen)",
+                    q.m, q.n, q.k, q.weight_bits, q.group_size, used);
+            return w4::launch_gemm_tc_experts(q, num_experts, expert_first_row, static_cast<cudaStream_t>(stream));
+        }
         for (int e = 0; e < num_experts; ++e)
         {
             int const row0 = expert_first_row[e], rows = expert_first_row[e + 1] - row0;

@@ -63,6 +63,7 @@ constexpr int kMmaWarp = kWProdWarp + 2;
 constexpr int kThreads = 32 * (kWProdWarp + 4);
 constexpr int kMaxStages = 8;      // activation / TMEM ring
 constexpr int kMaxWStages = 12;    // weight ring
+constexpr int kMaxExperts = 32;    // experts of one launch
 
 struct Args
 {
@@ -72,7 +73,13 @@ struct Args
     int m, n, k;
     int group_shift; // log2(group size), 31 = per-channel
     int bm;          // activation rows per tile
-    int tiles_n, tiles_m;
+    int tiles_n;
+    // Experts (an ordinary GEMM is one): expert e has rows first_row[e] .. first_row[e + 1] - 1 of the
+    // activations and of the output, tiles first_tile[e] .. first_tile[e + 1] - 1, the weights, scales and zeros
+    // of slice slice[e] of their tensors, and bias + slice[e] * n.
+    int num_experts;
+    int groups; // scale rows per expert
+    int first_row[kMaxExperts + 1], first_tile[kMaxExperts + 1], slice[kMaxExperts];
     int num_stages, num_wstages;
     int d_bufs;      // accumulators in TMEM: 2 up to 128 rows, else 1
     int weights_static;
@@ -334,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // Work items: (tile, split), splits adjacent. With SPLIT_CLUSTER a pair has exactly one: the grid is one
     // cluster per tile and a pair's rank in it is its split.
     int const pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    int const num_items = a.tiles_n * a.tiles_m * (SPLIT != SPLIT_NONE ? a.splits : 1);
+    int const num_items = a.first_tile[a.num_experts] * (SPLIT != SPLIT_NONE ? a.splits : 1);
     int const steps_all = (a.k + 127) >> 7; // the second half of the last step may lie past k: zeros, not multiplied
 
     bool const aligned = (smem_base & 1023u) == 0; // never false; the check keeps a wrong layout from being read
@@ -380,13 +387,29 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t const full0 = smem_u32(&bars->full[0]), empty0 = smem_u32(&bars->empty[0]);
     uint32_t const w_full0 = smem_u32(&bars->w_full[0][0]), w_empty0 = smem_u32(&bars->w_empty[0]);
 
-    // k range of a work item, in steps
-    auto item_range = [&](int item, int& tile, int& split, int& st0, int& st1)
+    struct Item
     {
-        tile = SPLIT != SPLIT_NONE ? item / a.splits : item;
-        split = SPLIT != SPLIT_NONE ? item - tile * a.splits : 0;
-        st0 = split * a.steps_split;
-        st1 = SPLIT != SPLIT_NONE ? min(steps_all, st0 + a.steps_split) : steps_all;
+        int n0;             // first column of the pair's tile
+        int row0, row_end;  // rows of the tile, and the end of the expert's
+        int slice, split;
+        int st0, st1;       // k steps
+    };
+    auto item_of = [&](int item)
+    {
+        Item it;
+        int const tile = SPLIT != SPLIT_NONE ? item / a.splits : item;
+        it.split = SPLIT != SPLIT_NONE ? item - tile * a.splits : 0;
+        it.st0 = it.split * a.steps_split;
+        it.st1 = SPLIT != SPLIT_NONE ? min(steps_all, it.st0 + a.steps_split) : steps_all;
+        int e = 0;
+        while (e + 1 < a.num_experts && tile >= a.first_tile[e + 1])
+            ++e;
+        int const t = tile - a.first_tile[e], tm = t / a.tiles_n;
+        it.n0 = (t - tm * a.tiles_n) * kPairN;
+        it.row0 = a.first_row[e] + tm * a.bm;
+        it.row_end = a.first_row[e + 1];
+        it.slice = a.slice[e];
+        return it;
     };
 
     if (!aligned)
@@ -414,18 +437,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int item = pair; item < num_items && ok; item += num_pairs)
         {
-            int tile, split, st0, st1;
-            item_range(item, tile, split, st0, st1);
-            int const n0 = (tile % a.tiles_n) * kPairN + int(rank) * BN;
-            for (int st = st0; st < st1; ++st)
+            Item const it = item_of(item);
+            int const n0 = it.n0 + int(rank) * BN, w_row = it.slice * (a.n / IL) + n0 / IL, s_row = it.slice * a.groups;
+            for (int st = it.st0; st < it.st1; ++st)
             {
                 ok = wait_bar<false>(w_empty0 + 8 * s, ph ^ 1, abort_flag);
                 if (!ok)
                     break;
                 uint32_t const dst = w_ring + uint32_t(s) * W_STAGE, bar = w_full0 + 8 * (turn * kMaxWStages + s);
-                int const g = a.group_shift >= 31 ? 0 : (st << 7) >> a.group_shift;
+                int const g = s_row + (a.group_shift >= 31 ? 0 : (st << 7) >> a.group_shift);
                 elect_expect_tx(bar, tx);
-                elect_tma_load_3d(dst, &tm_w, 0, n0 / IL, 2 * st, bar);
+                elect_tma_load_3d(dst, &tm_w, 0, w_row, 2 * st, bar);
                 elect_tma_load_2d(dst + W_BYTES, &tm_s, n0, g, bar);
                 if (HAS_ZERO)
                     elect_tma_load_2d(dst + W_BYTES + 512, &tm_z, n0, g, bar);
@@ -451,10 +473,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int item = pair; item < num_items && ok; item += num_pairs)
         {
-            int tile, split, st0, st1;
-            item_range(item, tile, split, st0, st1);
-            int const row0 = (tile / a.tiles_n) * a.bm + int(rank) * (a.bm >> 1);
-            for (int st = st0; st < st1; ++st)
+            Item const it = item_of(item);
+            int const row0 = it.row0 + int(rank) * (a.bm >> 1);
+            for (int st = it.st0; st < it.st1; ++st)
             {
                 ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
                 if (!ok)
@@ -499,12 +520,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t ph = 0;
             bool ok = true;
             uint32_t dph = 0; // bit b: parity of accumulator b's next drain
-            int db = 0, it = 0;
-            for (int item = pair; item < num_items && ok; item += num_pairs, ++it)
+            int db = 0, done = 0;
+            for (int item = pair; item < num_items && ok; item += num_pairs, ++done)
             {
-                int tile, split, st0, st1;
-                item_range(item, tile, split, st0, st1);
-                if (it >= a.d_bufs)
+                Item const it = item_of(item);
+                if (done >= a.d_bufs)
                 {
                     ok = wait_bar<true>(d_empty0 + 8 * db, (dph >> db) & 1u, abort_flag);
                     if (!ok)
@@ -514,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 uint32_t const d_tmem = tmem + uint32_t(db * a.bm);
                 uint32_t accumulate = 0;
-                for (int st = st0; st < st1; ++st)
+                for (int st = it.st0; st < it.st1; ++st)
                 {
                     ok = wait_bar<true>(full0 + 8 * s, ph, abort_flag);
                     if (!ok)
@@ -538,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 db = db + 1 == a.d_bufs ? 0 : db + 1;
             }
             // stay until the other CTA's last arrivals have landed
-            for (int i = 0; i < a.d_bufs && i < it && ok; ++i)
+            for (int i = 0; i < a.d_bufs && i < done && ok; ++i)
             {
                 db = db == 0 ? a.d_bufs - 1 : db - 1;
                 ok = wait_bar<true>(d_empty0 + 8 * db, (dph >> db) & 1u, abort_flag);
@@ -566,10 +586,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int item = pair; item < num_items && ok; item += num_pairs)
         {
-            int tile, split, st0, st1;
-            item_range(item, tile, split, st0, st1);
-            int st = st0 + skip;
-            for (; st < st1; st += kConvGroups)
+            Item const it = item_of(item);
+            int st = it.st0 + skip;
+            for (; st < it.st1; st += kConvGroups)
             {
                 ok = wait_bar<false>(w_full0 + 8 * (cgroup * kMaxWStages + ws), (w_seen >> ws) & 1u, abort_flag);
                 if (!ok)
@@ -646,7 +665,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     ph ^= 1;
                 }
             }
-            skip = st - st1;
+            skip = st - it.st1;
         }
     }
     else if (warp < kEpiWarps)
@@ -661,23 +680,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int item = pair; item < num_items && ok; item += num_pairs)
         {
-            int tile, split, st0, st1;
-            item_range(item, tile, split, st0, st1);
-            int const n = (tile % a.tiles_n) * kPairN + int(rank) * BN + warp * 32 + lane;
+            Item const it = item_of(item);
+            int const n = it.n0 + int(rank) * BN + warp * 32 + lane;
             bool const n_ok = n < a.n; // n is a multiple of 32: uniform over the warp
-            int const m0 = (tile / a.tiles_n) * a.bm;
-            float const bias_f = (SPLIT == SPLIT_NONE && bias && n_ok) ? P::to_float(bias[n]) : 0.f;
+            int const m0 = it.row0;
+            float const bias_f = (SPLIT == SPLIT_NONE && bias && n_ok) ? P::to_float(bias[size_t(it.slice) * a.n + n]) : 0.f;
             ok = wait_bar<false>(d_full0 + 8 * db, (dph >> db) & 1u, abort_flag);
             if (!ok)
                 break;
             dph ^= 1u << db;
             tc_fence_after();
-            float* part = SPLIT == SPLIT_WORKSPACE ? a.partial + size_t(split) * a.m * a.n + n : nullptr;
+            float* part = SPLIT == SPLIT_WORKSPACE ? a.partial + size_t(it.split) * a.m * a.n + n : nullptr;
             // two rows at a time: neighbouring lanes exchange halves, so that the even lane stores columns
             // n, n + 1 of the first row and the odd lane columns n - 1, n of the second
             uint16_t* out = static_cast<uint16_t*>(a.out) + (n & ~1);
             uint32_t const sel = lane & 1 ? 0x3276u : 0x5410u;
-            int const c_end = min(a.bm, a.m - m0);
+            int const c_end = min(a.bm, it.row_end - m0);
 #pragma unroll 1
             for (int c0 = 0; c0 < c_end; c0 += 32)
             {
@@ -707,7 +725,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     // fp32 partial tile; splitk_reduce_kernel, next on the stream, adds the partial tiles in
                     // split order (deterministic) and writes the output
                     float* dst = part + size_t(m0 + c0) * a.n;
-                    int const rows = a.m - m0 - c0;
+                    int const rows = it.row_end - m0 - c0;
 #pragma unroll
                     for (int j = 0; j < 32; ++j, dst += a.n)
                         if (j < rows)
@@ -725,10 +743,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
                         o[j] = prmt(o[j], __shfl_xor_sync(0xffffffffu, o[j], 1), sel);
-                    int const mrow = m0 + c0 + (lane & 1), rows = a.m - mrow; // this lane's rows: mrow, mrow + 2, ..
+                    int const mrow = m0 + c0 + (lane & 1), rows = it.row_end - mrow; // this lane's rows: mrow, mrow + 2, ..
                     uint16_t* dst = out + size_t(mrow) * a.n;
                     size_t const two_rows = size_t(a.n) * 2;
-                    if (m0 + c0 + 32 <= a.m)
+                    if (m0 + c0 + 32 <= it.row_end)
                     {
 #pragma unroll
                         for (int j = 0; j < 16; ++j, dst += two_rows)
@@ -758,15 +776,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     {
         // Every CTA adds the rows row % splits == its split of its 128 columns: a warp per row, four columns
         // per lane, the other splits' values from their shared memory.
-        int const tile = pair / a.splits, split = pair - tile * a.splits;
-        int const m0 = (tile / a.tiles_n) * a.bm, rows = min(a.bm, a.m - m0);
-        int const n = (tile % a.tiles_n) * kPairN + int(rank) * BN + 4 * lane;
+        Item const it = item_of(pair);
+        int const split = it.split, m0 = it.row0, rows = min(a.bm, it.row_end - m0);
+        int const n = it.n0 + int(rank) * BN + 4 * lane;
         if (n < a.n) // n is a multiple of 32
         {
             float b[4] = {0.f, 0.f, 0.f, 0.f};
             if (a.bias)
             {
-                uint2 const bw = *reinterpret_cast<uint2 const*>(static_cast<uint16_t const*>(a.bias) + n);
+                uint2 const bw = *reinterpret_cast<uint2 const*>(static_cast<uint16_t const*>(a.bias) + size_t(it.slice) * a.n + n);
                 P::unpack2(bw.x, b[0], b[1]);
                 P::unpack2(bw.y, b[2], b[3]);
             }
@@ -891,8 +909,16 @@ static int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t sm
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
 }
 
+// The experts of a launch: those of `slices` that have rows.
+struct Experts
+{
+    int num, slices;
+    int slice[kMaxExperts], first_row[kMaxExperts + 1];
+};
+
 template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
-static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream, TcPlan const& plan)
+static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream,
+    TcPlan const& plan)
 {
     constexpr int IL = BITS == 4 ? 4 : 2;
     constexpr int W_STAGE = 2 * (BN / IL) * 128 + 1024;
@@ -908,7 +934,15 @@ static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& 
     a.group_shift = p.group_size == 64 ? 6 : (p.group_size == 128 ? 7 : 31);
     a.bm = plan.bm;
     a.tiles_n = (p.n + kPairN - 1) / kPairN;
-    a.tiles_m = (p.m + plan.bm - 1) / plan.bm;
+    a.groups = p.group_size ? p.k / p.group_size : 1;
+    a.num_experts = ex.num;
+    for (int e = 0; e < ex.num; ++e)
+    {
+        a.slice[e] = ex.slice[e];
+        a.first_row[e] = ex.first_row[e];
+        a.first_tile[e + 1] = a.first_tile[e] + (ex.first_row[e + 1] - ex.first_row[e] + plan.bm - 1) / plan.bm * a.tiles_n;
+    }
+    a.first_row[ex.num] = ex.first_row[ex.num];
     a.weights_static = (p.flags & W4_GEMM_WEIGHTS_STATIC) ? 1 : 0;
     a.splits = plan.splits;
     a.steps_split = plan.steps_split;
@@ -940,10 +974,10 @@ static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& 
     if (!make_tensor_map_2d(&tm_act, dt, act, uint64_t(p.k), uint64_t(p.m), uint64_t(p.k) * 2, 64, uint32_t(plan.bm / 2),
             CU_TENSOR_MAP_SWIZZLE_128B))
         return W4_ERR_CUDA;
-    if (!make_tensor_map_3d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.weight, 128, uint64_t(p.n / IL), uint64_t(p.k / 64),
+    if (!make_tensor_map_3d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.weight, 128, uint64_t(p.n / IL) * ex.slices, uint64_t(p.k / 64),
             uint64_t(p.k) * 2, 128, 128, BN / IL, 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return W4_ERR_CUDA;
-    uint64_t const groups = p.group_size ? uint64_t(p.k / p.group_size) : 1;
+    uint64_t const groups = uint64_t(a.groups) * ex.slices;
     uint32_t const box_rows = p.group_size == 64 ? 2 : 1;
     if (!make_tensor_map_2d(&tm_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.scales, uint64_t(p.n), groups, uint64_t(p.n) * 2, BN,
             box_rows, CU_TENSOR_MAP_SWIZZLE_NONE))
@@ -969,7 +1003,7 @@ static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& 
                 configured[dev.device] = true;
         }
     }
-    int const items = a.tiles_n * a.tiles_m * a.splits;
+    int const items = a.first_tile[ex.num] * a.splits;
     int const pairs = SPLIT == SPLIT_CLUSTER || items < dev.num_sms / 2 ? items : dev.num_sms / 2;
     int rc = launch_pdl(kernel, 2 * pairs, kThreads, smem, SPLIT == SPLIT_CLUSTER ? 2 * a.splits : 2, stream, a, tm_act, tm_w,
         tm_s, tm_z);
@@ -983,29 +1017,30 @@ static int launch_one(W4GemmParams const& p, void const* act, DeviceInfo const& 
 }
 
 template <typename T, int BITS, bool HAS_ZERO>
-static int dispatch_split(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream)
+static int dispatch_split(W4GemmParams const& p, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream)
 {
-    TcPlan plan = gemm_tc_plan(p.m, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, true);
-    if (plan.splits > 1 && plan.cluster)
-        return launch_one<T, BITS, HAS_ZERO, SPLIT_CLUSTER>(p, act, dev, stream, plan);
-    if (plan.splits > 1)
-    {
-        // this form of split-k needs room for the partial tiles in the caller's workspace
-        size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
-        if (p.workspace && p.workspace_bytes >= act_copy + split_bytes(p.m, p.n, plan.splits))
-            return launch_one<T, BITS, HAS_ZERO, SPLIT_WORKSPACE>(p, act, dev, stream, plan);
-        plan = gemm_tc_plan(p.m, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false);
-    }
-    return launch_one<T, BITS, HAS_ZERO, SPLIT_NONE>(p, act, dev, stream, plan);
+    int rows[kMaxExperts];
+    for (int e = 0; e < ex.num; ++e)
+        rows[e] = ex.first_row[e + 1] - ex.first_row[e];
+    // the form of split-k that uses the caller's workspace needs room for the partial tiles there (and adds
+    // one bias)
+    size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
+    TcPlan plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, ex.num == 1);
+    if (plan.splits > 1 && !plan.cluster && (!p.workspace || p.workspace_bytes < act_copy + split_bytes(p.m, p.n, plan.splits)))
+        plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false);
+    if (plan.splits == 1)
+        return launch_one<T, BITS, HAS_ZERO, SPLIT_NONE>(p, act, ex, dev, stream, plan);
+    return plan.cluster ? launch_one<T, BITS, HAS_ZERO, SPLIT_CLUSTER>(p, act, ex, dev, stream, plan)
+                        : launch_one<T, BITS, HAS_ZERO, SPLIT_WORKSPACE>(p, act, ex, dev, stream, plan);
 }
 
 template <typename T>
-static int dispatch(W4GemmParams const& p, void const* act, DeviceInfo const& dev, cudaStream_t stream)
+static int dispatch(W4GemmParams const& p, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream)
 {
     bool const z = p.zeros != nullptr;
     if (p.weight_bits == 4)
-        return z ? dispatch_split<T, 4, true>(p, act, dev, stream) : dispatch_split<T, 4, false>(p, act, dev, stream);
-    return z ? dispatch_split<T, 8, true>(p, act, dev, stream) : dispatch_split<T, 8, false>(p, act, dev, stream);
+        return z ? dispatch_split<T, 4, true>(p, act, ex, dev, stream) : dispatch_split<T, 4, false>(p, act, ex, dev, stream);
+    return z ? dispatch_split<T, 8, true>(p, act, ex, dev, stream) : dispatch_split<T, 8, false>(p, act, ex, dev, stream);
 }
 
 // Clusters of 2 * splits CTAs the current device runs side by side: fixed by how its SMs are grouped.
@@ -1066,16 +1101,21 @@ static double step_us(int bm, int bits, int act_dtype)
 // (clusters of 4 and 8 CTAs about 1 us; 6 and more than 8 wait longer for enough free SMs side by side), splits
 // through the workspace a second kernel and their traffic. Fitted to 4096 and 8192 x 1024..14336 at 16 to
 // 777 rows: within 1 us of the best plan found by trying all at 14 of 16 points.
-TcPlan gemm_tc_plan(int m, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace)
+TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace)
 {
     int const pairs = num_sms > 1 ? num_sms / 2 : 1;
     int const steps = (k + 127) / 128;
     long const tiles_n = (n + tc::kPairN - 1) / tc::kPairN;
     TcPlan best{};
+    int m = 0; // most rows of an expert
+    for (int e = 0; e < experts; ++e)
+        m = m > rows[e] ? m : rows[e];
     int const most = m >= tc::kMaxBM ? tc::kMaxBM : (m + 31) & ~31;
     for (int bm = 32; bm <= most; bm += 32)
     {
-        long const tiles = tiles_n * ((m + bm - 1) / bm);
+        long tiles = 0;
+        for (int e = 0; e < experts; ++e)
+            tiles += tiles_n * ((rows[e] + bm - 1) / bm);
         double const step = step_us(bm, bits, act_dtype), drain = 0.01 * bm;
         int splits_max = m <= 256 && tiles < pairs ? int(pairs / tiles) : 1;
         splits_max = splits_max > 16 ? 16 : splits_max;
@@ -1108,7 +1148,7 @@ TcPlan gemm_tc_plan(int m, int n, int k, int num_sms, int bits, int act_dtype, b
 
 double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits, int act_dtype)
 {
-    return gemm_tc_plan(m, n, k, num_sms, bits, act_dtype, true).us;
+    return gemm_tc_plan(&m, 1, n, k, num_sms, bits, act_dtype, true).us;
 }
 
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale)
@@ -1124,7 +1164,7 @@ size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits,
     // forms that need none
     DeviceInfo const& dev = current_device_info();
     int const sms = dev.num_sms > 0 ? dev.num_sms : 148;
-    int const splits = gemm_tc_plan(m, n, k, sms, bits, act_dtype, true).splits;
+    int const splits = gemm_tc_plan(&m, 1, n, k, sms, bits, act_dtype, true).splits;
     size_t bytes = gemm_tc_workspace_min(m, k, has_act_scale);
     if (splits > 1)
         bytes = tc::split_align(bytes) + tc::split_bytes(m, n, splits);
@@ -1144,8 +1184,36 @@ int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream)
             return rc;
         act = p.workspace;
     }
-    return p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, act, dev, stream)
-                                        : tc::dispatch<__nv_bfloat16>(p, act, dev, stream);
+    tc::Experts const one{1, 1, {0}, {0, p.m}};
+    return p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, act, one, dev, stream)
+                                        : tc::dispatch<__nv_bfloat16>(p, act, one, dev, stream);
+}
+
+int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, cudaStream_t stream)
+{
+    DeviceInfo const& dev = current_device_info();
+    if (dev.num_sms <= 0)
+        return W4_ERR_CUDA;
+    tc::Experts ex{};
+    ex.slices = num_experts;
+    for (int e = 0; e < num_experts; ++e)
+    {
+        if (first_row[e + 1] > first_row[e])
+        {
+            ex.slice[ex.num] = e;
+            ex.first_row[ex.num] = first_row[e];
+            ex.first_row[++ex.num] = first_row[e + 1];
+        }
+        if (ex.num == tc::kMaxExperts || (e + 1 == num_experts && ex.num > 0))
+        {
+            int const rc = p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, p.act, ex, dev, stream)
+                                                        : tc::dispatch<__nv_bfloat16>(p, p.act, ex, dev, stream);
+            if (rc != W4_OK)
+                return rc;
+            ex.num = 0;
+        }
+    }
+    return W4_OK;
 }
 
 } // namespace w4

@@ -47,7 +47,10 @@ int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream);
 // Workspace: the minimum the kernel needs (scaled activation copy), and what also allows split-k.
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale);
 size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits, int act_dtype);
-// How the tensor-core kernel runs a problem: activation rows per tile, split-k factor and 128-wide k
+// The experts of a 3-D weight tensor in one launch (every 32 of those that have rows): p.m is the sum of the
+// rows, expert e has rows first_row[e] .. first_row[e + 1] - 1. No pre-quant scale, no workspace.
+int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, cudaStream_t stream);
+// How the tensor-core kernel runs a problem (or the experts of one, by their rows): activation rows per tile, split-k factor and 128-wide k
 // steps per work item, and the estimated duration (microseconds, from measured step costs); shared by the
 // launcher, the workspace size and the regime heuristic.
 struct TcPlan
@@ -58,7 +61,7 @@ struct TcPlan
     bool cluster = false; // the splits of a tile are one cluster (otherwise they meet in the workspace)
     double us = 0;
 };
-TcPlan gemm_tc_plan(int m, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace);
+TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace);
 double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits, int act_dtype);
 
 // out[m, k] = act[m, k] * scale[k], rounded to the element type (the reference's

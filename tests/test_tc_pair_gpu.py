@@ -43,3 +43,26 @@ def test_decode_regime_through_the_tensor_cores(m, n, k, bits):
     auto, decode = run_gpu(p), run_gpu(p, regime=pkg.W4_REGIME_GEMV)
     ref = oracle_out(p)
     assert max_err(auto, ref) <= oracle.tolerance(ref) and max_err(auto, decode) <= oracle.tolerance(ref)
+
+
+@pytest.mark.parametrize("bits,group,rows,k,n", [
+    (4, 128, [1] * 40, 256, 320),                # more experts than one launch holds; a pair tile half empty
+    (8, 0, [0, 33, 0, 1, 64, 300, 0], 576, 96),  # experts without rows, several row tiles, an odd half step
+    (4, 64, [5, 6], 4096, 256),                  # few tiles: cluster splits
+])
+def test_experts_in_one_launch(bits, group, rows, k, n):
+    full = group != 0
+    first = [0]
+    for r in rows:
+        first.append(first[-1] + r)
+    probs = [make_problem(max(r, 1), n, k, bits, group, torch.bfloat16, zero=full, bias=full, seed=e)
+             for e, r in enumerate(rows)]
+    act = torch.cat([p["act"][:r] for p, r in zip(probs, rows)]).cuda()
+    stack = lambda key: None if probs[0][key] is None else torch.stack([p[key] for p in probs]).cuda()
+    out = pkg.ops.moe_gemm(act, stack("processed"), stack("scales"), first, weight_bits=bits, group_size=group,
+                           zeros=stack("zeros"), bias=stack("bias"), alpha=0.5 if full else 1.0).cpu()
+    for e, (p, r) in enumerate(zip(probs, rows)):
+        if r:
+            ref = oracle_out(dict(p, act=p["act"][:r]), alpha=0.5 if full else 1.0)
+            assert max_err(out[first[e]:first[e + 1]], ref) <= oracle.tolerance(ref), e
+    assert pkg._lib.lib().w4_gemm_device_status() == 0
