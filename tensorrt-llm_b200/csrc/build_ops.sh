@@ -14,6 +14,6 @@ PY
 cuda_inc="${CUDA_HOME:-/usr/local/cuda}/include"
 g++ -std=c++17 -O2 -fPIC -shared -D_GLIBCXX_USE_CXX11_ABI="$abi" ${tinc//,/ } -I"$cuda_inc" \
     "$here/trtllm_ops.cpp" -o "$pkg/libtrtllm_ops.so" \
-    -L"$pkg" -lw4gemm -L"$tlib" -lc10 -lc10_cuda -ltorch_cpu -ltorch \
+    -L"$pkg" -lw4gemm -L"$tlib" -lc10 -lc10_cuda -ltorch_cpu -ltorch_cuda -ltorch \
     -Wl,-rpath,'$ORIGIN' -Wl,-rpath,"$tlib" -Wl,--no-as-needed
 echo "built $pkg/libtrtllm_ops.so"

@@ -16,11 +16,14 @@ namespace w4
 DeviceInfo const& current_device_info()
 {
     static DeviceInfo infos[64];
+    static std::atomic<bool> ready[64];
     static std::mutex mu;
     static DeviceInfo invalid;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
         return invalid;
+    if (ready[dev].load(std::memory_order_acquire))
+        return infos[dev];
     std::lock_guard<std::mutex> lock(mu);
     DeviceInfo& d = infos[dev];
     if (d.device != dev)
@@ -32,6 +35,7 @@ DeviceInfo const& current_device_info()
         d.num_sms = sms;
         d.max_smem_optin = smem;
         d.device = dev;
+        ready[dev].store(true, std::memory_order_release);
     }
     return d;
 }
@@ -45,6 +49,10 @@ template <typename T>
 __global__ void pre_quant_scale_kernel(uint4* out, uint4 const* act, uint4 const* scale, size_t total_vec, int k_vec)
 {
     using P = Pair<T>;
+    // programmatic dependent of what wrote the activations; the GEMM behind starts its own prologue (and
+    // fetches static weights) meanwhile
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     size_t const stride = size_t(gridDim.x) * blockDim.x;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vec; i += stride)
     {
@@ -72,13 +80,21 @@ int launch_pre_quant_scale(void* out, void const* act, void const* scale, int m,
         blocks = cap;
     if (blocks == 0)
         return W4_OK;
-    if (act_dtype == W4_DTYPE_FP16)
-        pre_quant_scale_kernel<__half><<<unsigned(blocks), threads, 0, stream>>>(static_cast<uint4*>(out),
-            static_cast<uint4 const*>(act), static_cast<uint4 const*>(scale), total_vec, k / 8);
-    else
-        pre_quant_scale_kernel<__nv_bfloat16><<<unsigned(blocks), threads, 0, stream>>>(static_cast<uint4*>(out),
-            static_cast<uint4 const*>(act), static_cast<uint4 const*>(scale), total_vec, k / 8);
-    return cudaGetLastError() == cudaSuccess ? W4_OK : W4_ERR_CUDA;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(blocks));
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto kernel = act_dtype == W4_DTYPE_FP16 ? pre_quant_scale_kernel<__half> : pre_quant_scale_kernel<__nv_bfloat16>;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<uint4*>(out), static_cast<uint4 const*>(act),
+               static_cast<uint4 const*>(scale), total_vec, k / 8)
+            == cudaSuccess
+        ? W4_OK
+        : W4_ERR_CUDA;
 }
 
 // Stages a small activation block from mapped pinned host memory into device memory: the loads cross

@@ -37,6 +37,7 @@
 // multicast to both CTAs: the step's activation stage and TMEM stage are free), `d_full` /
 // `d_empty` (accumulator).
 // All waits are bounded; a timeout sets the device status word and the CTAs drain and exit.
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -1043,21 +1044,23 @@ static int dispatch(W4GemmParams const& p, void const* act, Experts const& ex, D
     return z ? dispatch_split<T, 8, true>(p, act, ex, dev, stream) : dispatch_split<T, 8, false>(p, act, ex, dev, stream);
 }
 
-// Clusters of 2 * splits CTAs the current device runs side by side: fixed by how its SMs are grouped.
+// Clusters of 2 * splits CTAs the current device runs side by side, by splits: fixed by how its SMs are grouped.
 // Without a device, the numbers of a B200 with all 148 SMs.
-static int max_clusters(int splits)
+static int const* max_clusters()
 {
     struct Limits
     {
-        bool known = false;
+        std::atomic<bool> known{false};
         int clusters[kMaxClusterSplits + 1] = {0, 74, 33, 22, 15, 11, 7, 7, 7};
     };
     static std::mutex mu;
     static Limits devices[64], none;
     DeviceInfo const& dev = current_device_info();
-    std::lock_guard<std::mutex> lock(mu);
     Limits& l = dev.num_sms > 0 ? devices[dev.device] : none;
-    if (dev.num_sms > 0 && !l.known)
+    if (dev.num_sms <= 0 || l.known.load(std::memory_order_acquire))
+        return l.clusters;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!l.known.load(std::memory_order_relaxed))
     {
         auto kernel = gemm_kernel<__nv_bfloat16, 4, true, SPLIT_CLUSTER>;
         bool const ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin) == cudaSuccess
@@ -1078,9 +1081,9 @@ static int max_clusters(int splits)
             l.clusters[s] = ok && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
         }
         (void) cudaGetLastError(); // a cluster size the device refuses is no error of the caller's
-        l.known = true;
+        l.known.store(true, std::memory_order_release);
     }
-    return l.clusters[splits];
+    return l.clusters;
 }
 
 } // namespace tc
@@ -1106,6 +1109,7 @@ TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int
     int const pairs = num_sms > 1 ? num_sms / 2 : 1;
     int const steps = (k + 127) / 128;
     long const tiles_n = (n + tc::kPairN - 1) / tc::kPairN;
+    int const* const clusters = tc::max_clusters();
     TcPlan best{};
     int m = 0; // most rows of an expert
     for (int e = 0; e < experts; ++e)
@@ -1124,7 +1128,7 @@ TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int
             int const per = (steps + s - 1) / s;
             if ((steps + per - 1) / per != s || (s > 1 && per < 2))
                 continue; // an empty work item, or too little in each
-            bool const cluster = s > 1 && s <= tc::kMaxClusterSplits && tiles <= tc::max_clusters(s);
+            bool const cluster = s > 1 && s <= tc::kMaxClusterSplits && tiles <= clusters[s];
             if (s > 1 && !cluster && !may_use_workspace)
                 continue;
             double const waves = double((tiles * s + pairs - 1) / pairs);
