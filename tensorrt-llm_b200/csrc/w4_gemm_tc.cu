@@ -1093,12 +1093,12 @@ static int const* max_clusters()
 // (1024 tensor cycles at 256 rows).
 static double step_us(int bm, int bits, int act_dtype)
 {
-    double const conv = bits == 8 && act_dtype == W4_DTYPE_BF16 ? 0.35 : 0.27, mma = bm * (0.57 / 256);
+    double const conv = bits == 8 && act_dtype == W4_DTYPE_BF16 ? 0.33 : 0.25, mma = bm * (0.57 / 256);
     return conv > mma ? conv : mma;
 }
 
 // The plan with the shortest estimated time: row tiles in steps of 32 and, where the tiles leave pairs idle
-// (and only up to 256 rows, where the fp32 partial tiles stay small), split factors. A launch costs 2 us plus
+// (and only up to 256 rows, where the fp32 partial tiles stay small), split factors. A launch costs 2.5 us plus
 // the waves of its work items; an item's epilogue 0.3 us per 32 rows, of which the double-buffered
 // accumulators hide all but the last. Splits that share a cluster add the exchange of the partial tiles
 // (clusters of 4 and 8 CTAs about 1 us; 6 and more than 8 wait longer for enough free SMs side by side), splits
@@ -1132,7 +1132,7 @@ TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int
             if (s > 1 && !cluster && !may_use_workspace)
                 continue;
             double const waves = double((tiles * s + pairs - 1) / pairs);
-            double us = 2.0 + drain + waves * per * step + (waves - 1) * (bm <= 128 ? 0.1 : drain + 0.3);
+            double us = 2.5 + drain + waves * per * step + (waves - 1) * (bm <= 128 ? 0.1 : drain + 0.3);
             if (cluster)
                 us += (s == 2 || s == 4 ? 1.0 : 3.0) + 0.008 * bm;
             else if (s > 1)
@@ -1148,11 +1148,6 @@ TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int
         }
     }
     return best;
-}
-
-double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits, int act_dtype)
-{
-    return gemm_tc_plan(&m, 1, n, k, num_sms, bits, act_dtype, true).us;
 }
 
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale)

@@ -62,7 +62,6 @@ struct TcPlan
     double us = 0;
 };
 TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace);
-double gemm_tc_estimate_us(int m, int n, int k, int num_sms, int bits, int act_dtype);
 
 // out[m, k] = act[m, k] * scale[k], rounded to the element type (the reference's
 // apply_per_channel_scale, cpp/tensorrt_llm/kernels/preQuantScaleKernel.cu:43-95).
