@@ -258,34 +258,17 @@ double regime_prefill_us(int m, int n, int k, int num_sms, int weight_bits)
     return 7.0 + (splits > 1 ? 3.0 : 0.0) + waves(bm, splits) * step_us(bm) * double((steps + splits - 1) / splits);
 }
 
-// Microseconds of the decode kernel's passes as measured. Up to 8 rows: 3 us plus the weight bytes at
-// 4.1 (int4) or 3.6 TB/s (int8), 0.2 us per 1024 k beyond the first panel of 4096 (activations are reloaded),
-// 0.045 us per megabyte more above four rows and 0.15 of the total for 64-wide groups on int4 (weights are
-// rounded one by one). 16 rows as in regime_decode_us, int8 under float16 3 us plus the bytes at 3.6 TB/s.
-double decode_kernel_us(W4GemmParams const& p)
-{
-    double const mb = double(p.n) * double(p.k) * p.weight_bits / 8.0 / 1.0e6;
-    double us = 0;
-    int left = p.m;
-    for (; left > 8; left -= left < 16 ? left : 16)
-        us += p.weight_bits == 4 ? mb / 2.7 + 6.3 : (p.act_dtype == W4_DTYPE_BF16 ? mb / 3.1 + 5.0 : mb / 3.6 + 3.0);
-    if (left > 0)
-        us += 3.0 + mb / (p.weight_bits == 4 ? 4.1 : 3.6) + (left > 4 ? 0.045 * mb : 0.0)
-            + (p.k > 4096 ? 0.2 * (p.k - 4096) / 1024.0 : 0.0);
-    return p.weight_bits == 4 && p.group_size == 64 ? 1.15 * us : us;
-}
-
 // An automatic launch in the decode regime: the tensor-core kernel in the forms that need no workspace, where
 // its estimate is 1.5 us below the decode kernel's (whose launch also costs the host less). One row on
-// 4096 x 14336 int8 18.9 -> 14.5 us, eight rows on 14336 x 4096 int4 with 64-wide groups 13.9 -> 12.2, 16 rows
-// on 4096 x 14336 int4 17.2 -> 11.7; int4 at a few rows stays with the decode kernel (one row on 4096 x 14336
-// 10.4 against 11.8).
+// 4096 x 14336 int8 18.9 -> 14.5 us, six rows on 6144 x 24576 int4 with 64-wide groups 31.1 -> 24.6, 16 rows
+// on 4096 x 14336 int4 17.2 -> 11.7; int4 at a few rows stays with the decode kernels (one row on 4096 x 14336
+// 9.4 against 11.8).
 bool decode_takes_tensor_cores(W4GemmParams const& p)
 {
     if (p.act_scale)
         return false;
     w4::DeviceInfo const& dev = w4::current_device_info();
-    double const decode = decode_kernel_us(p);
+    double const decode = w4::gemv_estimate_us(p);
     return dev.num_sms > 0 && decode > 5.0
         && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 1.5 < decode;
 }

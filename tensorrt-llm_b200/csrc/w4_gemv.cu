@@ -1052,11 +1052,58 @@ static int dispatch_bits(Args const& a, int bits, int mb, DeviceInfo const& dev,
 
 } // namespace gemv
 
+// Microseconds of the passes of this file's kernel, as measured. Up to 8 rows: 3 us plus the weight bytes at
+// 4.1 (int4; k rounded up to panels of 4096, which a pass walks whatever they hold) or 3.6 TB/s (int8), 0.1 us
+// per 1024 k beyond the first panel (activations are reloaded), more above four rows and 15 % more for 64-wide
+// groups on int4 (weights are rounded one by one). 16 rows: int4 6.3 us plus the bytes at 2.7 TB/s, int8 3 us
+// at 3.6 TB/s, under bf16 activations 5 us at 3.1 TB/s (two nibble planes).
+static double staged_us(W4GemmParams const& p)
+{
+    bool const w4 = p.weight_bits == 4;
+    double const mb = double(p.n) * double(p.k) * p.weight_bits / 8.0 / 1.0e6;
+    double us = 0;
+    int left = p.m;
+    for (; left > 8; left -= left < 16 ? left : 16)
+        us += w4 ? mb / 2.7 + 6.3 : (p.act_dtype == W4_DTYPE_BF16 ? mb / 3.1 + 5.0 : mb / 3.6 + 3.0);
+    if (left > 0)
+    {
+        double const padded = w4 ? double((p.k + 4095) / 4096 * 4096) / p.k : 1.0, over = p.k > 4096 ? (p.k - 4096) / 1024.0 : 0.0;
+        us += 3.0 + mb * padded / (w4 ? 4.1 : 3.6) + (w4 ? 0.1 : 0.2) * over
+            + (left > 4 ? 0.003 * mb * (left - 4) * (left - 4) : 0.0);
+    }
+    return w4 && p.group_size == 64 ? 1.15 * us : us;
+}
+
+// The same of the streaming kernel: 2.9 us plus the bytes at 4.75 TB/s up to 42 MB and 5.6 TB/s beyond, and
+// 0.07 us per row and 1024 k for the activations, which every CTA lays out for itself before it starts (a
+// second panel when they do not fit costs another microsecond). Negative: not for this problem.
+static double streamed_us(W4GemmParams const& p)
+{
+    if (p.weight_bits != 4 || p.m > 8 || p.group_size == 64 || p.k % 128 != 0)
+        return -1.0;
+    double const mb = double(p.n) * double(p.k) / 2.0e6;
+    return 2.9 + (mb < 42.0 ? mb / 4.75 : 42.0 / 4.75 + (mb - 42.0) / 5.6) + 0.07 * p.m * (p.k / 1024.0)
+        + (p.m * p.k > 100000 ? 1.0 : 0.0);
+}
+
+double gemv_estimate_us(W4GemmParams const& p)
+{
+    double const a = staged_us(p), b = streamed_us(p);
+    return b > 0.0 && b < a ? b : a;
+}
+
 int launch_gemv(W4GemmParams const& p, cudaStream_t stream, PushTarget const* push)
 {
     DeviceInfo const& dev = current_device_info();
     if (dev.num_sms <= 0)
         return W4_ERR_CUDA;
+    double const streamed = push ? -1.0 : streamed_us(p);
+    if (streamed > 0.0 && streamed + 0.1 < staged_us(p))
+    {
+        int const rc = launch_gemv_stream(p, stream);
+        if (rc != W4_ERR_UNSUPPORTED)
+            return rc;
+    }
     size_t const elt = 2;
     // Passes over the weights: 16 rows at a time (two B fragments per weight fragment) while more
     // than 8 rows are left, then one pass of up to 8.

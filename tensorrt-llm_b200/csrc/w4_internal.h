@@ -38,6 +38,11 @@ struct PushTarget
     unsigned long long timeout_ns;
 };
 int launch_gemv(W4GemmParams const& p, cudaStream_t stream, PushTarget const* push = nullptr);
+// The decode kernel without staging, for int4 weights, 128-wide groups or none, whole 128-wide k units and up
+// to 8 rows (called by launch_gemv where it is the faster). W4_ERR_UNSUPPORTED: too many columns.
+int launch_gemv_stream(W4GemmParams const& p, cudaStream_t stream);
+// Estimated duration of launch_gemv (microseconds, from measurements).
+double gemv_estimate_us(W4GemmParams const& p);
 // Fills `t` for the one-shot packet protocol of this all-reduce call; false when the call would not
 // use that protocol (size, mode) or its arguments are not valid.
 bool allreduce_push_target(W4AllReduceParams const& r, PushTarget* t);

@@ -1,0 +1,38 @@
+"""The streaming decode kernel where its shares, tails and panels can go wrong (needs a B200)."""
+import pytest
+import torch
+
+import tensorrt_llm_b200 as pkg
+from oracle import woq_oracle as oracle
+from _cases import make_problem, max_err, oracle_subset, run_gpu, sample_cols
+
+pytestmark = pytest.mark.gpu
+
+
+# every one of these sizes is in the streaming kernel's range: few rows and k units that leave the staged
+# kernel's panels half empty, or many weights
+@pytest.mark.parametrize("m,n,k,group,dtype", [
+    (1, 8192, 2048, 128, torch.bfloat16),
+    (2, 8384, 2176, 128, torch.float16),    # odd number of units, ragged column ranges
+    (7, 8384, 2176, 0, torch.bfloat16),
+    (8, 12352, 1152, 128, torch.bfloat16),
+    (3, 9536, 4224, 128, torch.float16),    # one unit more than the staged kernel's panel
+    (5, 24640, 128, 0, torch.bfloat16),     # a single unit: most warps have no share of a column group
+    (6, 16384, 20480, 128, torch.bfloat16),  # two activation panels
+])
+def test_shares_tails_and_panels(m, n, k, group, dtype):
+    full = group != 0
+    p = make_problem(m, n, k, 4, group, dtype, zero=full, bias=full, prequant=full, seed=m + k)
+    if dtype == torch.bfloat16:  # values far outside float16's range, and zeros
+        p["act"][0] *= 2.0 ** 40
+        p["act"][-1, :130] = 0
+        if m > 1:
+            p["act"][1] *= 2.0 ** -60
+    alpha = 0.5 if full else 1.0
+    out = run_gpu(p, regime=pkg.W4_REGIME_GEMV, alpha=alpha)
+    cols = sample_cols(n, count=64)
+    for row in range(m):
+        ref = oracle_subset(p, [row], cols, alpha=alpha)
+        assert max_err(out[[row]][:, cols], ref) <= oracle.tolerance(ref), row
+    assert torch.equal(out, run_gpu(p, regime=pkg.W4_REGIME_GEMV, alpha=alpha))  # sums in a fixed order
+    assert pkg._lib.lib().w4_gemm_device_status() == 0
