@@ -47,7 +47,7 @@
  *                            - preprocess_weights_for_mixed_gemm with QuantType::W4_AFP8
  *                              (cutlass_preprocessors.cpp:114-116) and its conversion into the layout
  *                              the kernels consume (W4A8-AWQ layers).
- *   w4_gemm_launch_experts   - one GEMM per expert over 3-D weights
+ *   w4_gemm_launch_experts   - the GEMMs of all experts over 3-D weights
  *                              (cpp/tensorrt_llm/thop/weightOnlyQuantOp.cpp:136-147 lays them out).
  *   w4_gemm_run_host, w4_gemm_launch_static_scratch
  *                            - no counterpart: host buffers in and out; no workspace from the caller.
@@ -183,8 +183,9 @@ extern "C"
     int w4_gemm_run_host(const W4GemmParams* p, const void* host_act, void* host_out, void* stream);
 
     /*
-     * One GEMM per expert of a mixture-of-experts layer over 3-D weights, enqueued back to back on
-     * `stream`. p describes expert 0: weight is [E][K, N*bits/8], every expert's matrix laid out on its
+     * The GEMMs of all experts of a mixture-of-experts layer over 3-D weights: one launch of the
+     * tensor-core kernel for up to 32 experts with rows, or, with a pre-quant scale, a requested regime or
+     * rows for a single expert, one w4_gemm_launch after another. p describes expert 0: weight is [E][K, N*bits/8], every expert's matrix laid out on its
      * own - what preprocess_weights_for_mixed_gemm does with a 3-D tensor
      * (cpp/tensorrt_llm/thop/weightOnlyQuantOp.cpp:136-147, force_interleave); scales / zeros are
      * [E][K/G, N] (or [E][N]), bias [E][N]; act_scale [K] is shared. The rows of act and out are sorted
@@ -192,8 +193,8 @@ extern "C"
      * num_experts + 1 non-decreasing ints starting at 0; the running totals the reference's MoE GEMM
      * takes as total_tokens_including_expert,
      * cpp/tensorrt_llm/kernels/internal_cutlass_kernels/include/moe_gemm_kernels.h:236, kept on the host). p->m is ignored; the
-     * workspace must cover the largest per-expert row count (w4_gemm_workspace_bytes_max) and is
-     * reused by every expert. Experts without rows are skipped. Returns the first error.
+     * workspace is used expert by expert only and must then cover the largest per-expert row count
+     * (w4_gemm_workspace_bytes_max). Experts without rows are skipped. Returns the first error.
      */
     int w4_gemm_launch_experts(const W4GemmParams* p, int num_experts, const int* expert_first_row, void* stream);
 
