@@ -63,6 +63,7 @@ constexpr int kThreads = kConsumerThreads + 128; // + one producer warp group (o
 // gives its share back (setmaxnreg) and the consumer groups take it.
 constexpr int kProducerRegs = 24, kConsumerRegs = 112; // 128 * 24 + 512 * 112 <= 640 * 96 (the launch-time pool)
 constexpr int kRedBytes = 64 * 1024;            // shared memory for cross-warp partial sums
+constexpr int kRedBytesSmall = 52 * 1024;       // the same up to 6 rows (8 column groups at 6 rows)
 constexpr int kRedBytes16 = 112 * 1024;         // the same for 16-row passes (7 column groups)
 constexpr int kScaleBoxCols = 24;               // columns per scale/zero box: 16 + slack to start on a 16-byte boundary
 
@@ -904,9 +905,18 @@ static int launch_one(Args const& a, DeviceInfo const& dev, cudaStream_t stream)
     // barrier, and fewer of them measured faster than the two ring slots this costs (four slots
     // remain; ~72 KB are in flight at a time anyway).
     args.red_bytes = MB == 2 ? kRedBytes16 : kRedBytes;
-    size_t const fixed = size_t(args.red_bytes) + 64 + 1024; // + slack to start the ring on a 1024-byte boundary
-    // Shared memory per CTA: all a block may have.
-    size_t const smem_budget = size_t(dev.max_smem_optin);
+    size_t fixed = size_t(args.red_bytes) + 64 + 1024; // + slack to start the ring on a 1024-byte boundary
+    // Shared memory per CTA: all a block may have, or, where four slots and the sums of as many column groups
+    // still fit, what the streaming kernel leaves (kDecodeSmem).
+    size_t smem_budget = size_t(dev.max_smem_optin);
+    unsigned carveout = 100;
+    if (MB == 1 && a.m <= 6 && fixed - kRedBytes + kRedBytesSmall + 4 * size_t(args.slot_bytes + 16) <= kDecodeSmem)
+    {
+        args.red_bytes = kRedBytesSmall;
+        fixed += kRedBytesSmall - kRedBytes;
+        smem_budget = kDecodeSmem;
+        carveout = kDecodeCarveout;
+    }
     int slots = int((smem_budget - fixed) / (args.slot_bytes + 16));
     if (slots < 2)
         return W4_ERR_CUDA;
@@ -971,11 +981,13 @@ static int launch_one(Args const& a, DeviceInfo const& dev, cudaStream_t stream)
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = carveout;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, kernel, args, tm_scales, tm_zeros, tm_w) != cudaSuccess)
         return W4_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? W4_OK : W4_ERR_CUDA;

@@ -409,9 +409,8 @@ static int launch_one(Args a, DeviceInfo const& dev, cudaStream_t stream)
     int const mt = (a.m + 1) / 2;
     size_t const duo_bytes = 2 * (size_t(kUnitK) * a.m * 2 + size_t(2 * mt) * 16);
     size_t const fixed = size_t(kWarps) * a.slots * 8 * mt * 16;
-    // Loads in flight need their place in L1, which shares its memory with shared memory: 64 KB of them leave
-    // 192 KB of an SM's 256 at most.
-    constexpr size_t kSmemMost = 192 * 1024 - 1024;
+    // Loads in flight need their place in L1, which shares its memory with shared memory.
+    constexpr size_t kSmemMost = kDecodeSmem;
     if (fixed + duo_bytes > kSmemMost)
         return W4_ERR_UNSUPPORTED;
     int const duos = (a.k / kUnitK + 1) / 2, most = int((kSmemMost - fixed) / duo_bytes);
@@ -439,10 +438,10 @@ static int launch_one(Args a, DeviceInfo const& dev, cudaStream_t stream)
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    // The smallest shared memory that fits. Left alone the runtime keeps what the kernel in front had, and behind
-    // one that takes all of it 28 KB of L1 hold the loads back: 82 us instead of 49.5 at 8192 x 57344, four rows.
+    // Left alone the runtime keeps the split that the kernel in front had, and behind one that takes all shared
+    // memory 28 KB of L1 hold the loads back: 82 us instead of 49.5 at 8192 x 57344, four rows.
     attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    attr[1].val.sharedMemCarveout = unsigned((cfg.dynamicSmemBytes + 1024) * 100 / (228 * 1024) + 1);
+    attr[1].val.sharedMemCarveout = kDecodeCarveout;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
