@@ -259,7 +259,9 @@ double regime_prefill_us(int m, int n, int k, int num_sms, int weight_bits)
 }
 
 // An automatic launch in the decode regime: the tensor-core kernel in the forms that need no workspace, where
-// its estimate is 1.5 us below the decode kernel's (whose launch also costs the host less). One row on
+// its estimate is 1.5 us below the decode kernels' (whose launch also costs the host less), or 3 us up to 8 rows:
+// there its neighbours are decode kernels, with another L1 / shared memory split (four layers at four rows
+// 121.9 us with a tensor-core kernel among them that is 1 us faster by itself, 118.2 without). One row on
 // 4096 x 14336 int8 18.9 -> 14.5 us, six rows on 6144 x 24576 int4 with 64-wide groups 31.1 -> 24.6, 16 rows
 // on 4096 x 14336 int4 17.2 -> 11.7; int4 at a few rows stays with the decode kernels (one row on 4096 x 14336
 // 9.4 against 11.8).
@@ -270,7 +272,7 @@ bool decode_takes_tensor_cores(W4GemmParams const& p)
     w4::DeviceInfo const& dev = w4::current_device_info();
     double const decode = w4::gemv_estimate_us(p);
     return dev.num_sms > 0 && decode > 5.0
-        && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 1.5 < decode;
+        && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + (p.m <= 8 ? 3.0 : 1.5) < decode;
 }
 
 int resolve_regime(W4GemmParams const& p)
