@@ -1023,10 +1023,11 @@ static int dispatch_split(W4GemmParams const& p, void const* act, Experts const&
     int rows[kMaxExperts];
     for (int e = 0; e < ex.num; ++e)
         rows[e] = ex.first_row[e + 1] - ex.first_row[e];
-    // the form of split-k that uses the caller's workspace needs room for the partial tiles there (and adds
-    // one bias)
+    // The form of split-k that uses the caller's workspace needs room for the partial tiles there, and its second
+    // kernel adds up and stores all p.m rows with one bias: not for the experts of a 3-D weight, also where a
+    // launch has one expert only.
     size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
-    TcPlan plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, ex.num == 1);
+    TcPlan plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, ex.slices == 1);
     if (plan.splits > 1 && !plan.cluster && (!p.workspace || p.workspace_bytes < act_copy + split_bytes(p.m, p.n, plan.splits)))
         plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false);
     if (plan.splits == 1)

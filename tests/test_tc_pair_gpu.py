@@ -1,8 +1,11 @@
 """The CTA-pair tensor-core kernel at the sizes where its tiles, rings and splits can go wrong (needs a B200)."""
+import ctypes
+
 import pytest
 import torch
 
 import tensorrt_llm_b200 as pkg
+from tensorrt_llm_b200._lib import W4GemmParams
 from oracle import woq_oracle as oracle
 from _cases import make_problem, max_err, oracle_out, run_gpu
 
@@ -65,4 +68,31 @@ def test_experts_in_one_launch(bits, group, rows, k, n):
         if r:
             ref = oracle_out(dict(p, act=p["act"][:r]), alpha=0.5 if full else 1.0)
             assert max_err(out[first[e]:first[e + 1]], ref) <= oracle.tolerance(ref), e
+    assert pkg._lib.lib().w4_gemm_device_status() == 0
+
+
+def test_last_expert_of_a_launch_keeps_to_its_own_rows():
+    """33 experts are a launch of 32 and one of a single expert; given a workspace, that one must not use the
+    split that adds up and stores the whole output (a few tiles and a long k, where its plan would). Through the
+    C ABI, where callers pass a workspace."""
+    experts, rows, n, k = 33, 33, 64, 16384
+    assert pkg.ops.select_regime(rows, n, k, 64, 4, torch.bfloat16) == pkg.W4_REGIME_GEMM
+    first = [rows * e for e in range(experts + 1)]
+    probs = [make_problem(rows, n, k, 4, 64, torch.bfloat16, zero=True, bias=True, seed=e) for e in range(experts)]
+    act = torch.cat([p["act"] for p in probs]).cuda()
+    weight, scales, zeros, bias = (torch.stack([p[key] for p in probs]).cuda()
+                                   for key in ("processed", "scales", "zeros", "bias"))
+    out = torch.empty((experts * rows, n), dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(64 << 20, dtype=torch.uint8, device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    params = W4GemmParams(act=ptr(act), weight=ptr(weight), scales=ptr(scales), zeros=ptr(zeros), bias=ptr(bias),
+                          out=ptr(out), alpha=0.5, m=experts * rows, n=n, k=k, group_size=64, weight_bits=4,
+                          act_dtype=pkg._lib.W4_DTYPE_BF16, workspace=ptr(ws), workspace_bytes=ws.numel())
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    rc = pkg._lib.lib().w4_gemm_launch_experts(ctypes.byref(params), experts, (ctypes.c_int * len(first))(*first), stream)
+    assert rc == 0
+    got = out.cpu()
+    for e, p in enumerate(probs):
+        ref = oracle_out(p, alpha=0.5)
+        assert max_err(got[first[e]:first[e + 1]], ref) <= oracle.tolerance(ref), e
     assert pkg._lib.lib().w4_gemm_device_status() == 0
