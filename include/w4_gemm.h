@@ -90,7 +90,11 @@ extern "C"
         W4_DTYPE_FP32 = 2 /* only as the source type of w4_symmetric_quantize_device */
     };
 
-    /* Which kernel family runs. AUTO applies w4_gemm_select_regime(). */
+    /* Which kernel family runs. AUTO applies w4_gemm_select_regime(). The regime also decides the arithmetic: the
+     * decode kernels apply scales and zeros to 32-bit sums, the tensor-core kernel multiplies with weights that
+     * were scaled and rounded to the activation type first, as the reference's kernels do. (int4 with 64-wide
+     * groups is rounded that way in both, and there an automatic launch in the decode regime may run the
+     * tensor-core kernel, without a workspace.) */
     enum
     {
         W4_REGIME_AUTO = 0,
@@ -183,18 +187,20 @@ extern "C"
     int w4_gemm_run_host(const W4GemmParams* p, const void* host_act, void* host_out, void* stream);
 
     /*
-     * The GEMMs of all experts of a mixture-of-experts layer over 3-D weights: one launch of the
-     * tensor-core kernel for up to 32 experts with rows, or, with a pre-quant scale, a requested regime or
-     * rows for a single expert, one w4_gemm_launch after another. p describes expert 0: weight is [E][K, N*bits/8], every expert's matrix laid out on its
-     * own - what preprocess_weights_for_mixed_gemm does with a 3-D tensor
+     * The GEMMs of all experts of a mixture-of-experts layer over 3-D weights. Every expert is computed in the
+     * regime of its own rows; those in the tensor-core kernel's regime, if there are two or more, share launches
+     * of up to 32 experts, the others (all, with a pre-quant scale or a requested regime) are one
+     * w4_gemm_launch after another. p describes expert 0: weight is [E][K, N*bits/8], every expert's matrix laid
+     * out on its own - what preprocess_weights_for_mixed_gemm does with a 3-D tensor
      * (cpp/tensorrt_llm/thop/weightOnlyQuantOp.cpp:136-147, force_interleave); scales / zeros are
      * [E][K/G, N] (or [E][N]), bias [E][N]; act_scale [K] is shared. The rows of act and out are sorted
      * by expert: expert e owns rows expert_first_row[e] .. expert_first_row[e + 1] - 1 (host array of
      * num_experts + 1 non-decreasing ints starting at 0; the running totals the reference's MoE GEMM
      * takes as total_tokens_including_expert,
-     * cpp/tensorrt_llm/kernels/internal_cutlass_kernels/include/moe_gemm_kernels.h:236, kept on the host). p->m is ignored; the
-     * workspace is used expert by expert only and must then cover the largest per-expert row count
-     * (w4_gemm_workspace_bytes_max). Experts without rows are skipped. Returns the first error.
+     * cpp/tensorrt_llm/kernels/internal_cutlass_kernels/include/moe_gemm_kernels.h:236, kept on the host).
+     * p->m is ignored; the workspace serves one expert at a time, never a shared launch, and must then cover the
+     * largest per-expert row count (w4_gemm_workspace_bytes_max). Experts without rows are skipped. Returns the
+     * first error.
      */
     int w4_gemm_launch_experts(const W4GemmParams* p, int num_experts, const int* expert_first_row, void* stream);
 

@@ -258,16 +258,21 @@ double regime_prefill_us(int m, int n, int k, int num_sms, int weight_bits)
     return 7.0 + (splits > 1 ? 3.0 : 0.0) + waves(bm, splits) * step_us(bm) * double((steps + splits - 1) / splits);
 }
 
+// The regime also decides the arithmetic: decode kernels apply scales and zeros to 32-bit sums, the tensor-core
+// kernel rounds every scaled weight to the activation type first (outputs 2.3e-3 of their size from the exact
+// ones instead of 1.7e-3 for bf16, 2.9e-4 instead of 2.1e-4 for fp16). With 64-wide groups on int4 both round, so
+// that there the decode regime may take either.
+bool rounds_weights_anyway(W4GemmParams const& p)
+{
+    return p.weight_bits == 4 && p.group_size == 64;
+}
+
 // An automatic launch in the decode regime: the tensor-core kernel in the forms that need no workspace, where
-// its estimate is 1.5 us below the decode kernels' (whose launch also costs the host less), or 3 us up to 8 rows:
-// there its neighbours are decode kernels, with another L1 / shared memory split (four layers at four rows
-// 121.9 us with a tensor-core kernel among them that is 1 us faster by itself, 118.2 without). One row on
-// 4096 x 14336 int8 18.9 -> 14.5 us, six rows on 6144 x 24576 int4 with 64-wide groups 31.1 -> 24.6, 16 rows
-// on 4096 x 14336 int4 17.2 -> 11.7; int4 at a few rows stays with the decode kernels (one row on 4096 x 14336
-// 9.4 against 11.8).
+// its arithmetic is the same and its estimate is 1.5 us below the decode kernel's (whose launch also costs the
+// host less), or 3 us up to 8 rows. Six rows on 6144 x 24576: 31.1 -> 24.6 us.
 bool decode_takes_tensor_cores(W4GemmParams const& p)
 {
-    if (p.act_scale)
+    if (p.act_scale || !rounds_weights_anyway(p))
         return false;
     w4::DeviceInfo const& dev = w4::current_device_info();
     double const decode = w4::gemv_estimate_us(p);
@@ -289,6 +294,45 @@ bool takes_decode_kernel(W4GemmParams const& p)
         return false;
     bool const chosen = p.regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO;
     return !(chosen && decode_takes_tensor_cores(p));
+}
+
+// Which experts of a layer the shared launch of the tensor-core kernel takes: those in its own regime, or all.
+bool in_gemm_regime(W4GemmParams const& p, int rows)
+{
+    return rows > 0 && auto_regime(rows, p.n, p.k, p.group_size, p.weight_bits, p.act_dtype) == W4_REGIME_GEMM;
+}
+
+bool has_rows(W4GemmParams const& p, int rows)
+{
+    (void) p;
+    return rows > 0;
+}
+
+// Whether one launch for all experts is estimated faster than one for those in the tensor-core kernel's regime
+// and a launch of the decode kernel for each of the others (the first 32 with rows stand for all).
+bool sharing_is_faster(W4GemmParams const& p, int num_experts, int const* first_row)
+{
+    w4::DeviceInfo const& dev = w4::current_device_info();
+    if (dev.num_sms <= 0)
+        return false;
+    auto plan_us = [&](int const* rows, int num)
+    { return num ? w4::gemm_tc_plan(rows, num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us : 0.0; };
+    constexpr int kMost = 32;
+    int all[kMost], large[kMost], num_all = 0, num_large = 0;
+    double apart = 0.0;
+    for (int e = 0; e < num_experts && num_all < kMost; ++e)
+    {
+        W4GemmParams q = p;
+        q.m = first_row[e + 1] - first_row[e];
+        if (q.m == 0)
+            continue;
+        all[num_all++] = q.m;
+        if (in_gemm_regime(p, q.m))
+            large[num_large++] = q.m;
+        else
+            apart += w4::gemv_estimate_us(q);
+    }
+    return plan_us(all, num_all) < apart + plan_us(large, num_large);
 }
 
 void log_refusal(char const* entry, W4GemmParams const* p, int rc)
@@ -522,15 +566,13 @@ extern "C"
         size_t const weight_bytes = size_t(p->k) * p->n * p->weight_bits / 8;
         auto at = [](const void* base, size_t bytes) -> const void*
         { return base ? static_cast<const char*>(base) + bytes : nullptr; };
-        // Two or more experts with rows and nothing to do in front: all in one launch of the tensor-core kernel,
-        // whose work items then fill the chip together (eight experts of 4096 x 14336 int4 with 4 to 19 rows:
-        // one after another 100 us, together 72 us). One expert, or a pre-quant scale: expert by expert.
+        // Two or more experts that the tensor-core kernel may take and nothing to do in front: those in one launch,
+        // whose work items then fill the chip together. The others one after another.
+        bool (*joins)(W4GemmParams const&, int) = in_gemm_regime;
         int used = 0;
-        for (int e = 0; e < num_experts; ++e)
-            used += expert_first_row[e + 1] > expert_first_row[e];
-        if (used > 1 && !p->act_scale && p->regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO)
+        W4GemmParams q = *p;
+        if (!p->act_scale && p->regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO)
         {
-            W4GemmParams q = *p;
             q.m = expert_first_row[num_experts];
             q.regime = W4_REGIME_GEMM;
             int const rc = w4_gemm_validate(&q);
@@ -539,17 +581,27 @@ extern "C"
                 log_refusal("w4_gemm_launch_experts", p, rc);
                 return rc;
             }
+            if (rounds_weights_anyway(*p) && sharing_is_faster(*p, num_experts, expert_first_row))
+                joins = has_rows;
+            for (int e = 0; e < num_experts; ++e)
+                used += joins(*p, expert_first_row[e + 1] - expert_first_row[e]);
+        }
+        bool const shared = used > 1;
+        if (shared)
+        {
             if (log_level() <= W4_LOG_DEBUG)
                 log_line(W4_LOG_DEBUG, "w4_gemm_launch_experts m=%d n=%d k=%d bits=%d group=%d experts=%d tensor-core kernel (chosen)",
                     q.m, q.n, q.k, q.weight_bits, q.group_size, used);
-            return w4::launch_gemm_tc_experts(q, num_experts, expert_first_row, static_cast<cudaStream_t>(stream));
+            int const rc = w4::launch_gemm_tc_experts(q, num_experts, expert_first_row, joins, static_cast<cudaStream_t>(stream));
+            if (rc != W4_OK)
+                return rc;
         }
         for (int e = 0; e < num_experts; ++e)
         {
             int const row0 = expert_first_row[e], rows = expert_first_row[e + 1] - row0;
-            if (rows == 0)
+            if (rows == 0 || (shared && joins(*p, rows)))
                 continue;
-            W4GemmParams q = *p;
+            q = *p;
             q.m = rows;
             q.act = at(p->act, size_t(row0) * p->k * elt);
             q.out = const_cast<void*>(at(p->out, size_t(row0) * p->n * elt));

@@ -75,12 +75,12 @@ struct Args
     int group_shift; // log2(group size), 31 = per-channel
     int bm;          // activation rows per tile
     int tiles_n;
-    // Experts (an ordinary GEMM is one): expert e has rows first_row[e] .. first_row[e + 1] - 1 of the
+    // Experts (an ordinary GEMM is one): expert e has rows first_row[e] .. row_end[e] - 1 of the
     // activations and of the output, tiles first_tile[e] .. first_tile[e + 1] - 1, the weights, scales and zeros
     // of slice slice[e] of their tensors, and bias + slice[e] * n.
     int num_experts;
     int groups; // scale rows per expert
-    int first_row[kMaxExperts + 1], first_tile[kMaxExperts + 1], slice[kMaxExperts];
+    int first_row[kMaxExperts], row_end[kMaxExperts], first_tile[kMaxExperts + 1], slice[kMaxExperts];
     int num_stages, num_wstages;
     int d_bufs;      // accumulators in TMEM: 2 up to 128 rows, else 1
     int weights_static;
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         int const t = tile - a.first_tile[e], tm = t / a.tiles_n;
         it.n0 = (t - tm * a.tiles_n) * kPairN;
         it.row0 = a.first_row[e] + tm * a.bm;
-        it.row_end = a.first_row[e + 1];
+        it.row_end = a.row_end[e];
         it.slice = a.slice[e];
         return it;
     };
@@ -910,11 +910,11 @@ static int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t sm
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
 }
 
-// The experts of a launch: those of `slices` that have rows.
+// The experts of a launch, out of the `slices` of the weight tensor.
 struct Experts
 {
     int num, slices;
-    int slice[kMaxExperts], first_row[kMaxExperts + 1];
+    int slice[kMaxExperts], first_row[kMaxExperts], row_end[kMaxExperts];
 };
 
 template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
@@ -941,9 +941,9 @@ static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex,
     {
         a.slice[e] = ex.slice[e];
         a.first_row[e] = ex.first_row[e];
-        a.first_tile[e + 1] = a.first_tile[e] + (ex.first_row[e + 1] - ex.first_row[e] + plan.bm - 1) / plan.bm * a.tiles_n;
+        a.row_end[e] = ex.row_end[e];
+        a.first_tile[e + 1] = a.first_tile[e] + (ex.row_end[e] - ex.first_row[e] + plan.bm - 1) / plan.bm * a.tiles_n;
     }
-    a.first_row[ex.num] = ex.first_row[ex.num];
     a.weights_static = (p.flags & W4_GEMM_WEIGHTS_STATIC) ? 1 : 0;
     a.splits = plan.splits;
     a.steps_split = plan.steps_split;
@@ -1022,7 +1022,7 @@ static int dispatch_split(W4GemmParams const& p, void const* act, Experts const&
 {
     int rows[kMaxExperts];
     for (int e = 0; e < ex.num; ++e)
-        rows[e] = ex.first_row[e + 1] - ex.first_row[e];
+        rows[e] = ex.row_end[e] - ex.first_row[e];
     // The form of split-k that uses the caller's workspace needs room for the partial tiles there, and its second
     // kernel adds up and stores all p.m rows with one bias: not for the experts of a 3-D weight, also where a
     // launch has one expert only.
@@ -1184,12 +1184,13 @@ int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream)
             return rc;
         act = p.workspace;
     }
-    tc::Experts const one{1, 1, {0}, {0, p.m}};
+    tc::Experts const one{1, 1, {0}, {0}, {p.m}};
     return p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, act, one, dev, stream)
                                         : tc::dispatch<__nv_bfloat16>(p, act, one, dev, stream);
 }
 
-int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, cudaStream_t stream)
+int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, bool (*joins)(W4GemmParams const&, int),
+    cudaStream_t stream)
 {
     DeviceInfo const& dev = current_device_info();
     if (dev.num_sms <= 0)
@@ -1198,11 +1199,11 @@ int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* fi
     ex.slices = num_experts;
     for (int e = 0; e < num_experts; ++e)
     {
-        if (first_row[e + 1] > first_row[e])
+        if (joins(p, first_row[e + 1] - first_row[e]))
         {
             ex.slice[ex.num] = e;
             ex.first_row[ex.num] = first_row[e];
-            ex.first_row[++ex.num] = first_row[e + 1];
+            ex.row_end[ex.num++] = first_row[e + 1];
         }
         if (ex.num == tc::kMaxExperts || (e + 1 == num_experts && ex.num > 0))
         {

@@ -179,6 +179,15 @@ def test_regime_heuristic(lib):
         assert lib.w4_gemm_select_regime(m, 4096, 14336, 128, 4) == pkg.W4_REGIME_GEMM
 
 
+def test_experts_refuse_bad_shapes_before_anything_is_estimated():
+    lib = pkg._lib.lib()
+    first = (ctypes.c_int * 3)(0, 16, 40)
+    base = dict(act=16, weight=16, scales=16, out=16, alpha=1.0, n=128, k=128, group_size=64, weight_bits=4, act_dtype=1)
+    call = lambda **kw: lib.w4_gemm_launch_experts(ctypes.byref(pkg._lib.W4GemmParams(**dict(base, **kw))), 2, first, None)
+    assert [call(n=0), call(k=0), call(n=-64), call(k=96), call(weight_bits=3), call(act=24)] == [-2, -2, -2, -2, -4, -5]
+
+
+
 def test_regime_heuristic_knows_the_activation_type(lib):
     """int8 weights with bf16 activations: a decode pass costs more (two nibble planes), so two
     16-row passes over a small matrix lose to the tensor-core kernel where float16 still takes them
