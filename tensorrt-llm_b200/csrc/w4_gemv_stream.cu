@@ -12,11 +12,15 @@
 // fit) are laid out once in shared memory as the B operands of every unit.
 //
 // Arithmetic: for fp16 and bf16 activations alike the multiplication is fp16 x integer with fp32 sums. Nibbles
-// are placed into fp16 numbers where they lie: 1024 + u in mantissa bits 0..3, 1024 + 16 u in bits 4..7 (one
-// shift for eight weights; bf16 with its 7-bit mantissa takes three and 40 % more integer instructions, whose
-// pipe is the second bound). The two kinds have accumulators of their own; scale, zero, the 1/16 and the
-// constants are applied to the unit's sums. bf16 activations become fp16 exactly: each row of a unit is
-// scaled by the power of two that brings its largest value to 2^14, the factor is taken back with the sums.
+// become fp16 numbers where they lie: alone in the low mantissa bits they are the subnormals u * 2^-24 (bits 0..3)
+// and u * 2^-20 (bits 4..7), which the tensor cores multiply exactly (one shift for eight weights; bf16 with its
+// 7-bit mantissa takes three and 40 % more integer instructions, whose pipe is the second bound). Under an
+// exponent, as 1024 + u, they take as long, but then 1032 sum(a) has to cancel in every unit: positive
+// activations on integers of -1, 0 and 1 at 28672 k gave outputs 2.3e-3 (bf16) and 1.2e-2 (fp16) of their size
+// from the exact ones, now 1.6e-3 and 2.2e-4, the output's rounding. The two kinds have accumulators of their
+// own; scale, zero, the powers of two and the bias of 8 are applied to the unit's sums. bf16 activations become
+// fp16 exactly: each row of a unit is scaled by the power of two that brings its largest value to 2^14, the
+// factor is taken back with the sums.
 //
 // Measured (zeros, group 128): 4096 x 14336 at one row 10.5 -> 9.4 us, 14336 x 4096 12.2 -> 10.0, 2048 x 8192
 // 6.7 -> 4.5, 8192 x 57344 at four rows 58.1 -> 49.5 (4.7 TB/s).
@@ -37,9 +41,9 @@ constexpr int kThreads = 32 * kWarps;
 constexpr int kUnitK = 128;
 constexpr int kPieces = 4; // 16-byte pieces of a lane's activation fragment of a unit: one per weight register
 
-// What the magic constants and the bias of the integers add to a weight: u = q + 8 as 1024 + u, or as
-// (1024 + 16 u) / 16.
-constexpr float kBiasEven = 1024.f + 8.f, kBiasOdd = 64.f + 8.f;
+constexpr float kBias = 8.f;           // weights are stored as u = q + 8
+constexpr float kEven = 16777216.f;    // 2^24: what a sum over even nibbles has to be multiplied by
+constexpr float kOddByEven = 0.0625f;  // the odd ones lie four bits higher
 
 struct Args
 {
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(Args const a)
                 for (int p = 0; p < kPieces; ++p)
                     act_s[((u * kPieces + p) * a.m + row) * 4 + ft] = make_uint4(x[4 * p], x[4 * p + 1], x[4 * p + 2], x[4 * p + 3]);
                 if (ft == 0)
-                    row_s[u * MR + row] = make_float4(unscale, -fmaf(kBiasEven, se, kBiasOdd * so), unscale * (se + so), 0.f);
+                    row_s[u * MR + row] = make_float4(unscale, -kBias * (se + so), unscale * (se + so), 0.f);
             }
         }
     };
@@ -285,16 +289,13 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(Args const a)
     // One unit: 16 columns x 128 k, added to the running sums. `act`, `rows`: the unit's activations and factors.
     auto process = [&](Unit const& u, uint4 const* act, float4 const* rows)
     {
-        constexpr uint32_t kMagic = 0x64006400u; // 1024: a value in its low mantissa bits adds exactly
         float even[4], odd[4];
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj)
         {
             uint32_t const ra = u.wa[jj], rb = u.wb[jj], sa = ra >> 8, sb = rb >> 8;
-            uint32_t const ev[4] = {lop3_and_or(ra, 0x000f000fu, kMagic), lop3_and_or(rb, 0x000f000fu, kMagic),
-                lop3_and_or(sa, 0x000f000fu, kMagic), lop3_and_or(sb, 0x000f000fu, kMagic)};
-            uint32_t const od[4] = {lop3_and_or(ra, 0x00f000f0u, kMagic), lop3_and_or(rb, 0x00f000f0u, kMagic),
-                lop3_and_or(sa, 0x00f000f0u, kMagic), lop3_and_or(sb, 0x00f000f0u, kMagic)};
+            uint32_t const ev[4] = {ra & 0x000f000fu, rb & 0x000f000fu, sa & 0x000f000fu, sb & 0x000f000fu};
+            uint32_t const od[4] = {ra & 0x00f000f0u, rb & 0x00f000f0u, sa & 0x00f000f0u, sb & 0x00f000f0u};
             uint4 const b = act[jj * piece + act_lane];
             if (jj == 0)
             {
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(Args const a)
                 H::mma(odd, od, b.z, b.w);
             }
         }
-        // s f (S - C) + z f sum(a) with the row's factor f and constants C
+        // s f (S - 8 sum(a)) + z f sum(a) with the row's factor f
         float s[2], z[2] = {0.f, 0.f};
         P::unpack2(u.s, s[0], s[1]);
         if (HAS_ZERO)
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(Args const a)
         for (int c = 0; c < 4; ++c)
         {
             float4 const& f = c & 1 ? f1 : f0;
-            acc[c] = fmaf(s[c >> 1] * f.x, fmaf(odd[c], 0.0625f, even[c]) + f.y, acc[c]);
+            acc[c] = fmaf(s[c >> 1] * f.x, fmaf(fmaf(odd[c], kOddByEven, even[c]), kEven, f.y), acc[c]);
             if (HAS_ZERO)
                 acc[c] = fmaf(z[c >> 1], f.z, acc[c]);
         }

@@ -48,3 +48,30 @@ def test_experts_have_the_arithmetic_of_their_own_regime(bits, group, rows):
             ref = oracle_out(p)
             assert max_err(got, ref) <= oracle.tolerance(ref), e
     assert pkg.W4_REGIME_GEMV in regimes
+
+
+@pytest.mark.parametrize("m,n,k,group,dtype", [
+    (1, 1024, 28672, 128, torch.bfloat16),
+    (2, 4096, 12416, 0, torch.bfloat16),
+    (3, 4096, 12416, 128, torch.float16),
+])
+def test_streaming_sums_of_one_sign(m, n, k, group, dtype):
+    """Positive activations on integers q of -1, 0 and 1: what the streaming kernel's integers carry besides the
+    weight (u = q + 8, at most 9) must not drown the sums. Rounding to the output type errs to both sides, by half a
+    unit in the last place h at most: the mean over all outputs stays within 5 h / sqrt(3) of their size /
+    sqrt(their number). Truncation in the tensor cores errs to one: a 128-k unit's two chains add in eight steps,
+    step j loses 2^-23 of a sum of at most j / 8 * 9 sum|a|, together 40.5 * 2^-23 of scale * sum|a|."""
+    g = torch.Generator().manual_seed(m)
+    p = make_problem(m, n, k, 4, group, dtype, scale_lo=0.01, scale_hi=0.01001, seed=m)
+    q = torch.randint(-1, 2, (k, n), dtype=torch.int8, generator=g)
+    p["q"], p["act"] = q, (torch.rand((m, k), generator=g) + 0.5).to(dtype)
+    p["packed"] = pkg.quantize.pack_int8_tensor_to_packed_int4(q)
+    p["processed"] = pkg.quantize.preprocess_weights_for_mixed_gemm(p["packed"], torch.quint4x2)
+    s = p["scales"].double()
+    w = q.double() * (s if group == 0 else s.repeat_interleave(group, 0))
+    a = p["act"].double()
+    exact, size = a @ w, a.abs().sum(1, keepdim=True) * s.max()
+    out = run_gpu(p, regime=pkg.W4_REGIME_GEMV).double()
+    half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    rounding = 5 * half_ulp / 3 ** 0.5 * float(exact.square().mean().sqrt()) / exact.numel() ** 0.5
+    assert abs(float((out - exact).mean())) <= rounding + 40.5 * 2.0 ** -23 * float(size.mean())
