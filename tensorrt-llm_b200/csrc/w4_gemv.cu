@@ -64,6 +64,7 @@ constexpr int kThreads = kConsumerThreads + 128; // + one producer warp group (o
 constexpr int kProducerRegs = 24, kConsumerRegs = 112; // 128 * 24 + 512 * 112 <= 640 * 96 (the launch-time pool)
 constexpr int kRedBytes = 64 * 1024;            // shared memory for cross-warp partial sums
 constexpr int kRedBytesSmall = 52 * 1024;       // the same up to 6 rows (8 column groups at 6 rows)
+constexpr size_t kSmemSmall = 195 * 1024;       // shared memory of a CTA there, all in all
 constexpr int kRedBytes16 = 112 * 1024;         // the same for 16-row passes (7 column groups)
 constexpr int kScaleBoxCols = 24;               // columns per scale/zero box: 16 + slack to start on a 16-byte boundary
 
@@ -906,16 +907,19 @@ static int launch_one(Args const& a, DeviceInfo const& dev, cudaStream_t stream)
     // remain; ~72 KB are in flight at a time anyway).
     args.red_bytes = MB == 2 ? kRedBytes16 : kRedBytes;
     size_t fixed = size_t(args.red_bytes) + 64 + 1024; // + slack to start the ring on a 1024-byte boundary
-    // Shared memory per CTA: all a block may have, or, where four slots and the sums of as many column groups
-    // still fit, what the streaming kernel leaves (kDecodeSmem).
+    // Shared memory per CTA: all a block may have, or, up to 6 rows and where four slots and the sums of as many
+    // column groups still fit, so much less that L1 has 60 KB instead of 28: the activations, which every column group
+    // (and k panel) reloads, stay in it. 28672 x 8192 with pre-quant scale at 4 / 6 rows 38.6 / 41.6 -> 36.7 /
+    // 38.1 us, 4096 x 4096 5.5 / 5.9 -> 5.2 / 5.7; without the scale 36.0 / 37.3 -> 35.8 / 36.2 and at worst
+    // 14336 x 4096 at 6 rows 12.6 -> 12.9; one and two rows, 64-wide groups and int8 equal.
     size_t smem_budget = size_t(dev.max_smem_optin);
     unsigned carveout = 100;
-    if (MB == 1 && a.m <= 6 && fixed - kRedBytes + kRedBytesSmall + 4 * size_t(args.slot_bytes + 16) <= kDecodeSmem)
+    if (MB == 1 && a.m <= 6 && fixed - kRedBytes + kRedBytesSmall + 4 * size_t(args.slot_bytes + 16) <= kSmemSmall)
     {
         args.red_bytes = kRedBytesSmall;
         fixed += kRedBytesSmall - kRedBytes;
-        smem_budget = kDecodeSmem;
-        carveout = kDecodeCarveout;
+        smem_budget = kSmemSmall;
+        carveout = 85; // of 228 KB, rounded up: 196
     }
     int slots = int((smem_budget - fixed) / (args.slot_bytes + 16));
     if (slots < 2)

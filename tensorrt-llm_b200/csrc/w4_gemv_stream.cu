@@ -22,8 +22,8 @@
 // fp16 exactly: each row of a unit is scaled by the power of two that brings its largest value to 2^14, the
 // factor is taken back with the sums.
 //
-// Measured (zeros, group 128): 4096 x 14336 at one row 10.5 -> 9.4 us, 14336 x 4096 12.2 -> 10.0, 2048 x 8192
-// 6.7 -> 4.5, 8192 x 57344 at four rows 58.1 -> 49.5 (4.7 TB/s).
+// Measured against the kernel of w4_gemv.cu (zeros, group 128): 4096 x 14336 at one row 10.5 -> 9.1 us, 14336 x 4096
+// 12.2 -> 9.7, 2048 x 8192 6.7 -> 4.5, 8192 x 57344 at one row 54 -> 47 and at four 58 -> 50 (4.9 TB/s).
 #include <mutex>
 #include <type_traits>
 
@@ -410,8 +410,7 @@ static int launch_one(Args a, DeviceInfo const& dev, cudaStream_t stream)
     int const mt = (a.m + 1) / 2;
     size_t const duo_bytes = 2 * (size_t(kUnitK) * a.m * 2 + size_t(2 * mt) * 16);
     size_t const fixed = size_t(kWarps) * a.slots * 8 * mt * 16;
-    // Loads in flight need their place in L1, which shares its memory with shared memory.
-    constexpr size_t kSmemMost = kDecodeSmem;
+    constexpr size_t kSmemMost = 195 * 1024; // leaves L1 60 KB (see the launch attribute below)
     if (fixed + duo_bytes > kSmemMost)
         return W4_ERR_UNSUPPORTED;
     int const duos = (a.k / kUnitK + 1) / 2, most = int((kSmemMost - fixed) / duo_bytes);
@@ -439,10 +438,12 @@ static int launch_one(Args a, DeviceInfo const& dev, cudaStream_t stream)
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    // Left alone the runtime keeps the split that the kernel in front had, and behind one that takes all shared
-    // memory 28 KB of L1 hold the loads back: 82 us instead of 49.5 at 8192 x 57344, four rows.
+    // The loads in flight need their place in L1. Left alone the runtime keeps the split that the kernel in front
+    // had, and behind one that takes all shared memory 28 KB of L1 hold the loads back: 80 us instead of 47 at
+    // 8192 x 57344, one row. Half of the memory (more where the activations need it) is far from that: at 85 %
+    // some sizes of shared memory, 16 or 24 KB among them, still met the largest split, at 0 to 70 % none did.
     attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    attr[1].val.sharedMemCarveout = kDecodeCarveout;
+    attr[1].val.sharedMemCarveout = 50;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, a) == cudaSuccess ? W4_OK : W4_ERR_CUDA;

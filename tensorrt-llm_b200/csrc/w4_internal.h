@@ -38,11 +38,6 @@ struct PushTarget
     unsigned long long timeout_ns;
 };
 int launch_gemv(W4GemmParams const& p, cudaStream_t stream, PushTarget const* push = nullptr);
-// Shared memory of the decode kernels where both keep to it, and the share of an SM's 228 KB that they ask for
-// then (rounded up, 196 KB): with the same split an SM goes from one kernel to the other without running empty first
-// (four layers at four rows 121.0 -> 117.8 us).
-constexpr size_t kDecodeSmem = 195 * 1024;
-constexpr unsigned kDecodeCarveout = 85;
 // The decode kernel without staging, for int4 weights, 128-wide groups or none, whole 128-wide k units and up
 // to 8 rows (called by launch_gemv where it is the faster). W4_ERR_UNSUPPORTED: too many columns.
 int launch_gemv_stream(W4GemmParams const& p, cudaStream_t stream);

@@ -36,3 +36,30 @@ def test_shares_tails_and_panels(m, n, k, group, dtype):
         assert max_err(out[[row]][:, cols], ref) <= oracle.tolerance(ref), row
     assert torch.equal(out, run_gpu(p, regime=pkg.W4_REGIME_GEMV, alpha=alpha))  # sums in a fixed order
     assert pkg._lib.lib().w4_gemm_device_status() == 0
+
+
+def test_one_row_is_not_slower_than_eight():
+    """The weights are the same and the activations fewer. (With the wrong split of L1 and shared memory, which
+    depended on the activations' size, one row took 80 us here and eight 54.)"""
+    n, k = 57344, 8192
+    w = torch.randint(-128, 128, (k, n // 2), dtype=torch.int8, device="cuda")
+    s, z = (torch.rand(k // 128, n, device="cuda").bfloat16() for _ in range(2))
+
+    def us(m):
+        a, out = torch.randn(m, k, device="cuda").bfloat16(), torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+        call = lambda: pkg.ops.gemm_raw(a, w, s, out, n=n, k=k, weight_bits=4, group_size=128, zeros=z,
+                                        regime=pkg.W4_REGIME_GEMV, weights_static=True)
+        best = 1e9
+        for _ in range(8):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            call()
+            e0.record()
+            for _ in range(20):
+                call()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1) * 50)
+        return best
+
+    one, eight = us(1), us(8)
+    assert one < 1.15 * eight
