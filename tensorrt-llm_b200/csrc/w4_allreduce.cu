@@ -269,7 +269,7 @@ __device__ __forceinline__ uint4 sum_ranks(uint4 const (&v)[kMaxRanks], uint4 mi
         if (r < world)
             add8<T>(acc, r == rank ? mine : v[r]);
     if (bias_vec)
-        add8<T>(acc, __ldg(bias_vec));
+        add8<T>(acc, *bias_vec);
     return pack8<T>(acc);
 }
 

@@ -57,7 +57,7 @@ __global__ void pre_quant_scale_kernel(uint4* out, uint4 const* act, uint4 const
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total_vec; i += stride)
     {
         uint4 a = act[i];
-        uint4 const s = __ldg(scale + (i % k_vec));
+        uint4 const s = scale[i % k_vec]; // (not __ldg: the kernel in front may have written it)
         a.x = P::mul(a.x, s.x);
         a.y = P::mul(a.y, s.y);
         a.z = P::mul(a.z, s.z);

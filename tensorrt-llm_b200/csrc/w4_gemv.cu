@@ -421,10 +421,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                     uint4 x = make_uint4(0, 0, 0, 0);
                     if (valid)
                     {
-                        x = __ldg(reinterpret_cast<uint4 const*>(act + size_t(row) * a.k + k0) + v);
+                        // (not __ldg: the kernel in front may write it while this one is resident)
+                        x = *(reinterpret_cast<uint4 const*>(act + size_t(row) * a.k + k0) + v);
                         if (HAS_ACT_SCALE)
                         {
-                            uint4 const ps = __ldg(reinterpret_cast<uint4 const*>(act_scale + k0) + v);
+                            uint4 const ps = *(reinterpret_cast<uint4 const*>(act_scale + k0) + v);
                             x.x = P::mul(x.x, ps.x);
                             x.y = P::mul(x.y, ps.y);
                             x.z = P::mul(x.z, ps.z);
@@ -909,9 +910,10 @@ static int launch_one(Args const& a, DeviceInfo const& dev, cudaStream_t stream)
     size_t fixed = size_t(args.red_bytes) + 64 + 1024; // + slack to start the ring on a 1024-byte boundary
     // Shared memory per CTA: all a block may have, or, up to 6 rows and where four slots and the sums of as many
     // column groups still fit, so much less that L1 has 60 KB instead of 28: the activations, which every column group
-    // (and k panel) reloads, stay in it. 28672 x 8192 with pre-quant scale at 4 / 6 rows 38.6 / 41.6 -> 36.7 /
-    // 38.1 us, 4096 x 4096 5.5 / 5.9 -> 5.2 / 5.7; without the scale 36.0 / 37.3 -> 35.8 / 36.2 and at worst
-    // 14336 x 4096 at 6 rows 12.6 -> 12.9; one and two rows, 64-wide groups and int8 equal.
+    // (and k panel) reloads, stay in it. With non-coherent loads of them, 28672 x 8192 with pre-quant scale at
+    // 4 / 6 rows 38.6 / 41.6 -> 36.7 / 38.1 us, 4096 x 4096 5.5 / 5.9 -> 5.2 / 5.7; without the scale 36.0 / 37.3
+    // -> 35.8 / 36.2 and at worst 14336 x 4096 at 6 rows 12.6 -> 12.9; one and two rows, 64-wide groups and int8
+    // equal. With the ordinary loads of now the first four are 34.8 / 35.3 and 5.1 / 5.7.
     size_t smem_budget = size_t(dev.max_smem_optin);
     unsigned carveout = 100;
     if (MB == 1 && a.m <= 6 && fixed - kRedBytes + kRedBytesSmall + 4 * size_t(args.slot_bytes + 16) <= kSmemSmall)

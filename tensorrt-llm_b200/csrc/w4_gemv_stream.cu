@@ -63,28 +63,29 @@ struct Args
     int weights_static;
 };
 
-// Weights are read once and pass L1 by; activations and scales stay in it.
+// The loads are ordinary ones, not non-coherent: this kernel is resident while the kernels in front write its
+// activations (and, where they are not static, its weights); volatile, so that they stay behind
+// griddepcontrol.wait. Weights are read once and pass L1 by; activations and scales stay in it.
 __device__ __forceinline__ uint4 ld_stream16(uint8_t const* p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
 }
 
-// (volatile, so that they stay behind griddepcontrol.wait)
 __device__ __forceinline__ uint4 ld_act16(void const* p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 
-__device__ __forceinline__ uint32_t ld_nc4(uint8_t const* p)
+__device__ __forceinline__ uint32_t ld_scale4(uint8_t const* p)
 {
     uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 
@@ -161,9 +162,9 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(Args const a)
         uint4 const va = ld_stream16(w), vb = ld_stream16(w + 32);
         u.wa[0] = va.x, u.wa[1] = va.y, u.wa[2] = va.z, u.wa[3] = va.w;
         u.wb[0] = vb.x, u.wb[1] = vb.y, u.wb[2] = vb.z, u.wb[3] = vb.w;
-        u.s = ld_nc4(ld_s + so);
+        u.s = ld_scale4(ld_s + so);
         if (HAS_ZERO)
-            u.z = ld_nc4(ld_z + so);
+            u.z = ld_scale4(ld_z + so);
     };
     auto load_next = [&](Unit& u0, Unit& u1)
     {

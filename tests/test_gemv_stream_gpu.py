@@ -38,6 +38,23 @@ def test_shares_tails_and_panels(m, n, k, group, dtype):
     assert pkg._lib.lib().w4_gemm_device_status() == 0
 
 
+@pytest.mark.parametrize("n,k", [(8192, 2048), (1024, 1024)])  # streaming kernel, staged kernel
+def test_activations_written_by_the_kernel_in_front(n, k):
+    """The kernels are resident while the kernel in front still writes their activations: what they read is what it
+    wrote last. (A read past that rule need not show here; the loads are ordinary ones for that reason.)"""
+    p = make_problem(2, n, k, 4, 128, torch.bfloat16, zero=True, prequant=True, seed=k)
+    w, s, z, ps = (p[key].cuda() for key in ("processed", "scales", "zeros", "ps"))
+    call = lambda a: pkg.ops.weight_only_groupwise_quant_matmul(a, ps, w, s, z, None, 1.0, pkg.ZERO | pkg.PRE_QUANT_SCALE, 128,
+                                                                weights_static=True)
+    acts = [torch.randn(2, k, generator=torch.Generator().manual_seed(i)).bfloat16().cuda() for i in range(8)]
+    want = [call(a) for a in acts]
+    buf, got = torch.empty_like(acts[0]), []
+    for i in range(200):
+        buf.copy_(acts[i % 8])
+        got.append(call(buf))
+    assert all(torch.equal(got[i], want[i % 8]) for i in range(200))
+
+
 def test_one_row_is_not_slower_than_eight():
     """The weights are the same and the activations fewer. (With the wrong split of L1 and shared memory, which
     depended on the activations' size, one row took 80 us here and eight 54.)"""
