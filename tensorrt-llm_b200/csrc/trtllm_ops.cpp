@@ -292,14 +292,6 @@ TORCH_LIBRARY_IMPL(trtllm, CPU, m)
     m.impl("pack_int8_tensor_to_packed_int4", &pack_int8_tensor_to_packed_int4);
 }
 
-// The GEMM ops have no gradient: pass the autograd key by. (Without a registration the call goes through
-// the boxed fallback, which does the same and takes half a microsecond for it.)
-TORCH_LIBRARY_IMPL(trtllm, AutogradCUDA, m)
-{
-    m.impl("weight_only_quant_gemm", torch::CppFunction::makeFallthrough());
-    m.impl("weight_only_groupwise_quant_gemm", torch::CppFunction::makeFallthrough());
-}
-
 TORCH_LIBRARY_IMPL(trtllm, CUDA, m)
 {
     m.impl("weight_only_quant_gemm", &weight_only_quant_gemm);

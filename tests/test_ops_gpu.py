@@ -224,6 +224,24 @@ def test_w4a8_awq_layer(dtype, m):
         assert torch.equal(out3, out)
 
 
+@pytest.mark.parametrize("grouped", [False, True])
+def test_torch_op_has_no_gradient_and_says_so(grouped):
+    """An output of an input that wants a gradient is not silently detached: backward through it warns."""
+    p = make_problem(2, 256, 512, 4, 128 if grouped else 0, torch.bfloat16, seed=1)
+    act = _d(p["act"]).requires_grad_()
+    if grouped:
+        call = lambda: torch.ops.trtllm.weight_only_groupwise_quant_gemm(act, None, _d(p["processed"]), _d(p["scales"]), None,
+                                                                         None, 1.0, 0, 128)
+    else:
+        call = lambda: torch.ops.trtllm.weight_only_quant_gemm(act, _d(p["processed"]), _d(p["scales"]), 2)
+    out = call()
+    assert out.requires_grad
+    with pytest.warns(UserWarning, match="autograd kernel was not registered"):
+        out.sum().backward()
+    with torch.no_grad():
+        assert not call().requires_grad
+
+
 def test_debug_log_names_the_kernel_taken(capfd):
     """At DEBUG the library prints one line per launch: the shape and which kernel ran."""
     lib = pkg._lib.lib()
