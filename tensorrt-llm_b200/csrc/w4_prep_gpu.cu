@@ -396,8 +396,9 @@ struct StripArgs
     int tiles_cta; // 64-row tiles per CTA, the last one may have fewer (or none)
 };
 
-// max(|a|, |b|) of eight weights as they lie in memory: kept packed.
-template <typename W>
+// max(|a|, |b|) of eight weights as they lie in memory: kept packed. NAN_TOO: a NaN stays (the same instruction's
+// other form), otherwise the number beside it is taken.
+template <typename W, bool NAN_TOO>
 struct StripMax
 {
     using W2 = typename std::conditional<std::is_same<W, __half>::value, __half2, __nv_bfloat162>::type;
@@ -413,7 +414,8 @@ struct StripMax
         uint32_t const w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            m[i] = __hmax2(m[i], __habs2(*reinterpret_cast<W2 const*>(&w[i])));
+            m[i] = NAN_TOO ? __hmax2_nan(m[i], __habs2(*reinterpret_cast<W2 const*>(&w[i])))
+                           : __hmax2(m[i], __habs2(*reinterpret_cast<W2 const*>(&w[i])));
     }
     __device__ __forceinline__ void get(float (&x)[8]) const
     {
@@ -481,10 +483,10 @@ template <typename W>
 struct StripScales
 {
     float s[8], inv[8];
-    bool extreme; // some scale is near underflow or overflow: divide
-    __device__ __forceinline__ void load(float const* scale)
+    bool extreme; // some scale is near underflow or overflow, or a weight may be no number: divide
+    __device__ __forceinline__ void load(float const* scale, bool has_nan)
     {
-        extreme = false;
+        extreme = has_nan;
 #pragma unroll
         for (int e = 0; e < 8; ++e)
         {
@@ -509,7 +511,7 @@ __device__ __forceinline__ float quantize_boundary(float x, float s, float inv)
     float const a = fabsf(x), m = (fmaf(a, inv, -0.5f) + kRound) - kRound;
     float const half_u = __uint_as_float((__float_as_uint(m + 0.5f) - 1u) & 0x7f800000u) * 0x1p-24f;
     bool const up = fmaf(-m, s, a) - 0.5f * s >= -half_u * s && a > 0.f;
-    return fminf(copysignf(m + (up ? 1.f : 0.f), x), BITS == 8 ? 127.f : 7.f);
+    return x == x ? fminf(copysignf(m + (up ? 1.f : 0.f), x), BITS == 8 ? 127.f : 7.f) : 0.f;
 }
 
 // Eight weights of a row: q = clamp(round-half-away(fl(x / s))).
@@ -521,6 +523,7 @@ __device__ __forceinline__ float quantize_boundary(float x, float s, float inv)
 // is on one).
 // fp32 weights: the product with the reciprocal decides wherever it is not within 1e-4 of a half-integer
 // (its error is 2.3e-5 at most; NaNs are not away from one), else the comparison above.
+// A NaN becomes 0: the division's conversion to an integer gives that, the comparison says so.
 template <typename W, int BITS>
 __device__ __forceinline__ void quantize8(float const (&x)[8], StripScales<W> const& c, uint32_t (&word)[BITS / 4])
 {
@@ -572,7 +575,7 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     __shared__ float amax[S];
     __shared__ float scale_s[S];
     __shared__ __align__(8) uint64_t full[kMaxStripTiles];
-    __shared__ int failed;
+    __shared__ int failed, has_nan;
 
     uint32_t rank, ranks;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -583,6 +586,7 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     if (tid == 0)
     {
         failed = 0;
+        has_nan = 0;
         for (int i = 0; i < tiles; ++i)
             mbar_init(&full[i], 1);
         mbar_fence_init();
@@ -620,7 +624,7 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     }
     else
     {
-        StripMax<W> pm;
+        StripMax<W, true> pm;
         pm.clear();
         for (int i = 0; i < tiles && ok; ++i)
         {
@@ -629,6 +633,21 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
                 pm.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
         }
         pm.get(m);
+        bool nan = false;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            nan |= m[e] != m[e];
+        if (nan)
+        {
+            // once more without them; the threads that quantise this CTA's rows divide
+            has_nan = 1;
+            StripMax<W, false> numbers;
+            numbers.clear();
+            for (int i = 0; i < tiles && ok; ++i)
+                for (int r = tid / NV; r < 64; r += int(blockDim.x) / NV)
+                    numbers.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
+            numbers.get(m);
+        }
     }
     if (!ok)
         failed = 1;
@@ -697,7 +716,7 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     if (inside)
     {
         StripScales<W> sc;
-        sc.load(scale_s + cv * 8);
+        sc.load(scale_s + cv * 8, has_nan != 0);
 #pragma unroll 1
         for (int u = tid / NV; u < blocks * 4; u += int(blockDim.x) / NV)
         {

@@ -31,3 +31,21 @@ def test_strip_shapes(k, n, dtype, bits):
     assert torch.equal(s.cpu().float(), s_ref.float())
     assert torch.equal(u.cpu(), u_ref)
     assert torch.equal(p.cpu(), p_ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("k,bits", [(576, 4), (576, 8), (4672, 4), (9280, 8)])
+def test_not_a_number(k, bits, dtype):
+    """A NaN quantises to 0 and does not count for its column's scale."""
+    torch.manual_seed(k)
+    w = (torch.randn(k, 64) * 0.02).to(dtype)
+    nan = torch.zeros(k, 64, dtype=torch.bool)
+    nan[torch.randint(0, k, (40,)), torch.randint(0, 48, (40,))] = True
+    nan[:, 50] = True  # a whole column
+    nan[3, 51] = True  # in a column of zeros
+    w[:, 51] = 0
+    u_ref, p_ref, s_ref = o.symmetric_quantize(w.masked_fill(nan, 0), bits)
+    u, p, s = Q.symmetric_quantize_last_axis_of_batched_matrix_cuda(
+        w.masked_fill(nan, float("nan")).cuda(), torch.int8 if bits == 8 else torch.quint4x2, return_unprocessed=True)
+    assert torch.equal(s.cpu().float(), s_ref.float())
+    assert torch.equal(u.cpu(), u_ref) and torch.equal(p.cpu(), p_ref)
