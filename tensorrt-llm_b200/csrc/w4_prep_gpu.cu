@@ -592,7 +592,8 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
         mbar_fence_init();
     }
     __syncthreads();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // No griddepcontrol.launch_dependents: a GEMM behind the next kernel may take the weights that are written here for
+    // static, and fetches those as soon as the kernel in front of it lets it.
     asm volatile("griddepcontrol.wait;" ::: "memory"); // the weights, and what the outputs held before
     if (tid == 0)
         for (int i = 0; i < tiles; ++i)

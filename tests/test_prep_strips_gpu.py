@@ -1,7 +1,10 @@
 """The one-pass device quantiser where its strips, clusters and rounding can go wrong (needs a B200)."""
+import ctypes
+
 import pytest
 import torch
 
+import tensorrt_llm_b200 as pkg
 from oracle import woq_oracle as o
 from tensorrt_llm_b200 import quantize as Q
 
@@ -49,3 +52,37 @@ def test_not_a_number(k, bits, dtype):
         w.masked_fill(nan, float("nan")).cuda(), torch.int8 if bits == 8 else torch.quint4x2, return_unprocessed=True)
     assert torch.equal(s.cpu().float(), s_ref.float())
     assert torch.equal(u.cpu(), u_ref) and torch.equal(p.cpu(), p_ref)
+
+
+def test_gemm_two_launches_behind_the_quantiser():
+    """A layer whose weights were quantised before the preceding GEMM was enqueued may fetch them while that one
+    runs: they have to be complete by then. (In a graph, so that launches follow each other closely; the last few
+    columns are quantised when most of the chip has run empty.)"""
+    k, n = 4096, 14336
+    g = torch.Generator(device="cuda").manual_seed(1)
+    ws = [(torch.randn(k, n, generator=g, device="cuda") * 0.02).bfloat16() for _ in range(3)]
+    act = torch.randn(1, k, generator=g, device="cuda").bfloat16()
+    other = Q.symmetric_quantize_last_axis_of_batched_matrix_cuda(ws[0][:, :64].contiguous(), torch.quint4x2)
+    call = lambda p, s, out: pkg.ops.gemm_raw(act, p, s, out, n=out.numel(), k=k, weight_bits=4, group_size=0, weights_static=True)
+    want = torch.empty(3, n, device="cuda", dtype=torch.bfloat16)
+    for i, w in enumerate(ws):
+        p, s = Q.symmetric_quantize_last_axis_of_batched_matrix_cuda(w, torch.quint4x2)
+        torch.cuda.synchronize()
+        call(p, s, want[i])
+    lib, got = pkg._lib.lib(), torch.zeros(30, n, device="cuda", dtype=torch.bfloat16)
+    scales, scales_t = torch.empty(n, device="cuda"), torch.empty(n, device="cuda", dtype=torch.bfloat16)
+    processed, small = torch.empty_like(p), torch.empty(64, device="cuda", dtype=torch.bfloat16)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        for i in range(30):
+            rc = lib.w4_symmetric_quantize_device(ptr(processed), None, ptr(scales), ptr(scales_t), pkg._lib.W4_DTYPE_BF16,
+                                                  ptr(ws[i % 3]), pkg._lib.W4_DTYPE_BF16, k, n, 4, stream)
+            assert rc == 0
+            call(*other, small)
+            call(processed, scales_t, got[i])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(got[i], want[i % 3]) for i in range(30))
