@@ -268,8 +268,11 @@ bool rounds_weights_anyway(W4GemmParams const& p)
 }
 
 // An automatic launch in the decode regime: the tensor-core kernel in the forms that need no workspace, where
-// its arithmetic is the same and its estimate is 1.5 us below the decode kernel's (whose launch also costs the
-// host less), or 3 us up to 8 rows. Six rows on 6144 x 24576: 31.1 -> 24.6 us.
+// its arithmetic is the same and its estimate is 2 us below the decode kernel's. Estimates of the difference err
+// by up to 2.8 us: on eleven shapes from 4096 x 1024 to 6144 x 24576 at 1 to 16 rows this line never takes the slower
+// kernel and forgoes 1.2 us at most (4160 x 3008, eight rows); it would from 1.7 us down (8192 x 8192 at six rows 13.5
+// and 14.0). Six rows on 6144 x 24576 32.4 -> 25.7 us, one row on 1024 x 8192 7.7 -> 3.6, sixteen on 4096 x 14336
+// 18.0 -> 11.7.
 bool decode_takes_tensor_cores(W4GemmParams const& p)
 {
     if (p.act_scale || !rounds_weights_anyway(p))
@@ -277,7 +280,7 @@ bool decode_takes_tensor_cores(W4GemmParams const& p)
     w4::DeviceInfo const& dev = w4::current_device_info();
     double const decode = w4::gemv_estimate_us(p);
     return dev.num_sms > 0 && decode > 5.0
-        && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + (p.m <= 8 ? 3.0 : 1.5) < decode;
+        && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 2.0 < decode;
 }
 
 int resolve_regime(W4GemmParams const& p)
