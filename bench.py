@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Benchmark of the weight-only quantised GEMM hot path.
 
-    python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--no-sweep]
+    python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--no-sweep] [--report FILE]
 
 One "step" is one pass of the hot path over one batch: the W4A16 group-128 AWQ decode GEMM of
 BASELINE config 2 (bf16 activations [M=1, K=4096], int4 weights [4096, 14336] with bf16 scales and
@@ -16,14 +16,15 @@ the tensor-parallel Llama-3-70B layer set (column-parallel without communication
 with an all-reduce: NCCL and the library's peer-memory kernel) is timed and parity-checked in the
 same run and reported under "tp_llama70b".
 
-The JSON line also carries: "e2e" (same metric through torch.ops.trtllm with host buffers: the
+The JSON line also carries: "e2e" (same metric through the library's host entry point: the
 activations are copied from pinned host memory and the result read back inside the timed region;
 weights stay resident in HBM as they do in serving), "roofline" (achieved / measured HBM copy
-bandwidth), "cpu_baseline" (the CPU definition of the path timed on the host cores), "points"
-(every M of config 2, config 1, the prefill GEMM of config 3 with and without a pre-quant scale,
-weight preparation, split-k) and "sweep" (config 5: the Llama-3-8B shapes x weight formats x
-activation types x M = 1..8192 with the regime chosen, the roofline fraction against the bound that
-applies and a parity flag per point), and "clocks" (NVML samples taken during the timed region).
+bandwidth), "cpu_baseline" (the CPU definition of the path timed on the host cores), "clocks" (NVML
+samples taken during the timed region) and the times of "points" (every M of config 2, config 1, the
+prefill GEMM of config 3 with and without a pre-quant scale, weight preparation, split-k) and of "sweep"
+(config 5: the Llama-3-8B shapes x weight formats x activation types x M = 1..8192) in short. --report
+writes the line with both tables whole, the second with the regime chosen, the roofline fraction against
+the bound that applies and a parity flag per point, into a file (a line of 30 KB is cut by what reads it).
 
 --impl reference times the reference's CPU definition of the path (dequantise then matmul with
 torch on all host cores) on a bounded column sample of the same workload. Only that arm and the
@@ -463,16 +464,19 @@ def run_ours(args):
         "gpu_launches": args.steps,
         "roofline": {"bound": "hbm", "achieved": gbs_rank, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": gbs_rank / peaks["hbm_gbs"], "frac_of_8TBs": gbs_rank / 8000.0,
-                     "peak_source": peaks["source"], "kernel": "w4::gemv::gemv_kernel<bf16, int4, MB=1, zero, act_scale, folded>",
-                     "traffic": captured_traffic("gemv_c2_m1")},
+                     "peak_source": peaks["source"], "kernel": "w4::stream::stream_kernel<bf16, zero>",
+                     "traffic": captured_traffic("stream_c2_m1")},
         "clocks": clocks.summary(),
         "parity_err_frac_of_max": parity,
     }
 
+    report = {}
     if rank == 0 and world == 1:
-        line["points"] = extra_points(pkg, prob, device, peaks, stream)
+        report["points"] = extra_points(pkg, prob, device, peaks, stream)
+        line["points"] = short_points(report["points"])
         if not args.no_sweep:
-            line["sweep"] = sweep(pkg, device, peaks, stream)
+            report["sweep"] = sweep(pkg, device, peaks, stream)
+            line["sweep"] = short_sweep(report["sweep"])
         step, nbytes = cpu_step_fn(REF_SAMPLE_COLS)
         for _ in range(3):
             step()
@@ -490,9 +494,30 @@ def run_ours(args):
     if world > 1:
         line["tp_llama70b"] = tp_layer_set(pkg, device, rank, world, barrier, max_over_ranks)
     if rank == 0:
+        if args.report:
+            with open(args.report, "w") as f:
+                json.dump(dict(line, **report), f)
         emit_line(line)
     if use_dist:
         dist.destroy_process_group()
+
+
+def short_points(points):
+    """The times of the points alone: microseconds by name."""
+    def us(p):
+        if "us" in p:
+            return round(p["us"], 2)
+        if "ms" in p:
+            return round(p["ms"] * 1e3, 1)
+        return {k: round(v, 2) for k, v in p.items() if k.endswith("_us")} or None
+    return {name: p and us(p) for name, p in points.items()}
+
+
+def short_sweep(table):
+    slower = table["auto_not_fastest"]
+    return {"points": len(table["rows"]), "parity_all_ok": table["parity_all_ok"], "seconds": table["seconds"],
+            "auto_not_fastest": len(slower),
+            "auto_over_other_worst": round(max((s["auto_us"] / s["other_us"] for s in slower), default=1.0), 3)}
 
 
 def roofline_of(us, nbytes, flops, peaks):
@@ -523,7 +548,7 @@ def extra_points(pkg, prob, device, peaks, stream):
     points["c3_m4096"] = prefill_point(pkg, device, peaks, prequant=False)
     points["c3_m4096_prequant"] = prefill_point(pkg, device, peaks, prequant=True)
     points["prep_c2"] = prep_point(pkg, device, peaks)
-    points["splitk_m64_k8192_n1280"] = splitk_point(pkg, device)
+    points["splitk_m64_k14336_n512"] = splitk_point(pkg, device)
     return points
 
 
@@ -647,7 +672,7 @@ def prep_point(pkg, device, peaks):
     us_l = timed(lambda: Q.preprocess_weights_for_mixed_gemm_cuda(raw_d, torch.quint4x2))
     us_q = timed(lambda: Q.symmetric_quantize_last_axis_of_batched_matrix_cuda(w_d, torch.quint4x2))
     bytes_l = 2 * k * n // 2                      # read + write the packed matrix
-    bytes_q = 2 * k * n * 2 + k * n // 2          # two passes over the bf16 matrix (amax, quantise) + write
+    bytes_q = k * n * 2 + k * n // 2              # one pass over the bf16 matrix + write
     return {"layout_us": us_l, "layout_GB/s": bytes_l / us_l / 1e3,
             "layout_frac_of_measured_hbm": bytes_l / us_l / 1e3 / peaks["hbm_gbs"],
             "layout_cpu_ms_host_threads": cpu_ms,
@@ -657,16 +682,16 @@ def prep_point(pkg, device, peaks):
 
 
 def splitk_point(pkg, device):
-    """A few-tile tensor-core shape (Llama-3-70B qkv shard at tp=8, M=64) with and without the
-    optional split-k workspace, graph-timed."""
+    """A tensor-core shape of two tiles: without a workspace its k splits share a cluster, with one there may be
+    more of them than a cluster holds. Graph-timed."""
     from tensorrt_llm_b200 import ops
-    m, n, k = 64, 1280, 8192
+    m, n, k = 64, 512, 14336
     w = torch.randint(0, 256, (k, n // 2), dtype=torch.uint8, device=device).view(torch.int8)
     s = (torch.rand(k // 128, n, device=device) * 0.019 + 0.001).to(torch.bfloat16)
     act = torch.randn(m, k, device=device).to(torch.bfloat16)
     out = torch.empty(m, n, dtype=torch.bfloat16, device=device)
     res = {}
-    for label, nb in (("unsplit_us", 0), ("split_us", ops.workspace_bytes(m, n, k, 128, 4, torch.bfloat16, False,
+    for label, nb in (("cluster_us", 0), ("workspace_us", ops.workspace_bytes(m, n, k, 128, 4, torch.bfloat16, False,
                                                                            pkg.W4_REGIME_GEMM))):
         ws = torch.empty(nb, dtype=torch.uint8, device=device) if nb else None
         st = torch.cuda.Stream(device=device)
@@ -902,6 +927,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=10)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--no-sweep", action="store_true", help="skip the config-5 sweep (about half a minute)")
+    ap.add_argument("--report", help="file for the line with the whole tables in it")
     args = ap.parse_args()
     args.steps = max(1, min(args.steps, 20000))
     args.warmup = max(0, args.warmup)
