@@ -75,12 +75,12 @@ struct Args
     int group_shift; // log2(group size), 31 = per-channel
     int bm;          // activation rows per tile
     int tiles_n;
-    // Experts (an ordinary GEMM is one): expert e has rows first_row[e] .. row_end[e] - 1 of the
+    // Experts (an ordinary GEMM is one): expert e has rows first_row[e] .. first_row[e + 1] - 1 of the
     // activations and of the output, tiles first_tile[e] .. first_tile[e + 1] - 1, the weights, scales and zeros
     // of slice slice[e] of their tensors, and bias + slice[e] * n.
     int num_experts;
     int groups; // scale rows per expert
-    int first_row[kMaxExperts], row_end[kMaxExperts], first_tile[kMaxExperts + 1], slice[kMaxExperts];
+    int first_row[kMaxExperts + 1], first_tile[kMaxExperts + 1], slice[kMaxExperts];
     int num_stages, num_wstages;
     int d_bufs;      // accumulators in TMEM: 2 up to 128 rows, else 1
     int weights_static;
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         int const t = tile - a.first_tile[e], tm = t / a.tiles_n;
         it.n0 = (t - tm * a.tiles_n) * kPairN;
         it.row0 = a.first_row[e] + tm * a.bm;
-        it.row_end = a.row_end[e];
+        it.row_end = a.first_row[e + 1];
         it.slice = a.slice[e];
         return it;
     };
@@ -910,11 +910,18 @@ static int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t sm
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
 }
 
-// The experts of a launch, out of the `slices` of the weight tensor.
+// The experts of a launch: neighbours, out of the `slices` of the weight tensor, that have rows. Those that are
+// computed elsewhere get no tiles.
 struct Experts
 {
     int num, slices;
-    int slice[kMaxExperts], first_row[kMaxExperts], row_end[kMaxExperts];
+    int slice[kMaxExperts], first_row[kMaxExperts + 1];
+    bool elsewhere[kMaxExperts];
+
+    int rows(int e) const
+    {
+        return elsewhere[e] ? 0 : first_row[e + 1] - first_row[e];
+    }
 };
 
 template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
@@ -941,9 +948,9 @@ static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex,
     {
         a.slice[e] = ex.slice[e];
         a.first_row[e] = ex.first_row[e];
-        a.row_end[e] = ex.row_end[e];
-        a.first_tile[e + 1] = a.first_tile[e] + (ex.row_end[e] - ex.first_row[e] + plan.bm - 1) / plan.bm * a.tiles_n;
+        a.first_tile[e + 1] = a.first_tile[e] + (ex.rows(e) + plan.bm - 1) / plan.bm * a.tiles_n;
     }
+    a.first_row[ex.num] = ex.first_row[ex.num];
     a.weights_static = (p.flags & W4_GEMM_WEIGHTS_STATIC) ? 1 : 0;
     a.splits = plan.splits;
     a.steps_split = plan.steps_split;
@@ -1022,7 +1029,7 @@ static int dispatch_split(W4GemmParams const& p, void const* act, Experts const&
 {
     int rows[kMaxExperts];
     for (int e = 0; e < ex.num; ++e)
-        rows[e] = ex.row_end[e] - ex.first_row[e];
+        rows[e] = ex.rows(e);
     // The form of split-k that uses the caller's workspace needs room for the partial tiles there, and its second
     // kernel adds up and stores all p.m rows with one bias: not for the experts of a 3-D weight, also where a
     // launch has one expert only.
@@ -1104,7 +1111,9 @@ static double step_us(int bm, int bits, int act_dtype)
 // accumulators hide all but the last. Splits that share a cluster add the exchange of the partial tiles
 // (clusters of 4 and 8 CTAs about 1 us; 6 and more than 8 wait longer for enough free SMs side by side), splits
 // through the workspace a second kernel and their traffic. Fitted to 4096 and 8192 x 1024..14336 at 16 to
-// 777 rows: within 1 us of the best plan found by trying all at 14 of 16 points.
+// 777 rows, each launch by itself: within 1 us of the best plan found by trying all at 14 of 16 points. Beyond
+// that, and in long runs at the power limit, it is too low (14336 x 4096 at 4096 rows 228 us, measured 302 cool
+// and 356 sustained) and says only which row tile has the fewest waves.
 TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace)
 {
     int const pairs = num_sms > 1 ? num_sms / 2 : 1;
@@ -1184,7 +1193,7 @@ int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream)
             return rc;
         act = p.workspace;
     }
-    tc::Experts const one{1, 1, {0}, {0}, {p.m}};
+    tc::Experts const one{1, 1, {0}, {0, p.m}, {false}};
     return p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, act, one, dev, stream)
                                         : tc::dispatch<__nv_bfloat16>(p, act, one, dev, stream);
 }
@@ -1197,22 +1206,29 @@ int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* fi
         return W4_ERR_CUDA;
     tc::Experts ex{};
     ex.slices = num_experts;
+    bool any = false;
     for (int e = 0; e < num_experts; ++e)
     {
-        if (joins(p, first_row[e + 1] - first_row[e]))
+        int const rows = first_row[e + 1] - first_row[e];
+        if (rows > 0)
         {
             ex.slice[ex.num] = e;
             ex.first_row[ex.num] = first_row[e];
-            ex.row_end[ex.num++] = first_row[e + 1];
+            ex.elsewhere[ex.num] = !joins(p, rows);
+            any |= !ex.elsewhere[ex.num];
+            ex.first_row[++ex.num] = first_row[e + 1];
         }
-        if (ex.num == tc::kMaxExperts || (e + 1 == num_experts && ex.num > 0))
+        if (ex.num < tc::kMaxExperts && e + 1 < num_experts)
+            continue;
+        if (any)
         {
             int const rc = p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, p.act, ex, dev, stream)
                                                         : tc::dispatch<__nv_bfloat16>(p, p.act, ex, dev, stream);
             if (rc != W4_OK)
                 return rc;
-            ex.num = 0;
         }
+        ex.num = 0;
+        any = false;
     }
     return W4_OK;
 }

@@ -52,9 +52,9 @@ int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream);
 // Workspace: the minimum the kernel needs (scaled activation copy), and what also allows split-k.
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale);
 size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits, int act_dtype);
-// The experts of a 3-D weight tensor in one launch (every 32 of those that joins() with their rows): p.m is the
-// end of the last expert's rows, expert e has rows first_row[e] .. first_row[e + 1] - 1. No pre-quant scale, no
-// workspace.
+// Those experts of a 3-D weight tensor that joins() with their rows, in one launch for every 32 that have rows: p.m
+// is the end of the last expert's rows, expert e has rows first_row[e] .. first_row[e + 1] - 1. No pre-quant scale,
+// no workspace.
 int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, bool (*joins)(W4GemmParams const&, int),
     cudaStream_t stream);
 // How the tensor-core kernel runs a problem (or the experts of one, by their rows): activation rows per tile,
