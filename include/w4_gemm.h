@@ -98,7 +98,7 @@ extern "C"
     enum
     {
         W4_REGIME_AUTO = 0,
-        W4_REGIME_GEMV = 1, /* streaming decode kernel, any m (re-streams the weights every 8 rows) */
+        W4_REGIME_GEMV = 1, /* decode kernels, any m (the weights are read again for every 16 rows) */
         W4_REGIME_GEMM = 2  /* tcgen05 tensor-core kernel */
     };
 
@@ -116,10 +116,10 @@ extern "C"
      * W4GemmParams.flags.
      * W4_GEMM_WEIGHTS_STATIC: weight, scales, zeros and act_scale were completely written before the
      * kernel that precedes this GEMM on the stream was launched (true for inference weights, which
-     * are written once at load time). The decode kernel is a programmatic dependent launch: with
-     * this bit it starts fetching those tensors while the preceding kernel is still running and
-     * waits for that kernel only before it reads `act` and writes `out`. Without the bit it waits
-     * before its first fetch, which is always safe - set it only when the statement above holds
+     * are written once at load time). The GEMM kernels are programmatic dependent launches: with
+     * this bit they start fetching those tensors while the preceding kernel is still running and
+     * wait for that kernel only before they read `act` and write `out`. Without the bit they wait
+     * before their first fetch, which is always safe - set it only when the statement above holds
      * (it does NOT hold for a GEMM enqueued right behind w4_symmetric_quantize_device,
      * w4_preprocess_weights_device or any other kernel that writes the weights).
      */
@@ -258,7 +258,8 @@ extern "C"
      * tensor-core kernel and keeps that kernel's scratch - the activations multiplied by the AWQ
      * pre-quant scale, m * k * 2 bytes, and, for shapes with few output tiles when the rest of the
      * array has room, the fp32 partial tiles of its split-k behind them - in a
-     * W4_STATIC_SCRATCH_BYTES (8 MiB) array that is part of the library image. This entry point has no counterpart in the reference.
+     * W4_STATIC_SCRATCH_BYTES (8 MiB) array that is part of the library image. This entry point has no
+     * counterpart in the reference.
      *   - p->workspace / p->workspace_bytes are ignored; nothing is allocated or freed, here or
      *     in any library it calls.
      *   - m * k * 2 > W4_STATIC_SCRATCH_BYTES with act_scale set returns W4_ERR_STATIC_SCRATCH

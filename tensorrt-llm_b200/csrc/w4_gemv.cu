@@ -1,4 +1,6 @@
-// Decode-regime kernel (m = 1..8 or 9..16 per pass): streams the packed int4/int8 weights exactly once.
+// Decode-regime kernel, staged form (m = 1..8 or 9..16 per pass): streams the packed int4/int8 weights exactly
+// once. int4 with 128-wide groups or one scale per column and few rows may run w4_gemv_stream.cu instead
+// (launch_gemv below).
 //
 // Replaces weight_only::kernel of the reference project
 // (cpp/tensorrt_llm/kernels/weightOnlyBatchedGemv/kernel.h:31-120) and, for m >= 5 / m >= 16, the
@@ -1104,6 +1106,8 @@ static double streamed_us(W4GemmParams const& p)
         + (p.m * p.k > 100000 ? 1.0 : 0.0);
 }
 
+// The two estimates choose the kernel (launch_gemv): on 18 shapes from 4096 x 1024 to 8192 x 57344 at 1 to 8 rows the
+// chosen one takes 0.35 % longer in all than always the faster, and 0.85 us at most (4096 x 14336 at four rows).
 double gemv_estimate_us(W4GemmParams const& p)
 {
     double const a = staged_us(p), b = streamed_us(p);

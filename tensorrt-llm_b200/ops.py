@@ -44,7 +44,8 @@ def _require_cuda(t: torch.Tensor, name: str):
 
 
 def select_regime(m: int, n: int, k: int, group_size: int, weight_bits: int, dtype: torch.dtype = torch.float16) -> int:
-    """The kernel an automatic launch takes for this problem (activation type included)."""
+    """The regime of an automatic launch of this problem (activation type included): what workspace it needs and
+    how weights are rounded."""
     return _lib.lib().w4_gemm_select_regime_typed(m, n, k, group_size, weight_bits, _DTYPES[dtype])
 
 
@@ -102,7 +103,7 @@ def moe_gemm(act, weight, scales, expert_first_row: Sequence[int], *, weight_bit
         return out
     rows = [b - a for a, b in zip(first[:-1], first[1:]) if b > a]
     ws = None
-    if len(rows) == 1 or act_scale is not None:  # otherwise one launch that needs no workspace
+    if len(rows) == 1 or act_scale is not None:  # otherwise decode launches and a shared one, which need none
         nws = workspace_bytes_max(max(rows), n, k, group_size, weight_bits, act.dtype, act_scale is not None)
         ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=act.device)
     params = W4GemmParams(

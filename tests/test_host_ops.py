@@ -187,7 +187,6 @@ def test_experts_refuse_bad_shapes_before_anything_is_estimated():
     assert [call(n=0), call(k=0), call(n=-64), call(k=96), call(weight_bits=3), call(act=24)] == [-2, -2, -2, -2, -4, -5]
 
 
-
 def test_regime_heuristic_knows_the_activation_type(lib):
     """int8 weights with bf16 activations: a decode pass costs more (two nibble planes), so two
     16-row passes over a small matrix lose to the tensor-core kernel where float16 still takes them
