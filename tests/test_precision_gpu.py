@@ -25,7 +25,13 @@ def test_the_regime_decides_the_arithmetic(m, n, k, bits, group, dtype):
     assert torch.equal(run_gpu(p), run_gpu(p, regime=pkg.W4_REGIME_GEMV))
 
 
-@pytest.mark.parametrize("bits,group,rows", [(4, 128, [3, 16, 40, 0, 9, 120]), (8, 0, [1, 1, 64, 5]), (8, 128, [2, 7])])
+@pytest.mark.parametrize("bits,group,rows", [
+    (4, 128, [3, 16, 40, 0, 9, 120]),
+    (8, 0, [1, 1, 64, 5]),
+    (8, 128, [2, 7]),
+    (4, 128, [1, 64] * 20),             # more than one launch's experts, every other computed elsewhere
+    (4, 64, [3, 16, 40, 0, 9, 120]),    # rounded alike in both regimes: any kernel may take any of them
+])
 def test_experts_have_the_arithmetic_of_their_own_regime(bits, group, rows):
     n, k, dtype = 1024, 2048, torch.bfloat16
     first = [0]
@@ -42,7 +48,7 @@ def test_experts_have_the_arithmetic_of_their_own_regime(bits, group, rows):
             continue
         got, regime = out[first[e]:first[e + 1]], pkg.ops.select_regime(r, n, k, group, bits, dtype)
         regimes.add(regime)
-        if regime == pkg.W4_REGIME_GEMV:
+        if regime == pkg.W4_REGIME_GEMV and (bits, group) != (4, 64):
             assert torch.equal(got, run_gpu(p, regime=regime)), e
         else:
             ref = oracle_out(p)
