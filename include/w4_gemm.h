@@ -92,9 +92,10 @@ extern "C"
 
     /* Which kernel family runs. AUTO applies w4_gemm_select_regime(). The regime also decides the arithmetic: the
      * decode kernels apply scales and zeros to 32-bit sums, the tensor-core kernel multiplies with weights that
-     * were scaled and rounded to the activation type first, as the reference's kernels do. (int4 with 64-wide
-     * groups is rounded that way in both, and there an automatic launch in the decode regime may run the
-     * tensor-core kernel, without a workspace.) */
+     * were scaled and rounded to the activation type first, as the reference's kernels do (with one scale per column
+     * and no zeros it multiplies the integers and scales the sums). An automatic launch in the decode regime may run
+     * the tensor-core kernel too where that is faster, without a workspace and with scales and zeros applied to
+     * 32-bit sums; int4 with 64-wide groups is rounded either way. */
     enum
     {
         W4_REGIME_AUTO = 0,
@@ -143,7 +144,8 @@ extern "C"
      *   n          the real number of output features (not the packed extent)
      *   workspace  scratch of w4_gemm_workspace_bytes(); may be NULL when that is 0. Mandatory only when
      *              act_scale is set and the tensor-core kernel runs (m*k*2 bytes); the rest lets that
-     *              kernel split k over idle SMs and is optional (smaller: it runs unsplit)
+     *              kernel cut k anywhere and is optional (smaller: it does without). What it holds before a launch
+     *              does not matter; launches that may overlap on the GPU need one each
      */
     typedef struct W4GemmParams
     {
@@ -188,9 +190,9 @@ extern "C"
 
     /*
      * The GEMMs of all experts of a mixture-of-experts layer over 3-D weights. Every expert is computed in the
-     * regime of its own rows; those in the tensor-core kernel's regime, if there are two or more, share launches
-     * of up to 32 experts, the others (all, with a pre-quant scale or a requested regime) are one
-     * w4_gemm_launch after another. p describes expert 0: weight is [E][K, N*bits/8], every expert's matrix laid
+     * regime of its own rows, as far as the arithmetic goes; two or more share launches of up to 32 experts of the
+     * tensor-core kernel where that is faster, the others (all, with a pre-quant scale or a requested regime)
+     * are one w4_gemm_launch after another. p describes expert 0: weight is [E][K, N*bits/8], every expert's matrix laid
      * out on its own - what preprocess_weights_for_mixed_gemm does with a 3-D tensor
      * (cpp/tensorrt_llm/thop/weightOnlyQuantOp.cpp:136-147, force_interleave); scales / zeros are
      * [E][K/G, N] (or [E][N]), bias [E][N]; act_scale [K] is shared. The rows of act and out are sorted
@@ -198,8 +200,9 @@ extern "C"
      * num_experts + 1 non-decreasing ints starting at 0; the running totals the reference's MoE GEMM
      * takes as total_tokens_including_expert,
      * cpp/tensorrt_llm/kernels/internal_cutlass_kernels/include/moe_gemm_kernels.h:236, kept on the host).
-     * p->m is ignored; the workspace serves one expert at a time, never a shared launch, and must then cover the
-     * largest per-expert row count (w4_gemm_workspace_bytes_max). Experts without rows are skipped. Returns the
+     * p->m is ignored; the workspace, for experts that are launched one after another, has to cover the largest
+     * per-expert row count (w4_gemm_workspace_bytes_max); a shared launch needs none and uses what there is for partial
+     * tiles (4 MiB for experts of up to 32 rows). Experts without rows are skipped. Returns the
      * first error.
      */
     int w4_gemm_launch_experts(const W4GemmParams* p, int num_experts, const int* expert_first_row, void* stream);
@@ -207,6 +210,12 @@ extern "C"
     /* Bytes of scratch w4_gemm_launch needs for this problem in the regime it would pick. */
     size_t w4_gemm_workspace_bytes(int m, int n, int k, int group_size, int weight_bits, int act_dtype,
         int has_act_scale, int regime);
+
+    /* Bytes of workspace with which w4_gemm_launch(p) runs its fastest form, for callers that allocate per call; never
+     * less than it needs. Reads m, n, k, group_size, weight_bits, act_dtype, regime and which of act_scale and zeros
+     * are given. In the decode regime, which needs none, it can be more than w4_gemm_workspace_bytes() (0 there): the
+     * tensor-core kernel, where it is the faster one, cuts the k range anywhere if it has room for partial tiles. */
+    size_t w4_gemm_workspace_wanted(const W4GemmParams* p);
 
     /* The largest w4_gemm_workspace_bytes() over m = 1..max_m: what a plugin reserves at configure
      * time (getWorkspaceSize), since the optional split-k part peaks at small m, not at max_m. */

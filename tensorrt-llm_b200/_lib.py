@@ -26,7 +26,7 @@ EXPORTS = (
     "w4_pack_int4", "w4_unpack_int4", "w4_gemm_launch_static_scratch", "w4_gemm_static_scratch_bytes",
     "w4_preprocess_weights_device", "w4_symmetric_quantize_device", "w4_allreduce", "w4_allreduce_emulated",
     "w4_allreduce_workspace_bytes",
-    "w4_gemm_workspace_bytes_max", "w4_gemm_run_host", "w4_gemm_launch_experts",
+    "w4_gemm_workspace_bytes_max", "w4_gemm_workspace_wanted", "w4_gemm_run_host", "w4_gemm_launch_experts",
     "w4_preprocess_weights_w4a8", "w4_relayout_w4a8_to_w4a16", "w4_gemm_launch_push", "w4_gemm_allreduce",
     "w4_relayout_w4a8_to_w4a16_device", "w4_set_log_level", "w4_get_log_level",
     "w4_gemm_select_regime_typed",
@@ -92,6 +92,8 @@ def lib() -> ctypes.CDLL:
         l.w4_gemm_static_scratch_bytes.restype = ctypes.c_size_t
         l.w4_gemm_workspace_bytes.restype = ctypes.c_size_t
         l.w4_gemm_workspace_bytes.argtypes = [ctypes.c_int] * 8
+        l.w4_gemm_workspace_wanted.restype = ctypes.c_size_t
+        l.w4_gemm_workspace_wanted.argtypes = [ctypes.POINTER(W4GemmParams)]
         l.w4_gemm_workspace_bytes_max.restype = ctypes.c_size_t
         l.w4_gemm_workspace_bytes_max.argtypes = [ctypes.c_int] * 7
         l.w4_gemm_select_regime.argtypes = [ctypes.c_int] * 5

@@ -196,12 +196,6 @@ Tensor run_gemm(Tensor const& act, Tensor const& weight, Tensor const& scales, v
         return out;
 
     auto const stream = at::cuda::getCurrentCUDAStream(act.device().index());
-    size_t const ws_bytes = w4_gemm_workspace_bytes(int(m), int(n), int(k), group_size, bits, dt, act_scale != nullptr,
-        W4_REGIME_AUTO);
-    Tensor ws;
-    if (ws_bytes)
-        ws = empty_on(act, {int64_t(ws_bytes)}, at::kByte);
-
     W4GemmParams p{};
     p.act = act.data_ptr();
     p.act_scale = act_scale;
@@ -218,9 +212,15 @@ Tensor run_gemm(Tensor const& act, Tensor const& weight, Tensor const& scales, v
     p.weight_bits = bits;
     p.act_dtype = dt;
     p.regime = W4_REGIME_AUTO;
-    p.workspace = ws_bytes ? ws.data_ptr() : nullptr;
-    p.workspace_bytes = ws_bytes;
     p.flags = weights_static ? W4_GEMM_WEIGHTS_STATIC : 0u;
+    size_t const ws_bytes = w4_gemm_workspace_wanted(&p);
+    Tensor ws;
+    if (ws_bytes)
+    {
+        ws = empty_on(act, {int64_t(ws_bytes)}, at::kByte);
+        p.workspace = ws.data_ptr();
+        p.workspace_bytes = ws_bytes;
+    }
     check_status(w4_gemm_launch(&p, stream.stream()), "w4_gemm_launch");
     return out;
 }

@@ -262,27 +262,33 @@ double regime_prefill_us(int m, int n, int k, int num_sms, int weight_bits)
 
 // The regime also decides the arithmetic: decode kernels apply scales and zeros to 32-bit sums, the tensor-core
 // kernel rounds every scaled weight to the activation type first (outputs 2.3e-3 of their size from the exact
-// ones instead of 1.7e-3 for bf16, 2.9e-4 instead of 2.1e-4 for fp16). With 64-wide groups on int4 both round, so
-// that there the decode regime may take either.
+// ones instead of 1.7e-3 for bf16, 2.9e-4 instead of 2.1e-4 for fp16), unless it is asked not to or there is nothing to
+// round (one scale per column, no zeros). With 64-wide groups on int4 the decode kernel rounds as well, so that there
+// the decode regime may take either.
 bool rounds_weights_anyway(W4GemmParams const& p)
 {
     return p.weight_bits == 4 && p.group_size == 64;
 }
 
-// An automatic launch in the decode regime: the tensor-core kernel in the forms that need no workspace, where
-// its arithmetic is the same and its estimate is 2 us below the decode kernel's. Estimates of the difference err
-// by up to 2.8 us: on eleven shapes from 4096 x 1024 to 6144 x 24576 at 1 to 16 rows this line never takes the slower
-// kernel and forgoes 1.2 us at most (4160 x 3008, eight rows); it would from 1.7 us down (8192 x 8192 at six rows 13.5
-// and 14.0). Six rows on 6144 x 24576 32.4 -> 25.7 us, one row on 1024 x 8192 7.7 -> 3.6, sixteen on 4096 x 14336
-// 18.0 -> 11.7.
+// The tensor-core kernel's arithmetic for an automatic launch in the decode regime.
+bool wants_exact(W4GemmParams const& p)
+{
+    return !rounds_weights_anyway(p);
+}
+
+// A launch in the decode regime: the tensor-core kernel, with arithmetic that is no coarser, where its
+// estimate is kTakeUs below the decode kernel's. (It needs no workspace; with one it has more forms to choose from.)
+constexpr double kTakeUs = 1.0;
+
 bool decode_takes_tensor_cores(W4GemmParams const& p)
 {
-    if (p.act_scale || !rounds_weights_anyway(p))
+    if (p.act_scale || (p.weight_bits == 4 && p.group_size == 128 && p.m <= 8)) // (the streaming kernel's: never)
         return false;
     w4::DeviceInfo const& dev = w4::current_device_info();
     double const decode = w4::gemv_estimate_us(p);
-    return dev.num_sms > 0 && decode > 5.0
-        && w4::gemm_tc_plan(&p.m, 1, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us + 2.0 < decode;
+    size_t const room = p.workspace ? p.workspace_bytes : 0;
+    return dev.num_sms > 0 && decode > 4.5
+        && w4::gemm_tc_plan(&p.m, 1, p, w4::gemm_tc_mode(p, wants_exact(p)), dev.num_sms, room).us + kTakeUs < decode;
 }
 
 int resolve_regime(W4GemmParams const& p)
@@ -292,13 +298,18 @@ int resolve_regime(W4GemmParams const& p)
     return auto_regime(p.m, p.n, p.k, p.group_size, p.weight_bits, p.act_dtype);
 }
 
-// Whether the launch runs the decode kernel.
+// Whether the launch runs a decode kernel. Automatic and requested launches in the decode regime choose alike, so that
+// one is the other bit for bit; W4_FORCE_REGIME=gemv is the way to have the decode kernels whatever they take.
 bool takes_decode_kernel(W4GemmParams const& p)
 {
     if (resolve_regime(p) != W4_REGIME_GEMV)
         return false;
-    bool const chosen = p.regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO;
-    return !(chosen && decode_takes_tensor_cores(p));
+    return forced_regime() == W4_REGIME_GEMV || !decode_takes_tensor_cores(p);
+}
+
+int launch_tensor_cores(W4GemmParams const& p, cudaStream_t stream)
+{
+    return w4::launch_gemm_tc(p, stream, resolve_regime(p) == W4_REGIME_GEMV && wants_exact(p));
 }
 
 // Which experts of a layer the shared launch of the tensor-core kernel takes: those in its own regime, or all.
@@ -307,23 +318,39 @@ bool in_gemm_regime(W4GemmParams const& p, int rows)
     return rows > 0 && auto_regime(rows, p.n, p.k, p.group_size, p.weight_bits, p.act_dtype) == W4_REGIME_GEMM;
 }
 
+bool in_decode_regime(W4GemmParams const& p, int rows)
+{
+    return rows > 0 && !in_gemm_regime(p, rows);
+}
+
 bool has_rows(W4GemmParams const& p, int rows)
 {
     (void) p;
     return rows > 0;
 }
 
-// Whether one launch for all experts is estimated faster than one for those in the tensor-core kernel's regime
-// and a launch of the decode kernel for each of the others (the first 32 with rows stand for all).
-bool sharing_is_faster(W4GemmParams const& p, int num_experts, int const* first_row)
+// How the experts of a layer are launched (nothing in front of them, regime left to the library).
+enum ExpertsForm
+{
+    EXPERTS_APART,  // those in the GEMM regime in one launch of the tensor-core kernel, the others one after another
+    EXPERTS_TWO,    // the others in one of their own, with the decode regime's arithmetic
+    EXPERTS_SHARED  // all in one launch, with arithmetic that is right for all
+};
+
+// The form that is estimated fastest (the first 32 experts with rows stand for all).
+ExpertsForm experts_form(W4GemmParams const& p, int num_experts, int const* first_row)
 {
     w4::DeviceInfo const& dev = w4::current_device_info();
-    if (dev.num_sms <= 0)
-        return false;
-    auto plan_us = [&](int const* rows, int num)
-    { return num ? w4::gemm_tc_plan(rows, num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false).us : 0.0; };
+    // Experts of up to 2 MiB: a decode launch takes 3 to 4 us and overlaps its neighbours, and outputs stay bit for bit
+    // what a decode launch for the expert alone gives, which those who test such layers compare them with.
+    if (dev.num_sms <= 0 || (!rounds_weights_anyway(p) && size_t(p.k) * p.n * p.weight_bits / 8 <= (size_t(2) << 20)))
+        return EXPERTS_APART;
+    int const round = w4::gemm_tc_mode(p, false), exact = w4::gemm_tc_mode(p, wants_exact(p));
+    size_t const room = p.workspace ? p.workspace_bytes : 0;
+    auto plan_us = [&](int const* rows, int num, int mode)
+    { return num ? w4::gemm_tc_plan(rows, num, p, mode, dev.num_sms, room).us : 0.0; };
     constexpr int kMost = 32;
-    int all[kMost], large[kMost], num_all = 0, num_large = 0;
+    int all[kMost], small[kMost], large[kMost], num_all = 0, num_small = 0, num_large = 0;
     double apart = 0.0;
     for (int e = 0; e < num_experts && num_all < kMost; ++e)
     {
@@ -335,9 +362,15 @@ bool sharing_is_faster(W4GemmParams const& p, int num_experts, int const* first_
         if (in_gemm_regime(p, q.m))
             large[num_large++] = q.m;
         else
-            apart += w4::gemv_estimate_us(q);
+        {
+            small[num_small++] = q.m;
+            double const tc = plan_us(&q.m, 1, exact), decode = w4::gemv_estimate_us(q);
+            apart += tc < decode ? tc : decode;
+        }
     }
-    return plan_us(all, num_all) < apart + plan_us(large, num_large);
+    double const larger = plan_us(large, num_large, round);
+    double const us[] = {apart + larger, num_small > 1 ? plan_us(small, num_small, exact) + larger : 1e9, plan_us(all, num_all, exact)};
+    return us[2] <= us[0] && us[2] <= us[1] ? EXPERTS_SHARED : us[1] < us[0] ? EXPERTS_TWO : EXPERTS_APART;
 }
 
 void log_refusal(char const* entry, W4GemmParams const* p, int rc)
@@ -448,11 +481,22 @@ extern "C"
         return w4::gemm_tc_workspace_bytes(m, n, k, has_act_scale, weight_bits, act_dtype);
     }
 
+    size_t w4_gemm_workspace_wanted(const W4GemmParams* p)
+    {
+        if (!p || p->m <= 0)
+            return 0;
+        bool const decode = resolve_regime(*p) == W4_REGIME_GEMV;
+        W4GemmParams q = *p;
+        q.workspace = q.weight ? const_cast<void*>(q.weight) : &q; // any: only whether there is one matters here
+        q.workspace_bytes = ~size_t(0);
+        return decode && takes_decode_kernel(q) ? 0 : w4::gemm_tc_workspace(*p, decode && wants_exact(*p));
+    }
+
     size_t w4_gemm_workspace_bytes_max(int max_m, int n, int k, int group_size, int weight_bits, int act_dtype,
         int has_act_scale)
     {
         size_t best = 0;
-        // split-k is only used up to 256 rows; beyond that the size grows with m (or is zero)
+        // partial tiles are only used up to 256 rows; beyond that the size grows with m (or is zero)
         for (int m = 1; m <= max_m && m <= 256; ++m)
         {
             size_t const b = w4_gemm_workspace_bytes(m, n, k, group_size, weight_bits, act_dtype, has_act_scale,
@@ -495,7 +539,7 @@ extern "C"
                 p->m, p->n, p->k, p->weight_bits, p->group_size, p->zeros != nullptr, p->bias != nullptr,
                 p->act_scale != nullptr, double(p->alpha), gemv ? "decode kernel" : "tensor-core kernel",
                 p->regime == W4_REGIME_AUTO ? " (chosen)" : " (requested)");
-        rc = gemv ? w4::launch_gemv(*p, s) : w4::launch_gemm_tc(*p, s);
+        rc = gemv ? w4::launch_gemv(*p, s) : launch_tensor_cores(*p, s);
         if (rc != W4_OK)
             log_line(W4_LOG_ERROR, "w4_gemm_launch failed: %s (m=%d n=%d k=%d bits=%d group=%d)", w4_status_string(rc),
                 p->m, p->n, p->k, p->weight_bits, p->group_size);
@@ -571,10 +615,10 @@ extern "C"
         size_t const weight_bytes = size_t(p->k) * p->n * p->weight_bits / 8;
         auto at = [](const void* base, size_t bytes) -> const void*
         { return base ? static_cast<const char*>(base) + bytes : nullptr; };
-        // Two or more experts that the tensor-core kernel may take and nothing to do in front: those in one launch,
-        // whose work items then fill the chip together. The others one after another.
-        bool (*joins)(W4GemmParams const&, int) = in_gemm_regime;
-        int used = 0;
+        // Nothing to do in front: two or more experts share launches of the tensor-core kernel, whose work items then
+        // fill the chip together. Those that do not, one after another.
+        bool (*joins[2])(W4GemmParams const&, int) = {nullptr, nullptr};
+        bool exact[2] = {false, false};
         W4GemmParams q = *p;
         if (!p->act_scale && p->regime == W4_REGIME_AUTO && forced_regime() == W4_REGIME_AUTO)
         {
@@ -586,25 +630,33 @@ extern "C"
                 log_refusal("w4_gemm_launch_experts", p, rc);
                 return rc;
             }
-            if (rounds_weights_anyway(*p) && sharing_is_faster(*p, num_experts, expert_first_row))
-                joins = has_rows;
-            for (int e = 0; e < num_experts; ++e)
-                used += joins(*p, expert_first_row[e + 1] - expert_first_row[e]);
+            ExpertsForm const form = experts_form(*p, num_experts, expert_first_row);
+            joins[0] = form == EXPERTS_SHARED ? has_rows : in_gemm_regime;
+            exact[0] = form == EXPERTS_SHARED && wants_exact(*p);
+            if (form == EXPERTS_TWO)
+                joins[1] = in_decode_regime, exact[1] = wants_exact(*p);
         }
-        bool const shared = used > 1;
-        if (shared)
+        for (int j = 0; j < 2; ++j)
         {
+            int used = 0;
+            for (int e = 0; joins[j] && e < num_experts; ++e)
+                used += joins[j](*p, expert_first_row[e + 1] - expert_first_row[e]);
+            if (used < 2)
+            {
+                joins[j] = nullptr;
+                continue;
+            }
             if (log_level() <= W4_LOG_DEBUG)
                 log_line(W4_LOG_DEBUG, "w4_gemm_launch_experts m=%d n=%d k=%d bits=%d group=%d experts=%d tensor-core kernel (chosen)",
                     q.m, q.n, q.k, q.weight_bits, q.group_size, used);
-            int const rc = w4::launch_gemm_tc_experts(q, num_experts, expert_first_row, joins, static_cast<cudaStream_t>(stream));
+            int const rc = w4::launch_gemm_tc_experts(q, num_experts, expert_first_row, joins[j], exact[j], static_cast<cudaStream_t>(stream));
             if (rc != W4_OK)
                 return rc;
         }
         for (int e = 0; e < num_experts; ++e)
         {
             int const row0 = expert_first_row[e], rows = expert_first_row[e + 1] - row0;
-            if (rows == 0 || (shared && joins(*p, rows)))
+            if (rows == 0 || (joins[0] && joins[0](*p, rows)) || (joins[1] && joins[1](*p, rows)))
                 continue;
             q = *p;
             q.m = rows;
@@ -655,7 +707,7 @@ extern "C"
         W4GemmParams q = *p;
         if (out_dev)
             q.out = out_dev;
-        int const lrc = takes_decode_kernel(q) ? w4::launch_gemv(q, s) : w4::launch_gemm_tc(q, s);
+        int const lrc = takes_decode_kernel(q) ? w4::launch_gemv(q, s) : launch_tensor_cores(q, s);
         if (lrc != W4_OK)
             return lrc;
         if (!out_dev && cudaMemcpyAsync(host_out, p->out, out_bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)

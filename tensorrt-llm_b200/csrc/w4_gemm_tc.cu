@@ -2,10 +2,12 @@
 //
 // Replaces CutlassFpAIntBGemmRunner::gemm of the reference project
 // (cpp/tensorrt_llm/kernels/cutlass_kernels/fpA_intB_gemm/fpA_intB_gemm_template.h:394-465), which
-// on compute capability 10.x runs an Ampere mma.sync kernel. Same math as that kernel: every
+// on compute capability 10.x runs an Ampere mma.sync kernel. Same math as that kernel (SCALE_ROUND): every
 // weight is dequantised to T as round_T(fma(q, scale, zero))
 // (cpp/tensorrt_llm/cutlass_extensions/include/cutlass_extensions/gemm/warp/mma_tensorop_dequantizer.h:247-262),
-// products are accumulated in fp32, alpha and bias are applied in the epilogue.
+// products are accumulated in fp32, alpha and bias are applied in the epilogue. Two other forms multiply the
+// integers and apply scales and zeros to fp32 sums, as the decode kernels do, whose regime this kernel serves
+// too where it is the faster one (see ScaleMode).
 //
 // Orientation. The output tile is computed transposed: D[n, m] = sum_k W[n, k] * A[m, k]. The
 // dequantised weights are the MMA's "A" operand and live in tensor memory (one TMEM lane per
@@ -30,7 +32,8 @@
 //                         per step, a ring of its own that runs far ahead (its latency is
 //                         HBM's) and, with static weights, ahead of the preceding kernel
 //   next                  activation producer: two boxes of 64 k x BM/2 rows per step
-//   last                  MMA issuer (first CTA of the pair) and TMEM alloc/free (both)
+//   next                  MMA issuer (first CTA of the pair) and TMEM alloc/free (both)
+//   last                  scale / zero producer (SCALE_GROUP)
 // A step is 128 k (eight tcgen05.mma of K = 16). Hand-offs, all mbarriers: `w_full` / `w_empty` (weight
 // ring, local), `full` (first CTA: both CTAs' halves of the step's activations landed and the eight
 // conversion warps of both CTAs stored their part of the step's weights), `empty` (tcgen05.commit,
@@ -38,6 +41,9 @@
 // `d_empty` (accumulator).
 // All waits are bounded; a timeout sets the device status word and the CTAs drain and exit.
 #include <atomic>
+#include <chrono>
+#include <cstddef>
+#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -61,10 +67,21 @@ constexpr int kConvWarp0 = kEpiWarps;
 constexpr int kWProdWarp = kConvWarp0 + 4 * kConvGroups;
 constexpr int kActWarp = kWProdWarp + 1;
 constexpr int kMmaWarp = kWProdWarp + 2;
+constexpr int kScaleWarp = kWProdWarp + 3;
 constexpr int kThreads = 32 * (kWProdWarp + 4);
 constexpr int kMaxStages = 8;      // activation / TMEM ring
 constexpr int kMaxWStages = 12;    // weight ring
+constexpr int kScaleStages = 24;   // ring of scale and zero rows (SCALE_GROUP)
+constexpr int kScaleStage = 512;   // 128 scales, 128 zeros
+constexpr int kOnesCols = 32;      // (eight are used)
+constexpr int kMaxDBufs = 4;
+constexpr int kGroupBytes = kScaleStages * kScaleStage + 4 * 4096; // and the sums that warps pass on (SCALE_GROUP)
+constexpr int kGroupBM = 32;       // activation rows per tile of SCALE_GROUP
 constexpr int kMaxExperts = 32;    // experts of one launch
+// SPLIT_RANGES: up to this many rows, and rows of a tile. Beyond, the parts are larger and the time is the tensor cores'
+// under the power limit, which idle pairs help to stay under (777 rows on 14336 x 4096: 72.9 us, whole tiles 71.3).
+constexpr int kMaxRangesRows = 256, kMaxRangesBM = 128;
+constexpr size_t kSmemMost = 227 * 1024; // what the plan takes for a block's shared memory
 
 struct Args
 {
@@ -82,24 +99,51 @@ struct Args
     int groups; // scale rows per expert
     int first_row[kMaxExperts + 1], first_tile[kMaxExperts + 1], slice[kMaxExperts];
     int num_stages, num_wstages;
-    int d_bufs;      // accumulators in TMEM: 2 up to 128 rows, else 1
+    int d_bufs;      // accumulators in TMEM
+    int has_zero;
+    void const* scales; // SCALE_RAW
     int weights_static;
-    // Split-k: an output tile's k range is cut into `splits` work items that run on different CTA pairs.
-    int splits;       // 1 = off
-    int steps_split;  // 128-wide k steps per work item
-    float* partial;   // [splits, m, n] fp32 (SPLIT_WORKSPACE)
+    // SPLIT_CLUSTER: an output tile's k range is cut into `splits` work items of `steps_split` 128-wide k steps.
+    int splits, steps_split;
+    // SPLIT_RANGES: partial tiles in the workspace, [range][CTA of the pair][epilogue warp] blocks of bm x 32 fp32
+    // values, and a flag for each block, which holds `tag` from when the block is written until it is read.
+    float* partial;
+    unsigned long long* flags;
+    unsigned long long tag;
 };
 
-// Where the fp32 partial tiles of a split tile meet. CLUSTER: the splits' CTA pairs form one cluster of
-// 2 * splits CTAs, every CTA leaves its partial tile in its own shared memory and adds a share of the rows
-// over all of them through distributed shared memory. WORKSPACE: partial tiles in the caller's workspace,
-// added by a second kernel; for more splits than a cluster can hold, and where the device cannot
-// co-schedule such clusters. Both add in split order (deterministic).
+// Where scales and zeros are applied. ROUND: to the weights, round_T(fma(q, s, z)), as the reference's tensor-core kernel
+// does. RAW (one scale per column, no zeros): the integers are multiplied as they are, the scale is applied to the
+// fp32 sum by the epilogue. GROUP: likewise for every scale group; the sums of a group go to an accumulator of
+// their own, which the epilogue warps scale and add up in registers, rows of 32 at most. With zeros a second
+// accumulator holds the sums of the activations (a weight operand of ones). RAW and GROUP round nothing but the
+// output, as the decode kernels do: 1.66e-3 of the outputs' size for bf16 and 2.07e-4 for fp16 against 2.37e-3 and
+// 2.97e-4 (decode kernels 1.66e-3, 2.08e-4).
+// Few rows, microseconds, the decode kernels first: RAW int8 bf16 on 4096 x 14336 at one row 19.4 -> 13.4, at sixteen
+// 24.3 -> 13.7, on 28672 x 8192 72 -> 40 (5.9 TB/s; memory is what bounds it there), int4 at sixteen rows 18.5 -> 11.2;
+// GROUP int8 at sixteen rows 25 -> 18.3, int4 18.8 -> 16.5, on 8192 x 18944 41.8 -> 29.2. A step of GROUP takes
+// 0.33 to 0.38 us (0.49 with 64-wide groups) where RAW takes 0.2: neither more accumulators or stages, nor an
+// epilogue that does nothing but wait, nor three conversion groups change that; missing the instruction caches is
+// twice as frequent a stall as in RAW.
+enum ScaleMode
+{
+    SCALE_ROUND,
+    SCALE_RAW,
+    SCALE_GROUP
+};
+
+// How CTA pairs share the k range of a tile. CLUSTER: the splits' CTA pairs form one cluster of 2 * splits CTAs,
+// every CTA leaves its partial tile in its own shared memory and adds a share of the rows over all of them through
+// distributed shared memory. RANGES: the steps of all tiles, one tile behind the other, are cut into equal ranges,
+// one per pair, wherever the cuts fall. A pair that begins inside a tile leaves its part in the caller's workspace;
+// the pair that began the tile adds the parts to its own, in the order of k, and stores the tile. Both are
+// deterministic. RANGES cost about 3.5 us from a pair's last MMA to the stored tile: 64 rows on 8192 x 10240 (40 tiles
+// for 74 pairs) 20.2 -> 18.3 us, 256 rows 40.4 -> 35.0, few rows on 7168 x 20480 31 -> 24.
 enum SplitMode
 {
     SPLIT_NONE,
     SPLIT_CLUSTER,
-    SPLIT_WORKSPACE
+    SPLIT_RANGES
 };
 constexpr int kMaxClusterSplits = 8; // clusters of 16 CTAs
 
@@ -112,8 +156,11 @@ struct __align__(16) Barriers
     // (The `empty` phases come from commits, which complete in order.)
     uint64_t w_full[kConvGroups][kMaxWStages];
     uint64_t w_empty[kMaxWStages];
-    uint64_t d_full[2];           // accumulator complete
-    uint64_t d_empty[2];          // first CTA: the epilogue warps of both CTAs drained the accumulator
+    uint64_t d_full[kMaxDBufs];   // accumulator complete
+    uint64_t d_empty[kMaxDBufs];  // first CTA: the epilogue warps of both CTAs drained the accumulator
+    uint64_t s_full[kScaleStages], s_empty[kScaleStages]; // SCALE_GROUP
+    uint64_t pass_full[kEpiWarps], pass_empty[kEpiWarps]; // sums of the second group of epilogue warps (SCALE_GROUP)
+    uint64_t part[kEpiWarps];     // partial tiles of other pairs landed in shared memory (SPLIT_RANGES)
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -160,6 +207,33 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
         }
     }
     return true;
+}
+
+// Bounded wait, by a converged warp, for flags in global memory that other blocks set to `tag`, one per lane that
+// has one; what those blocks wrote before is then visible to the lane, and to TMA copies that it issues.
+__device__ __forceinline__ bool wait_flag(unsigned long long const* flag, unsigned long long tag, bool mine, volatile int* abort_flag)
+{
+    for (uint32_t polls = 1;; ++polls)
+    {
+        unsigned long long v = tag;
+        if (mine)
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(flag) : "memory");
+        if (__all_sync(0xffffffffu, v == tag))
+            break;
+        if ((polls & 1023u) == 0 && (*abort_flag || polls >= 2 * kMaxWaitPolls))
+        {
+            *abort_flag = 1;
+            atomicExch(&g_device_status, kDeviceTimeout);
+            return false;
+        }
+    }
+    asm volatile("fence.proxy.async;" ::: "memory");
+    return true;
+}
+
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Address of this CTA's shared variable in CTA `rank` of the cluster.
@@ -218,6 +292,24 @@ __device__ __forceinline__ void tc_mma4_ts_elect(uint32_t d_tmem, uint32_t a_tme
         : "memory");
 }
 
+// The same with one K = 16 block of weights for all four.
+__device__ __forceinline__ void tc_mma4_ones_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred p, pt, pe;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "setp.ne.b32 p, %7, 0;\n"
+        "setp.eq.b32 pt, 0, 0;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %6, p;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %3, %6, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %4, %6, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %5, %6, pt;\n"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "l"(b_desc + 2), "l"(b_desc + 4), "l"(b_desc + 6), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
 // Arrives on the barrier at this offset in both CTAs of the pair (`mask`: their ranks in the cluster) once
 // all MMAs issued so far have completed.
 __device__ __forceinline__ void tc_commit_pair_elect(uint32_t bar_addr, uint16_t mask)
@@ -229,6 +321,68 @@ __device__ __forceinline__ void tc_commit_pair_elect(uint32_t bar_addr, uint16_t
         "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
         "}\n" ::"r"(bar_addr),
         "h"(mask)
+        : "memory");
+}
+
+// A whole step into an accumulator of its own, with the commits that free the step's stages and hand the accumulator
+// over: the fewer elections and operands, the sooner the issuing warp is back at its waits (3 % of a step).
+__device__ __forceinline__ void tc_step_d_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint64_t b1, uint32_t idesc,
+    uint32_t acc, uint32_t empty_bar, uint16_t mask, uint32_t d_full_bar)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred p, pt, pe;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "setp.ne.b32 p, %18, 0;\n"
+        "setp.eq.b32 pt, 0, 0;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %9, %17, p;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%2], %10, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%3], %11, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%4], %12, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%5], %13, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%6], %14, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%7], %15, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%8], %16, %17, pt;\n"
+        "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%19], %20;\n"
+        "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%21], %20;\n"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(a_tmem + 8), "r"(a_tmem + 16), "r"(a_tmem + 24), "r"(a_tmem + 32), "r"(a_tmem + 40), "r"(a_tmem + 48),
+        "r"(a_tmem + 56), "l"(b0), "l"(b0 + 2), "l"(b0 + 4), "l"(b0 + 6), "l"(b1), "l"(b1 + 2), "l"(b1 + 4), "l"(b1 + 6), "r"(idesc),
+        "r"(acc), "r"(empty_bar), "h"(mask), "r"(d_full_bar), "r"(0u), "r"(0u)
+        : "memory");
+}
+
+__device__ __forceinline__ void tc_step_d_ones_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint64_t b1, uint32_t idesc,
+    uint32_t acc, uint32_t empty_bar, uint16_t mask, uint32_t d_full_bar, uint32_t d_sums, uint32_t ones)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred p, pt, pe;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "setp.ne.b32 p, %18, 0;\n"
+        "setp.eq.b32 pt, 0, 0;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %9, %17, p;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%2], %10, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%3], %11, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%4], %12, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%5], %13, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%6], %14, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%7], %15, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%8], %16, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %9, %17, p;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %10, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %11, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %12, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %13, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %14, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %15, %17, pt;\n"
+        "@pe tcgen05.mma.cta_group::2.kind::f16 [%22], [%23], %16, %17, pt;\n"
+        "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%19], %20;\n"
+        "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%21], %20;\n"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(a_tmem + 8), "r"(a_tmem + 16), "r"(a_tmem + 24), "r"(a_tmem + 32), "r"(a_tmem + 40), "r"(a_tmem + 48),
+        "r"(a_tmem + 56), "l"(b0), "l"(b0 + 2), "l"(b0 + 4), "l"(b0 + 6), "l"(b1), "l"(b1 + 2), "l"(b1 + 4), "l"(b1 + 6), "r"(idesc),
+        "r"(acc), "r"(empty_bar), "h"(mask), "r"(d_full_bar), "r"(d_sums), "r"(ones)
         : "memory");
 }
 
@@ -300,6 +454,42 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32])
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// Waits for this thread's loads from tensor memory; `v` (a load's result) is not used before.
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
+                 "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
+
+__device__ __forceinline__ uint64_t pack_u32x2(uint32_t lo, uint32_t hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi)
+{
+    return pack_u32x2(__float_as_uint(lo), __float_as_uint(hi));
+}
+
+// acc += x * y, two fp32 values at a time, each rounded once.
+__device__ __forceinline__ void fma_f32x2(uint64_t& acc, uint64_t x, uint64_t y)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
+}
+
 // Shared-memory matrix descriptor of a K-major, 128-byte-swizzled tile of T whose rows are 128
 // bytes (64 elements) wide: 8-row groups are 1024 bytes apart, descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr)
@@ -312,7 +502,8 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr)
 }
 
 
-template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
+// HAS_ZERO matters to SCALE_GROUP only: a zero of 0 costs SCALE_ROUND nothing.
+template <typename T, int BITS, int MODE, bool HAS_ZERO, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
     gemm_kernel(Args const a, __grid_constant__ CUtensorMap const tm_act, __grid_constant__ CUtensorMap const tm_w,
         __grid_constant__ CUtensorMap const tm_s, __grid_constant__ CUtensorMap const tm_z)
@@ -320,6 +511,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     using P = Pair<T>;
     constexpr int IL = BITS == 4 ? 4 : 2;
     constexpr int SEG_CHUNKS = 8 / IL;               // 16-byte chunks of one column inside a 128-byte line (64 k)
+    constexpr int CONV_GROUPS = MODE == SCALE_GROUP ? 2 : kConvGroups; // (integers as they are need fewer instructions)
+    constexpr int EPI_GROUPS = MODE == SCALE_GROUP ? 2 : 1;
     constexpr int LINE_TILE = (BN / IL) * 128;       // this CTA's interleaved rows x one line
     constexpr int W_BYTES = 2 * LINE_TILE;           // a step: two lines per row
     constexpr int W_STAGE = W_BYTES + 1024;          // + up to two rows of 128 scales, and of zeros
@@ -332,42 +525,70 @@ __global__ void __launch_bounds__(kThreads, 1)
     int const act_half = a.bm * 64;       // bm / 2 rows of 128 bytes: 64 k
     int const act_stage = 2 * act_half;
     uint32_t const w_ring = smem_base + uint32_t(a.num_stages) * act_stage;
-    Barriers* bars = reinterpret_cast<Barriers*>(smem + size_t(a.num_stages) * act_stage + size_t(a.num_wstages) * W_STAGE);
+    uint32_t const s_ring = w_ring + uint32_t(a.num_wstages) * W_STAGE;
+    Barriers* bars = reinterpret_cast<Barriers*>(
+        smem + (s_ring - smem_base) + (MODE == SCALE_GROUP ? kGroupBytes : 0));
     volatile int* abort_flag = &bars->abort_flag;
 
     int const warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     uint32_t cta_rank;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
     uint32_t const rank = cta_rank & 1u, lead_rank = cta_rank & ~1u; // in the pair; the pair's first CTA
-    // Work items: (tile, split), splits adjacent. With SPLIT_CLUSTER a pair has exactly one: the grid is one
-    // cluster per tile and a pair's rank in it is its split.
+    // A pair's work: tiles tile_first, tile_first + tile_step .. tile_last, of the first from step st_first, of the last
+    // to st_end, of the others all steps. SPLIT_CLUSTER: one tile; the grid is one cluster per tile and a pair's rank
+    // in it is its split. SPLIT_RANGES: a pair waits for parts of the ranges behind its own, so the ranges go to the
+    // pairs in reverse: a block only ever waits for blocks in front of it in the grid, which are running or done.
+    // (The shuffles tell the compiler that these are the same for the whole warp: loops over them would otherwise
+    // issue every tensor-core instruction and copy with operands out of vector registers, 0.36 us a step.)
     int const pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    int const num_items = a.first_tile[a.num_experts] * (SPLIT != SPLIT_NONE ? a.splits : 1);
     int const steps_all = (a.k + 127) >> 7; // the second half of the last step may lie past k: zeros, not multiplied
+    int const num_tiles = a.first_tile[a.num_experts];
+    auto uniform = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };
+    auto range_begin = [&](int range) { return int((int64_t(num_tiles) * steps_all * range) / num_pairs); };
+    int const range = num_pairs - 1 - pair;
+    int tile_first = pair, tile_last = num_tiles - 1, tile_step = num_pairs, st_first = 0, st_end = steps_all, split = 0;
+    if (SPLIT == SPLIT_CLUSTER)
+    {
+        tile_first = tile_last = uniform(pair / a.splits);
+        split = pair - tile_first * a.splits;
+        st_first = split * a.steps_split;
+        st_end = min(steps_all, st_first + a.steps_split);
+    }
+    if (SPLIT == SPLIT_RANGES)
+    {
+        int const begin = range_begin(range), end = range_begin(range + 1);
+        tile_first = uniform(begin / steps_all);
+        st_first = uniform(begin - tile_first * steps_all);
+        tile_last = uniform((end - 1) / steps_all);
+        st_end = uniform(end - tile_last * steps_all);
+        tile_step = 1;
+    }
+    auto first_step = [&](int tile) { return SPLIT != SPLIT_NONE && tile == tile_first ? st_first : 0; };
+    auto end_step = [&](int tile) { return SPLIT != SPLIT_NONE && tile == tile_last ? st_end : steps_all; };
 
     bool const aligned = (smem_base & 1023u) == 0; // never false; the check keeps a wrong layout from being read
+    if (warp == 0)
+    {
+        // Arrivals that complete a phase; a lane each, one after another they would take half a microsecond.
+        constexpr int kBars = int(offsetof(Barriers, tmem_base) / 8);
+        constexpr int kEmpty = offsetof(Barriers, empty) / 8, kWEmpty = offsetof(Barriers, w_empty) / 8,
+                      kDFull = offsetof(Barriers, d_full) / 8, kDEmpty = offsetof(Barriers, d_empty) / 8,
+                      kSFull = offsetof(Barriers, s_full) / 8, kSEmpty = offsetof(Barriers, s_empty) / 8,
+                      kPass = offsetof(Barriers, pass_full) / 8;
+        for (int i = lane; i < kBars; i += 32)
+            mbar_init(&bars->full[0] + i,
+                i < kEmpty                          ? 1 + 8 // expect_tx of the first CTA + four conversion warps of each CTA
+                    : i >= kWEmpty && i < kDFull    ? 4 // conversion warps
+                    : i >= kDEmpty && i < kSFull    ? 2 * kEpiWarps // of both CTAs
+                    : i >= kSEmpty && i < kPass     ? kEpiWarps
+                                                    : 1);
+        mbar_fence_init();
+    }
     if (threadIdx.x == 0)
     {
-        for (int s = 0; s < a.num_stages; ++s)
-        {
-            mbar_init(&bars->full[s], 1 + 8); // expect_tx of the first CTA + four conversion warps of each CTA
-            mbar_init(&bars->empty[s], 1);
-        }
-        for (int s = 0; s < a.num_wstages; ++s)
-        {
-            for (int g = 0; g < kConvGroups; ++g)
-                mbar_init(&bars->w_full[g][s], 1);
-            mbar_init(&bars->w_empty[s], 4);
-        }
-        for (int b = 0; b < 2; ++b)
-        {
-            mbar_init(&bars->d_full[b], 1);
-            mbar_init(&bars->d_empty[b], 2 * kEpiWarps);
-        }
         bars->abort_flag = aligned ? 0 : 1;
         if (!aligned)
             atomicExch(&g_device_status, kDeviceTimeout);
-        mbar_fence_init();
     }
     if (warp == kMmaWarp)
     {
@@ -383,25 +604,23 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t const tmem = bars->tmem_base;
-    uint32_t const a_ring = tmem + uint32_t(a.d_bufs * a.bm); // TMEM ring of converted weights, behind the accumulators
+    // TMEM: accumulators (with zeros of groups, each with one for the sums of activations), ones, converted weights
+    uint32_t const d_cols = MODE == SCALE_GROUP && HAS_ZERO ? 2 * kGroupBM : uint32_t(a.bm);
+    uint32_t const ones = tmem + uint32_t(a.d_bufs) * d_cols;
+    uint32_t const a_ring = ones + (MODE == SCALE_GROUP && HAS_ZERO ? kOnesCols : 0);
 
     uint32_t const full0 = smem_u32(&bars->full[0]), empty0 = smem_u32(&bars->empty[0]);
     uint32_t const w_full0 = smem_u32(&bars->w_full[0][0]), w_empty0 = smem_u32(&bars->w_empty[0]);
 
-    struct Item
+    struct Place
     {
         int n0;             // first column of the pair's tile
         int row0, row_end;  // rows of the tile, and the end of the expert's
-        int slice, split;
-        int st0, st1;       // k steps
+        int slice;
     };
-    auto item_of = [&](int item)
+    auto place_of = [&](int tile)
     {
-        Item it;
-        int const tile = SPLIT != SPLIT_NONE ? item / a.splits : item;
-        it.split = SPLIT != SPLIT_NONE ? item - tile * a.splits : 0;
-        it.st0 = it.split * a.steps_split;
-        it.st1 = SPLIT != SPLIT_NONE ? min(steps_all, it.st0 + a.steps_split) : steps_all;
+        Place it;
         int e = 0;
         while (e + 1 < a.num_experts && tile >= a.first_tile[e + 1])
             ++e;
@@ -423,37 +642,75 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0)
         {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_w) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_s) : "memory");
-            if (HAS_ZERO)
+            if (MODE != SCALE_RAW)
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_s) : "memory");
+            if (MODE != SCALE_RAW && a.has_zero)
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_z) : "memory");
         }
         __syncwarp();
         // Weights that the preceding kernel may still be writing must not be fetched early.
         if (!a.weights_static)
             asm volatile("griddepcontrol.wait;" ::: "memory");
-        uint32_t const scale_bytes = a.group_shift == 6 ? 512u : 256u;
-        uint32_t const tx = W_BYTES + scale_bytes * (HAS_ZERO ? 2 : 1);
+        uint32_t const scales_tx = (a.group_shift == 6 ? 512u : 256u) * (a.has_zero ? 2 : 1);
+        uint32_t const tx = W_BYTES + (MODE == SCALE_ROUND ? scales_tx : 0);
         int s = 0, turn = 0; // turn: the group that converts the step
         uint32_t ph = 0;
         bool ok = true;
-        for (int item = pair; item < num_items && ok; item += num_pairs)
+        for (int tile = tile_first; tile <= tile_last && ok; tile += tile_step)
         {
-            Item const it = item_of(item);
+            Place const it = place_of(tile);
             int const n0 = it.n0 + int(rank) * BN, w_row = it.slice * (a.n / IL) + n0 / IL, s_row = it.slice * a.groups;
-            for (int st = it.st0; st < it.st1; ++st)
+            for (int st = first_step(tile), st1 = end_step(tile); st < st1; ++st)
             {
                 ok = wait_bar<false>(w_empty0 + 8 * s, ph ^ 1, abort_flag);
                 if (!ok)
                     break;
                 uint32_t const dst = w_ring + uint32_t(s) * W_STAGE, bar = w_full0 + 8 * (turn * kMaxWStages + s);
-                int const g = s_row + (a.group_shift >= 31 ? 0 : (st << 7) >> a.group_shift);
                 elect_expect_tx(bar, tx);
                 elect_tma_load_3d(dst, &tm_w, 0, w_row, 2 * st, bar);
-                elect_tma_load_2d(dst + W_BYTES, &tm_s, n0, g, bar);
-                if (HAS_ZERO)
-                    elect_tma_load_2d(dst + W_BYTES + 512, &tm_z, n0, g, bar);
-                turn = turn + 1 == kConvGroups ? 0 : turn + 1;
+                if (MODE == SCALE_ROUND)
+                {
+                    int const g = s_row + (a.group_shift >= 31 ? 0 : (st << 7) >> a.group_shift);
+                    elect_tma_load_2d(dst + W_BYTES, &tm_s, n0, g, bar);
+                    if (a.has_zero)
+                        elect_tma_load_2d(dst + W_BYTES + 512, &tm_z, n0, g, bar);
+                }
+                turn = turn + 1 == CONV_GROUPS ? 0 : turn + 1;
                 if (++s == a.num_wstages)
+                {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+    }
+    else if (MODE == SCALE_GROUP && warp == kScaleWarp)
+    {
+        // ------------------------------------------------------------------ scale and zero producer
+        if (!a.weights_static)
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t const s_full0 = smem_u32(&bars->s_full[0]), s_empty0 = smem_u32(&bars->s_empty[0]);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int tile = tile_first; tile <= tile_last && ok; tile += tile_step)
+        {
+            Place const it = place_of(tile);
+            int const n0 = it.n0 + int(rank) * BN, s_row = it.slice * a.groups;
+            int const per_step = a.group_shift == 6 ? 2 : 1;
+            int const u1 = a.group_shift == 6 ? min(2 * end_step(tile), (a.k + 63) >> 6) : end_step(tile);
+            for (int u = first_step(tile) * per_step; u < u1; ++u)
+            {
+                ok = wait_bar<false>(s_empty0 + 8 * s, ph ^ 1, abort_flag);
+                if (!ok)
+                    break;
+                uint32_t const dst = s_ring + uint32_t(s) * kScaleStage, bar = s_full0 + 8 * s;
+                int const g = s_row + (a.group_shift >= 31 ? 0 : u);
+                elect_expect_tx(bar, HAS_ZERO ? 512u : 256u);
+                elect_tma_load_2d(dst, &tm_s, n0, g, bar);
+                if (HAS_ZERO)
+                    elect_tma_load_2d(dst + 256, &tm_z, n0, g, bar);
+                if (++s == kScaleStages)
                 {
                     s = 0;
                     ph ^= 1;
@@ -472,11 +729,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         int s = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int item = pair; item < num_items && ok; item += num_pairs)
+        for (int tile = tile_first; tile <= tile_last && ok; tile += tile_step)
         {
-            Item const it = item_of(item);
+            Place const it = place_of(tile);
             int const row0 = it.row0 + int(rank) * (a.bm >> 1);
-            for (int st = it.st0; st < it.st1; ++st)
+            for (int st = first_step(tile), st1 = end_step(tile); st < st1; ++st)
             {
                 ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
                 if (!ok)
@@ -520,32 +777,79 @@ __global__ void __launch_bounds__(kThreads, 1)
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            uint32_t dph = 0; // bit b: parity of accumulator b's next drain
-            int db = 0, done = 0;
-            for (int item = pair; item < num_items && ok; item += num_pairs, ++done)
+            uint32_t dph = 0;
+            int db = 0;
+            for (int tile = tile_first; tile <= tile_last && ok; tile += tile_step)
             {
-                Item const it = item_of(item);
-                if (done >= a.d_bufs)
+                if (MODE != SCALE_GROUP)
                 {
-                    ok = wait_bar<true>(d_empty0 + 8 * db, (dph >> db) & 1u, abort_flag);
+                    ok = wait_bar<true>(d_empty0 + 8 * db, dph ^ 1, abort_flag);
                     if (!ok)
                         break;
-                    dph ^= 1u << db;
-                    tc_fence_after();
                 }
-                uint32_t const d_tmem = tmem + uint32_t(db * a.bm);
                 uint32_t accumulate = 0;
-                for (int st = it.st0; st < it.st1; ++st)
+                for (int st = first_step(tile), st1 = end_step(tile); st < st1; ++st)
                 {
                     ok = wait_bar<true>(full0 + 8 * s, ph, abort_flag);
                     if (!ok)
                         break;
-                    tc_fence_after();
                     uint64_t const desc = desc0 + uint64_t(s) * desc_stage;
                     uint32_t const a_col = a_ring + uint32_t(s) * kStageCols;
-                    tc_mma4_ts_elect(d_tmem, a_col, desc, idesc, accumulate);
-                    if (st * 128 + 64 < a.k)
-                        tc_mma4_ts_elect(d_tmem, a_col + 32, desc + desc_half, idesc, 1u);
+                    bool const second = st * 128 + 64 < a.k;
+                    if (MODE == SCALE_GROUP)
+                    {
+                        ok = wait_bar<true>(d_empty0 + 8 * db, dph ^ 1, abort_flag);
+                        if (!ok)
+                            break;
+                        accumulate = 0;
+                    }
+                    tc_fence_after();
+                    uint32_t d = tmem + uint32_t(db) * d_cols;
+                    if (MODE == SCALE_GROUP && second && a.group_shift != 6)
+                    {
+                        if (HAS_ZERO)
+                            tc_step_d_ones_elect(d, a_col, desc, desc + desc_half, idesc, 0u, empty0 + 8 * s, both,
+                                d_full0 + 8 * db, d + kGroupBM, ones);
+                        else
+                            tc_step_d_elect(d, a_col, desc, desc + desc_half, idesc, 0u, empty0 + 8 * s, both, d_full0 + 8 * db);
+                        if (++s == a.num_stages)
+                        {
+                            s = 0;
+                            ph ^= 1;
+                        }
+                        if (++db == a.d_bufs)
+                        {
+                            db = 0;
+                            dph ^= 1;
+                        }
+                        continue;
+                    }
+                    tc_mma4_ts_elect(d, a_col, desc, idesc, accumulate);
+                    if (MODE == SCALE_GROUP && HAS_ZERO)
+                        tc_mma4_ones_elect(d + kGroupBM, ones, desc, idesc, 0u);
+                    if (second)
+                    {
+                        accumulate = 1u;
+                        if (MODE == SCALE_GROUP && a.group_shift == 6)
+                        {
+                            // two groups in the step: the second has an accumulator of its own
+                            tc_commit_pair_elect(d_full0 + 8 * db, both);
+                            if (++db == a.d_bufs)
+                            {
+                                db = 0;
+                                dph ^= 1;
+                            }
+                            ok = wait_bar<true>(d_empty0 + 8 * db, dph ^ 1, abort_flag);
+                            if (!ok)
+                                break;
+                            tc_fence_after();
+                            d = tmem + uint32_t(db) * d_cols;
+                            accumulate = 0;
+                        }
+                        tc_mma4_ts_elect(d, a_col + 32, desc + desc_half, idesc, accumulate);
+                        if (MODE == SCALE_GROUP && HAS_ZERO)
+                            tc_mma4_ones_elect(d + kGroupBM, ones, desc + desc_half, idesc, accumulate);
+                    }
                     accumulate = 1u;
                     tc_commit_pair_elect(empty0 + 8 * s, both); // frees the activation stage and the TMEM stage
                     if (++s == a.num_stages)
@@ -553,20 +857,40 @@ __global__ void __launch_bounds__(kThreads, 1)
                         s = 0;
                         ph ^= 1;
                     }
+                    if (MODE == SCALE_GROUP)
+                    {
+                        tc_commit_pair_elect(d_full0 + 8 * db, both);
+                        if (++db == a.d_bufs)
+                        {
+                            db = 0;
+                            dph ^= 1;
+                        }
+                    }
                 }
-                if (ok)
-                    tc_commit_pair_elect(d_full0 + 8 * db, both);
-                db = db + 1 == a.d_bufs ? 0 : db + 1;
+                if (MODE != SCALE_GROUP)
+                {
+                    if (ok)
+                        tc_commit_pair_elect(d_full0 + 8 * db, both);
+                    if (++db == a.d_bufs)
+                    {
+                        db = 0;
+                        dph ^= 1;
+                    }
+                }
             }
             // stay until the other CTA's last arrivals have landed
-            for (int i = 0; i < a.d_bufs && i < done && ok; ++i)
+            for (int i = 0; i < a.d_bufs && ok; ++i)
             {
-                db = db == 0 ? a.d_bufs - 1 : db - 1;
-                ok = wait_bar<true>(d_empty0 + 8 * db, (dph >> db) & 1u, abort_flag);
+                ok = wait_bar<true>(d_empty0 + 8 * db, dph ^ 1, abort_flag);
+                if (++db == a.d_bufs)
+                {
+                    db = 0;
+                    dph ^= 1;
+                }
             }
         }
     }
-    else if (warp >= kConvWarp0 && warp < kWProdWarp)
+    else if (warp >= kConvWarp0 && warp < kConvWarp0 + 4 * CONV_GROUPS)
     {
         // ------------------------------------------------------------------ conversion
         int const quad = warp & 3;                     // TMEM lane quadrant this warp may touch
@@ -579,130 +903,282 @@ __global__ void __launch_bounds__(kThreads, 1)
         int const w_row = n_local / IL;
         uint32_t const w_off = uint32_t(w_row * 128 + ((((n_local % IL) * SEG_CHUNKS) ^ (w_row & 7)) << 4));
 
-        // Own steps are every kConvGroups-th, counted over all items; the rings run on from item to item.
+        // Which tile a step belongs to does not matter here: the pair's steps are counted through, own ones are every
+        // CONV_GROUPS-th.
+        int const tiles = (tile_last - tile_first + tile_step) / tile_step;
+        int const steps = SPLIT == SPLIT_NONE ? tiles * steps_all : (tiles - 1) * steps_all + st_end - st_first;
         int s = cgroup, ws = cgroup;
         uint32_t ph = 0;
         uint32_t w_seen = 0; // bit ws: parity of this group's next phase on w_full[cgroup][ws]
-        int skip = cgroup;   // steps from the start of the item to the next own step
         bool ok = true;
-        for (int item = pair; item < num_items && ok; item += num_pairs)
+        if (MODE == SCALE_GROUP && HAS_ZERO && cgroup == 0)
         {
-            Item const it = item_of(item);
-            int st = it.st0 + skip;
-            for (; st < it.st1; st += kConvGroups)
+            // the operand of ones; ordered in front of the MMAs by the arrival behind the group's first step
+            uint32_t const one2 = kFmt ? 0x3f803f80u : 0x3c003c00u;
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(ones + (uint32_t(quad * 32) << 16)),
+                         "r"(one2)
+                         : "memory");
+        }
+        for (int st = cgroup; st < steps; st += CONV_GROUPS)
+        {
+            ok = wait_bar<false>(w_full0 + 8 * (cgroup * kMaxWStages + ws), (w_seen >> ws) & 1u, abort_flag);
+            if (!ok)
+                break;
+            w_seen ^= 1u << ws;
+            uint8_t const* wst = smem + (w_ring - smem_base) + size_t(ws) * W_STAGE;
+            uint16_t const* sc = reinterpret_cast<uint16_t const*>(wst + W_BYTES) + n_local;
+            uint4 raw[SEG_CHUNKS];
+            uint32_t s_now = 0, z_now = 0, s_next = 0, z_next = 0;
+            if (MODE == SCALE_ROUND)
             {
-                ok = wait_bar<false>(w_full0 + 8 * (cgroup * kMaxWStages + ws), (w_seen >> ws) & 1u, abort_flag);
-                if (!ok)
-                    break;
-                w_seen ^= 1u << ws;
-                uint8_t const* wst = smem + (w_ring - smem_base) + size_t(ws) * W_STAGE;
-                uint16_t const* sc = reinterpret_cast<uint16_t const*>(wst + W_BYTES) + n_local;
-                uint4 raw[2][SEG_CHUNKS];
-                uint32_t s2[2], z2[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                {
-                    int const grow = h && a.group_shift == 6 ? 128 : 0;
-                    s2[h] = sc[grow];
-                    s2[h] = prmt(s2[h], s2[h], 0x1010u);
-                    if (HAS_ZERO)
-                    {
-                        z2[h] = sc[grow + 256];
-                        z2[h] = prmt(z2[h], z2[h], 0x1010u);
-                    }
-#pragma unroll
-                    for (int c = 0; c < SEG_CHUNKS; ++c)
-                        raw[h][c] = *reinterpret_cast<uint4 const*>(wst + h * LINE_TILE + (w_off ^ uint32_t(c << 4)));
-                }
-                __syncwarp();
-                if (lane == 0)
-                    arrive_local(w_empty0 + 8 * ws);
-                uint32_t const a_col = lane_ring + uint32_t(s) * kStageCols;
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                {
-                    uint32_t v[32]; // TMEM columns of the half step: k = 2 * column (+1)
-#pragma unroll
-                    for (int c = 0; c < SEG_CHUNKS; ++c)
-                    {
-                        uint32_t const r[4] = {raw[h][c].x, raw[h][c].y, raw[h][c].z, raw[h][c].w};
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                        {
-                            // pair p of register j holds k = 32c + 2j + 8p (+1) (int4), 16c + 2j + 8p (+1) (int8)
-                            constexpr int PAIRS = BITS == 4 ? 4 : 2;
-                            uint32_t q[PAIRS];
-                            if constexpr (BITS == 4)
-                                cvt_int4x8<T>(r[j], q);
-                            else
-                                cvt_int8x4<T>(r[j], q);
-#pragma unroll
-                            for (int p = 0; p < PAIRS; ++p)
-                                v[4 * PAIRS * c + j + 4 * p] = HAS_ZERO ? P::fma(q[p], s2[h], z2[h]) : P::mul(q[p], s2[h]);
-                        }
-                    }
-                    if (h == 0)
-                    {
-                        ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
-                        if (!ok)
-                            break;
-                        tc_fence_after();
-                    }
-                    tc_st32(a_col + 32 * h, v);
-                }
-                if (!ok)
-                    break;
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    arrive_cluster_relaxed(lead_full0 + 8 * s);
-                ws += kConvGroups;
-                ws -= ws >= a.num_wstages ? a.num_wstages : 0;
-                s += kConvGroups;
-                if (s >= a.num_stages)
-                {
-                    s -= a.num_stages;
-                    ph ^= 1;
-                }
+                int const grow = a.group_shift == 6 ? 128 : 0;
+                s_now = sc[0];
+                s_next = sc[grow];
+                z_now = a.has_zero ? sc[256] : 0;
+                z_next = a.has_zero ? sc[grow + 256] : 0;
             }
-            skip = st - it.st1;
+#pragma unroll
+            for (int c = 0; c < SEG_CHUNKS; ++c)
+                raw[c] = *reinterpret_cast<uint4 const*>(wst + (w_off ^ uint32_t(c << 4)));
+            uint32_t const a_col = lane_ring + uint32_t(s) * kStageCols;
+            // With SCALE_GROUP the halves of a step share their instructions: the roles' loops together do not fit the
+            // instruction caches otherwise (2 % of a step; in the other modes 1 to 2 % the other way).
+            constexpr int UNROLL = MODE == SCALE_GROUP ? 1 : 2;
+#pragma unroll UNROLL
+            for (int h = 0; h < 2; ++h)
+            {
+                uint32_t const s2 = prmt(s_now, s_now, 0x1010u), z2 = prmt(z_now, z_now, 0x1010u);
+                uint32_t v[32]; // TMEM columns of the half step: k = 2 * column (+1)
+#pragma unroll
+                for (int c = 0; c < SEG_CHUNKS; ++c)
+                {
+                    uint32_t const r[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                    {
+                        // pair p of register j holds k = 32c + 2j + 8p (+1) (int4), 16c + 2j + 8p (+1) (int8)
+                        constexpr int PAIRS = BITS == 4 ? 4 : 2;
+                        uint32_t q[PAIRS];
+                        if constexpr (BITS == 4)
+                            cvt_int4x8<T>(r[j], q);
+                        else
+                            cvt_int8x4<T>(r[j], q);
+#pragma unroll
+                        for (int p = 0; p < PAIRS; ++p)
+                            v[4 * PAIRS * c + j + 4 * p] = MODE == SCALE_ROUND ? P::fma(q[p], s2, z2) : q[p];
+                    }
+                }
+                if (h == 0)
+                {
+                    // the second half's weights, on their way while the first half's are stored
+#pragma unroll
+                    for (int c = 0; c < SEG_CHUNKS; ++c)
+                        raw[c] = *reinterpret_cast<uint4 const*>(wst + LINE_TILE + (w_off ^ uint32_t(c << 4)));
+                    s_now = s_next;
+                    z_now = z_next;
+                    __syncwarp();
+                    if (lane == 0)
+                        arrive_local(w_empty0 + 8 * ws);
+                    ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
+                    if (!ok)
+                        break;
+                    tc_fence_after();
+                }
+                tc_st32(a_col + 32 * h, v);
+            }
+            if (!ok)
+                break;
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                arrive_cluster_relaxed(lead_full0 + 8 * s);
+            ws += CONV_GROUPS;
+            ws -= ws >= a.num_wstages ? a.num_wstages : 0;
+            s += CONV_GROUPS;
+            if (s >= a.num_stages)
+            {
+                s -= a.num_stages;
+                ph ^= 1;
+            }
         }
     }
-    else if (warp < kEpiWarps)
+    else if (warp < kEpiWarps || (EPI_GROUPS > 1 && warp < kWProdWarp)) // (between conversion and producers: the second group)
     {
         // ------------------------------------------------------------------ epilogue
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        uint32_t const lane_addr = tmem + (uint32_t(warp * 32) << 16);
+        int const quad = warp & 3, epi_group = EPI_GROUPS > 1 && warp >= kEpiWarps ? 1 : 0;
+        uint32_t const lane_addr = tmem + (uint32_t(quad * 32) << 16);
         uint16_t const* bias = static_cast<uint16_t const*>(a.bias);
         uint32_t const d_full0 = smem_u32(&bars->d_full[0]), lead_d_empty0 = cluster_addr(smem_u32(&bars->d_empty[0]), lead_rank);
-        uint32_t dph = 0;
-        int db = 0;
+        uint32_t const s_full0 = smem_u32(&bars->s_full[0]), s_empty0 = smem_u32(&bars->s_empty[0]);
+        uint32_t dph = 0, sph = 0;
+        int db = epi_group, ss = epi_group;
+        uint32_t pass_ph = 0;
+        int own = epi_group; // groups of k from the start of the tile to the first that is this warp's turn
         bool ok = true;
-        for (int item = pair; item < num_items && ok; item += num_pairs)
+        // SCALE_GROUP: scale and zero of this lane's column in the next group
+        auto next_scales = [&](uint64_t& s2, uint64_t& z2)
         {
-            Item const it = item_of(item);
-            int const n = it.n0 + int(rank) * BN + warp * 32 + lane;
+            if (!wait_bar<false>(s_full0 + 8 * ss, sph, abort_flag))
+                return false;
+            uint16_t const* sc = reinterpret_cast<uint16_t const*>(smem + (s_ring - smem_base) + ss * kScaleStage) + quad * 32 + lane;
+            float const sf = P::to_float(sc[0]), zf = HAS_ZERO ? P::to_float(sc[128]) : 0.f;
+            s2 = pack_f32x2(sf, sf);
+            z2 = pack_f32x2(zf, zf);
+            __syncwarp();
+            if (lane == 0)
+                arrive_local(s_empty0 + 8 * ss);
+            ss += EPI_GROUPS;
+            if (ss >= kScaleStages)
+            {
+                ss -= kScaleStages;
+                sph ^= 1;
+            }
+            return true;
+        };
+        for (int tile = tile_first; tile <= tile_last && ok; tile += tile_step)
+        {
+            Place const it = place_of(tile);
+            int const n = it.n0 + int(rank) * BN + quad * 32 + lane;
             bool const n_ok = n < a.n; // n is a multiple of 32: uniform over the warp
             int const m0 = it.row0;
-            float const bias_f = (SPLIT == SPLIT_NONE && bias && n_ok) ? P::to_float(bias[size_t(it.slice) * a.n + n]) : 0.f;
-            ok = wait_bar<false>(d_full0 + 8 * db, (dph >> db) & 1u, abort_flag);
+            float const bias_f = (SPLIT != SPLIT_CLUSTER && bias && n_ok) ? P::to_float(bias[size_t(it.slice) * a.n + n]) : 0.f;
+            float factor = a.alpha;
+            if (MODE == SCALE_RAW && SPLIT != SPLIT_CLUSTER && n_ok)
+                factor *= P::to_float(static_cast<uint16_t const*>(a.scales)[size_t(it.slice) * a.n + n]);
+            int const c_end = min(a.bm, it.row_end - m0);
+            uint32_t v[32];
+            if (MODE == SCALE_GROUP)
+            {
+                // The sums of every group as its MMAs complete. One warp per tensor-memory quadrant has to keep up with
+                // the conversion, next to whose instructions its own wait for issue slots: the next group's scales are
+                // read while a load from tensor memory is under way, and the sums are taken in pairs (fma.f32x2).
+                uint64_t acc[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    acc[j] = 0;
+                int const st0 = first_step(tile), st1 = end_step(tile);
+                int const units = a.group_shift == 6 ? min(2 * st1, (a.k + 63) >> 6) - 2 * st0 : st1 - st0;
+                uint64_t s2 = 0, z2 = 0;
+                if (own < units)
+                    ok = next_scales(s2, z2);
+                for (; own < units && ok; own += EPI_GROUPS)
+                {
+                    ok = wait_bar<false>(d_full0 + 8 * db, dph, abort_flag);
+                    if (!ok)
+                        break;
+                    tc_fence_after();
+                    uint32_t const d = lane_addr + uint32_t(db) * d_cols;
+                    uint64_t const s2_now = s2, z2_now = z2;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (16 * h < c_end)
+                        {
+                            uint32_t x[16], y[16];
+                            tc_ld16(d + 16 * h, x);
+                            if (HAS_ZERO)
+                                tc_ld16(d + kGroupBM + 16 * h, y);
+                            if (h == 0 && own + EPI_GROUPS < units)
+                                ok = next_scales(s2, z2);
+                            tc_wait_ld(x);
+                            if (HAS_ZERO)
+                                tc_wait_ld(y);
+                            if (16 * h + 16 >= c_end)
+                            {
+                                // everything is in registers: the accumulator may be overwritten
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0)
+                                    arrive_cluster_relaxed(lead_d_empty0 + 8 * db);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                            {
+                                fma_f32x2(acc[8 * h + j], pack_u32x2(x[2 * j], x[2 * j + 1]), s2_now);
+                                if (HAS_ZERO)
+                                    fma_f32x2(acc[8 * h + j], pack_u32x2(y[2 * j], y[2 * j + 1]), z2_now);
+                            }
+                        }
+                    db += EPI_GROUPS;
+                    if (db >= a.d_bufs)
+                    {
+                        db -= a.d_bufs;
+                        dph ^= 1;
+                    }
+                }
+                own -= units;
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(acc[j]));
+                // The second group's sums go to the first.
+                float* const pass = reinterpret_cast<float*>(smem + (s_ring - smem_base) + kScaleStages * kScaleStage) + quad * 1024 + lane;
+                if (ok && epi_group == 1)
+                    ok = wait_bar<false>(smem_u32(&bars->pass_empty[quad]), pass_ph ^ 1u, abort_flag);
+                if (ok && EPI_GROUPS > 1 && epi_group == 0)
+                    ok = wait_bar<false>(smem_u32(&bars->pass_full[quad]), pass_ph, abort_flag);
+                if (!ok)
+                    break;
+                pass_ph ^= 1u;
+                if (epi_group == 1)
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        pass[32 * j] = __uint_as_float(v[j]);
+                else if (EPI_GROUPS > 1)
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        v[j] = __float_as_uint(__uint_as_float(v[j]) + pass[32 * j]);
+                __syncwarp();
+                if (lane == 0)
+                    arrive_local(smem_u32(epi_group == 1 ? &bars->pass_full[quad] : &bars->pass_empty[quad]));
+                if (epi_group == 1)
+                    continue;
+            }
+            else
+            {
+                ok = wait_bar<false>(d_full0 + 8 * db, dph, abort_flag);
+                tc_fence_after();
+            }
             if (!ok)
                 break;
-            dph ^= 1u << db;
-            tc_fence_after();
-            float* part = SPLIT == SPLIT_WORKSPACE ? a.partial + size_t(it.split) * a.m * a.n + n : nullptr;
             // two rows at a time: neighbouring lanes exchange halves, so that the even lane stores columns
             // n, n + 1 of the first row and the odd lane columns n - 1, n of the second
             uint16_t* out = static_cast<uint16_t*>(a.out) + (n & ~1);
             uint32_t const sel = lane & 1 ? 0x3276u : 0x5410u;
-            int const c_end = min(a.bm, it.row_end - m0);
+            // SPLIT_RANGES: the ranges behind this one that have a part of the tile (this item is then the pair's last)
+            int parts = 0;
+            uint32_t const part_block = uint32_t(a.bm) * 128u; // bytes of an epilogue warp's part: [row / 4][lane][4]
+            uint32_t const part_bytes = uint32_t((c_end + 31) >> 5) * 4096u;
+            if (SPLIT == SPLIT_RANGES && first_step(tile) == 0 && end_step(tile) < steps_all && n_ok)
+            {
+                // All steps of this pair have been multiplied: its rings are free for the parts.
+                while (range_begin(range + 1 + parts) < (tile + 1) * steps_all)
+                    ++parts;
+                if (lane == 0)
+                    mbar_expect_tx(&bars->part[quad], uint32_t(parts) * part_bytes);
+                // lane q: part q
+                size_t const block = size_t(range + 1 + lane) * (2 * kEpiWarps) + rank * kEpiWarps + quad;
+                ok = wait_flag(a.flags + block, a.tag, lane < parts, abort_flag);
+                if (ok && lane < parts)
+                {
+                    bulk_g2s(smem + uint32_t(lane * kEpiWarps + quad) * part_block,
+                        reinterpret_cast<uint8_t const*>(a.partial) + block * part_block, part_bytes, &bars->part[quad]);
+                    st_relaxed(a.flags + block, 0ull); // as nobody's: a replayed launch has the same tag
+                }
+                __syncwarp();
+                ok = ok && wait_bar<false>(smem_u32(&bars->part[quad]), 0, abort_flag);
+                if (!ok)
+                    break;
+            }
+            // SPLIT_RANGES: a part of a tile that an earlier range began
+            bool const is_part = SPLIT == SPLIT_RANGES && first_step(tile) > 0;
+            size_t const my_block = size_t(range) * (2 * kEpiWarps) + rank * kEpiWarps + quad;
 #pragma unroll 1
             for (int c0 = 0; c0 < c_end; c0 += 32)
             {
-                uint32_t v[32];
-                tc_ld32(lane_addr + uint32_t(db * a.bm + c0), v);
-                if (c0 + 32 >= c_end)
+                if (MODE != SCALE_GROUP)
+                    tc_ld32(lane_addr + uint32_t(db) * d_cols + uint32_t(c0), v);
+                if (MODE != SCALE_GROUP && c0 + 32 >= c_end)
                 {
                     // everything is in registers: the accumulator may be overwritten
                     tc_fence_before();
@@ -713,7 +1189,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (SPLIT == SPLIT_CLUSTER)
                 {
                     // [row][128 columns] in the activation ring, which no copy or MMA uses any more
-                    float* dst = reinterpret_cast<float*>(smem) + c0 * BN + warp * 32 + lane;
+                    float* dst = reinterpret_cast<float*>(smem) + c0 * BN + quad * 32 + lane;
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         dst[j * BN] = __uint_as_float(v[j]);
@@ -721,26 +1197,40 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 if (!n_ok)
                     continue;
-                if (SPLIT == SPLIT_WORKSPACE)
+                if (is_part)
                 {
-                    // fp32 partial tile; splitk_reduce_kernel, next on the stream, adds the partial tiles in
-                    // split order (deterministic) and writes the output
-                    float* dst = part + size_t(m0 + c0) * a.n;
-                    int const rows = it.row_end - m0 - c0;
+                    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(a.partial) + my_block * part_block)
+                        + (c0 >> 2) * 32 + lane;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j, dst += a.n)
-                        if (j < rows)
-                            __stcg(dst, __uint_as_float(v[j]));
+                    for (int j = 0; j < 8; ++j)
+                        __stcg(dst + 32 * j, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                 __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
                 }
                 else
                 {
+                    if (SPLIT == SPLIT_RANGES)
+#pragma unroll 1
+                        for (int q = 0; q < parts; ++q)
+                        {
+                            float4 const* src
+                                = reinterpret_cast<float4 const*>(smem + uint32_t(q * kEpiWarps + quad) * part_block) + (c0 >> 2) * 32 + lane;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                            {
+                                float4 const x = src[32 * j];
+                                v[4 * j] = __float_as_uint(__uint_as_float(v[4 * j]) + x.x);
+                                v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + x.y);
+                                v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + x.z);
+                                v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + x.w);
+                            }
+                        }
                     // (row pointers are advanced, not computed from the row: with an address product per
                     // row and a bounds test in front of every store a chunk took twice as long)
                     uint32_t o[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        o[j] = P::pack2(fmaf(a.alpha, __uint_as_float(v[2 * j]), bias_f),
-                            fmaf(a.alpha, __uint_as_float(v[2 * j + 1]), bias_f));
+                        o[j] = P::pack2(fmaf(factor, __uint_as_float(v[2 * j]), bias_f),
+                            fmaf(factor, __uint_as_float(v[2 * j + 1]), bias_f));
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
                         o[j] = prmt(o[j], __shfl_xor_sync(0xffffffffu, o[j], 1), sel);
@@ -762,7 +1252,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
             }
-            db = db + 1 == a.d_bufs ? 0 : db + 1;
+            if (is_part && n_ok)
+            {
+                // The pair that adds the parts copies the block by TMA: its values are ordered in front of the flag
+                // for both proxies.
+                asm volatile("fence.proxy.async;" ::: "memory");
+                __threadfence();
+                __syncwarp();
+                if (lane == 0)
+                    st_relaxed(a.flags + my_block, a.tag);
+            }
+            if (MODE != SCALE_GROUP && ++db == a.d_bufs)
+            {
+                db = 0;
+                dph ^= 1;
+            }
         }
     }
 
@@ -777,12 +1281,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     {
         // Every CTA adds the rows row % splits == its split of its 128 columns: a warp per row, four columns
         // per lane, the other splits' values from their shared memory.
-        Item const it = item_of(pair);
-        int const split = it.split, m0 = it.row0, rows = min(a.bm, it.row_end - m0);
+        Place const it = place_of(tile_first);
+        int const m0 = it.row0, rows = min(a.bm, it.row_end - m0);
         int const n = it.n0 + int(rank) * BN + 4 * lane;
         if (n < a.n) // n is a multiple of 32
         {
-            float b[4] = {0.f, 0.f, 0.f, 0.f};
+            float b[4] = {0.f, 0.f, 0.f, 0.f}, f[4] = {a.alpha, a.alpha, a.alpha, a.alpha};
+            if (MODE == SCALE_RAW)
+            {
+                uint2 const sw = *reinterpret_cast<uint2 const*>(static_cast<uint16_t const*>(a.scales) + size_t(it.slice) * a.n + n);
+                P::unpack2(sw.x, f[0], f[1]);
+                P::unpack2(sw.y, f[2], f[3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    f[i] *= a.alpha;
+            }
             if (a.bias)
             {
                 uint2 const bw = *reinterpret_cast<uint2 const*>(static_cast<uint16_t const*>(a.bias) + size_t(it.slice) * a.n + n);
@@ -808,8 +1321,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                         sum.w += x[q].w;
                     }
                 uint2 o;
-                o.x = P::pack2(fmaf(a.alpha, sum.x, b[0]), fmaf(a.alpha, sum.y, b[1]));
-                o.y = P::pack2(fmaf(a.alpha, sum.z, b[2]), fmaf(a.alpha, sum.w, b[3]));
+                o.x = P::pack2(fmaf(f[0], sum.x, b[0]), fmaf(f[1], sum.y, b[1]));
+                o.y = P::pack2(fmaf(f[2], sum.z, b[2]), fmaf(f[3], sum.w, b[3]));
                 *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.out) + size_t(m0 + row) * a.n + n) = o;
             }
         }
@@ -831,61 +1344,28 @@ static size_t split_align(size_t bytes)
     return (bytes + 255) & ~size_t(255);
 }
 
-// Workspace for split-k: `splits` fp32 copies of the output.
-static size_t split_bytes(int m, int n, int splits)
+// Workspace of SPLIT_RANGES: the ranges' flags, and behind them their partial tiles.
+static size_t flag_bytes(int ranges)
 {
-    return size_t(splits) * m * n * sizeof(float);
+    return split_align(size_t(ranges) * 2 * kEpiWarps * sizeof(unsigned long long));
 }
 
-// out[m, n] = alpha * sum over splits (in order) of partial[s, m, n] + bias[n]; four columns per thread.
-template <typename T>
-__global__ void __launch_bounds__(256)
-    splitk_reduce_kernel(T* out, float const* partial, T const* bias, float alpha, size_t mn_vec, int n_vec, int splits)
+static size_t ranges_bytes(int ranges, int bm)
 {
-    using P = Pair<T>;
-    // programmatic dependent of the GEMM: its launch overlaps the GEMM's tail
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    size_t const i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= mn_vec)
-        return;
-    float4 const* src = reinterpret_cast<float4 const*>(partial) + i;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    int sp = 0;
-    for (; sp + 4 <= splits; sp += 4)
-    {
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            v[u] = __ldcg(src + size_t(sp + u) * mn_vec);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-        {
-            acc.x += v[u].x;
-            acc.y += v[u].y;
-            acc.z += v[u].z;
-            acc.w += v[u].w;
-        }
-    }
-    for (; sp < splits; ++sp)
-    {
-        float4 const v = __ldcg(src + size_t(sp) * mn_vec);
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-        acc.w += v.w;
-    }
-    float b[4] = {0.f, 0.f, 0.f, 0.f};
-    if (bias)
-    {
-        uint2 const bw = *reinterpret_cast<uint2 const*>(bias + size_t(i % n_vec) * 4);
-        P::unpack2(bw.x, b[0], b[1]);
-        P::unpack2(bw.y, b[2], b[3]);
-    }
-    uint2 o;
-    o.x = uint32_t(P::from_float(fmaf(alpha, acc.x, b[0]))) | (uint32_t(P::from_float(fmaf(alpha, acc.y, b[1]))) << 16);
-    o.y = uint32_t(P::from_float(fmaf(alpha, acc.z, b[2]))) | (uint32_t(P::from_float(fmaf(alpha, acc.w, b[3]))) << 16);
-    *reinterpret_cast<uint2*>(out + i * 4) = o;
+    return flag_bytes(ranges) + size_t(ranges) * kPairN * bm * sizeof(float);
+}
+
+// A launch's tag: flags hold it only where this launch set them, whatever the workspace held before (and a replay of
+// a captured launch, which has the tag of the one before, finds its flags cleared).
+static unsigned long long next_tag()
+{
+    static std::atomic<unsigned long long> count{
+        (unsigned long long) std::chrono::steady_clock::now().time_since_epoch().count() * 0x2545f4914f6cdd1dull};
+    unsigned long long z = count.fetch_add(0x9e3779b97f4a7c15ull, std::memory_order_relaxed);
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull; // splitmix64
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    z ^= z >> 31;
+    return z ? z : 1;
 }
 
 // Launches a kernel as a programmatic dependent of whatever precedes it in the stream (every kernel
@@ -910,6 +1390,36 @@ static int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t sm
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
 }
 
+// Rings: as many 128-k steps as fit TMEM next to the accumulators (4 at 256 and at 128 rows, more in
+// between and below), the rest of shared memory for weight blocks.
+struct Rings
+{
+    int d_bufs, stages, wstages;
+    size_t bytes;
+};
+
+static Rings rings_of(int bm, int bits, int mode, bool has_zero, size_t smem_most)
+{
+    Rings r;
+    int d_cols = bm, ones = 0;
+    r.d_bufs = bm <= 128 ? 2 : 1;
+    if (mode == SCALE_GROUP)
+    {
+        // an accumulator lives for a step: its MMAs, and the epilogue warps' loads, take turns
+        r.d_bufs = has_zero ? 2 : kMaxDBufs;
+        d_cols = has_zero ? 2 * kGroupBM : kGroupBM;
+        ones = has_zero ? kOnesCols : 0;
+    }
+    r.stages = (kTmemCols - r.d_bufs * d_cols - ones) / kStageCols;
+    r.stages = r.stages < kMaxStages ? r.stages : kMaxStages;
+    size_t const w_stage = size_t(128) * BN * bits / 8 + 1024, act = size_t(r.stages) * bm * 128;
+    size_t const left = smem_most - act - (mode == SCALE_GROUP ? kGroupBytes : 0) - sizeof(Barriers) - 16;
+    r.wstages = int(left / w_stage);
+    r.wstages = r.wstages < kMaxWStages ? r.wstages : kMaxWStages;
+    r.bytes = act + size_t(r.wstages) * w_stage;
+    return r;
+}
+
 // The experts of a launch: neighbours, out of the `slices` of the weight tensor, that have rows. Those that are
 // computed elsewhere get no tiles.
 struct Experts
@@ -924,13 +1434,12 @@ struct Experts
     }
 };
 
-template <typename T, int BITS, bool HAS_ZERO, int SPLIT>
+template <typename T, int BITS, int MODE, bool HAS_ZERO, int SPLIT>
 static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream,
     TcPlan const& plan)
 {
     constexpr int IL = BITS == 4 ? 4 : 2;
-    constexpr int W_STAGE = 2 * (BN / IL) * 128 + 1024;
-    auto kernel = gemm_kernel<T, BITS, HAS_ZERO, SPLIT>;
+    auto kernel = gemm_kernel<T, BITS, MODE, HAS_ZERO, SPLIT>;
 
     Args a{};
     a.bias = p.bias;
@@ -954,24 +1463,24 @@ static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex,
     a.weights_static = (p.flags & W4_GEMM_WEIGHTS_STATIC) ? 1 : 0;
     a.splits = plan.splits;
     a.steps_split = plan.steps_split;
-    if (SPLIT == SPLIT_WORKSPACE)
+    if (SPLIT == SPLIT_RANGES)
     {
-        // partial tiles go to the workspace, behind the scaled copy of the activations if there is one
+        // behind the scaled copy of the activations if there is one
         size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
-        a.partial = reinterpret_cast<float*>(static_cast<char*>(p.workspace) + act_copy);
+        char* const ws = static_cast<char*>(p.workspace) + act_copy;
+        a.flags = reinterpret_cast<unsigned long long*>(ws);
+        a.partial = reinterpret_cast<float*>(ws + flag_bytes(plan.ranges));
+        a.tag = next_tag();
     }
-    // Rings: as many 128-k steps as fit TMEM next to the accumulators (4 at 256 and at 128 rows, more in
-    // between and below), the rest of shared memory for weight blocks.
-    a.d_bufs = plan.bm <= 128 ? 2 : 1;
-    int const stages = (kTmemCols - a.d_bufs * plan.bm) / kStageCols;
-    a.num_stages = stages < kMaxStages ? stages : kMaxStages;
-    size_t const fixed = sizeof(Barriers) + 16;
-    size_t const act_bytes = size_t(a.num_stages) * plan.bm * 128;
-    if (size_t(dev.max_smem_optin) < fixed + act_bytes + 3 * W_STAGE)
+    Rings const r = rings_of(plan.bm, BITS, MODE, HAS_ZERO, size_t(dev.max_smem_optin));
+    if (r.wstages < 3)
         return W4_ERR_CUDA;
-    size_t const wstages = (size_t(dev.max_smem_optin) - fixed - act_bytes) / W_STAGE;
-    a.num_wstages = wstages < size_t(kMaxWStages) ? int(wstages) : kMaxWStages;
-    size_t const smem = act_bytes + size_t(a.num_wstages) * W_STAGE + fixed;
+    a.d_bufs = r.d_bufs;
+    a.num_stages = r.stages;
+    a.num_wstages = r.wstages;
+    a.has_zero = p.zeros != nullptr;
+    a.scales = p.scales;
+    size_t const smem = r.bytes + (MODE == SCALE_GROUP ? kGroupBytes : 0) + sizeof(Barriers) + 16;
 
     // Activations [m, k] of T, boxes of 64 k x bm / 2 rows, 128-byte swizzle (rows past m read as 0).
     // Weights as bytes [k / 64 lines, n / IL interleaved rows, 128], boxes of two lines x 128 / IL rows.
@@ -986,12 +1495,12 @@ static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex,
             uint64_t(p.k) * 2, 128, 128, BN / IL, 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return W4_ERR_CUDA;
     uint64_t const groups = uint64_t(a.groups) * ex.slices;
-    uint32_t const box_rows = p.group_size == 64 ? 2 : 1;
+    uint32_t const box_rows = MODE == SCALE_ROUND && p.group_size == 64 ? 2 : 1;
     if (!make_tensor_map_2d(&tm_s, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.scales, uint64_t(p.n), groups, uint64_t(p.n) * 2, BN,
             box_rows, CU_TENSOR_MAP_SWIZZLE_NONE))
         return W4_ERR_CUDA;
     tm_z = tm_s;
-    if (HAS_ZERO
+    if (p.zeros
         && !make_tensor_map_2d(&tm_z, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.zeros, uint64_t(p.n), groups, uint64_t(p.n) * 2, BN,
             box_rows, CU_TENSOR_MAP_SWIZZLE_NONE))
         return W4_ERR_CUDA;
@@ -1011,45 +1520,48 @@ static int launch_one(W4GemmParams const& p, void const* act, Experts const& ex,
                 configured[dev.device] = true;
         }
     }
-    int const items = a.first_tile[ex.num] * a.splits;
-    int const pairs = SPLIT == SPLIT_CLUSTER || items < dev.num_sms / 2 ? items : dev.num_sms / 2;
-    int rc = launch_pdl(kernel, 2 * pairs, kThreads, smem, SPLIT == SPLIT_CLUSTER ? 2 * a.splits : 2, stream, a, tm_act, tm_w,
+    int const tiles = a.first_tile[ex.num];
+    int const pairs = SPLIT == SPLIT_CLUSTER ? tiles * a.splits
+        : SPLIT == SPLIT_RANGES              ? plan.ranges
+        : tiles < dev.num_sms / 2            ? tiles
+                                             : dev.num_sms / 2;
+    return launch_pdl(kernel, 2 * pairs, kThreads, smem, SPLIT == SPLIT_CLUSTER ? 2 * a.splits : 2, stream, a, tm_act, tm_w,
         tm_s, tm_z);
-    if (rc == W4_OK && SPLIT == SPLIT_WORKSPACE)
-    {
-        size_t const mn_vec = size_t(p.m) * p.n / 4; // n is a multiple of 32
-        rc = launch_pdl(splitk_reduce_kernel<T>, int((mn_vec + 255) / 256), 256, 0, 1, stream, static_cast<T*>(p.out),
-            static_cast<float const*>(a.partial), static_cast<T const*>(p.bias), p.alpha, mn_vec, p.n / 4, a.splits);
-    }
-    return rc;
 }
 
-template <typename T, int BITS, bool HAS_ZERO>
+template <typename T, int BITS, int MODE, bool HAS_ZERO>
 static int dispatch_split(W4GemmParams const& p, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream)
 {
     int rows[kMaxExperts];
     for (int e = 0; e < ex.num; ++e)
         rows[e] = ex.rows(e);
-    // The form of split-k that uses the caller's workspace needs room for the partial tiles there, and its second
-    // kernel adds up and stores all p.m rows with one bias: not for the experts of a 3-D weight, also where a
-    // launch has one expert only.
     size_t const act_copy = (act != p.act) ? split_align(size_t(p.m) * p.k * 2) : 0;
-    TcPlan plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, ex.slices == 1);
-    if (plan.splits > 1 && !plan.cluster && (!p.workspace || p.workspace_bytes < act_copy + split_bytes(p.m, p.n, plan.splits)))
-        plan = gemm_tc_plan(rows, ex.num, p.n, p.k, dev.num_sms, p.weight_bits, p.act_dtype, false);
-    if (plan.splits == 1)
-        return launch_one<T, BITS, HAS_ZERO, SPLIT_NONE>(p, act, ex, dev, stream, plan);
-    return plan.cluster ? launch_one<T, BITS, HAS_ZERO, SPLIT_CLUSTER>(p, act, ex, dev, stream, plan)
-                        : launch_one<T, BITS, HAS_ZERO, SPLIT_WORKSPACE>(p, act, ex, dev, stream, plan);
+    size_t const room = p.workspace && p.workspace_bytes > act_copy ? p.workspace_bytes - act_copy : 0;
+    TcPlan const plan = gemm_tc_plan(rows, ex.num, p, MODE, dev.num_sms, room);
+    if (plan.ranges)
+        return launch_one<T, BITS, MODE, HAS_ZERO, SPLIT_RANGES>(p, act, ex, dev, stream, plan);
+    return plan.splits > 1 ? launch_one<T, BITS, MODE, HAS_ZERO, SPLIT_CLUSTER>(p, act, ex, dev, stream, plan)
+                           : launch_one<T, BITS, MODE, HAS_ZERO, SPLIT_NONE>(p, act, ex, dev, stream, plan);
 }
 
-template <typename T>
-static int dispatch(W4GemmParams const& p, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream)
+template <typename T, int BITS>
+static int dispatch_mode(W4GemmParams const& p, int mode, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream)
 {
-    bool const z = p.zeros != nullptr;
-    if (p.weight_bits == 4)
-        return z ? dispatch_split<T, 4, true>(p, act, ex, dev, stream) : dispatch_split<T, 4, false>(p, act, ex, dev, stream);
-    return z ? dispatch_split<T, 8, true>(p, act, ex, dev, stream) : dispatch_split<T, 8, false>(p, act, ex, dev, stream);
+    if (mode == SCALE_ROUND)
+        return dispatch_split<T, BITS, SCALE_ROUND, true>(p, act, ex, dev, stream);
+    if (mode == SCALE_RAW)
+        return dispatch_split<T, BITS, SCALE_RAW, false>(p, act, ex, dev, stream);
+    return p.zeros ? dispatch_split<T, BITS, SCALE_GROUP, true>(p, act, ex, dev, stream)
+                   : dispatch_split<T, BITS, SCALE_GROUP, false>(p, act, ex, dev, stream);
+}
+
+static int dispatch(W4GemmParams const& p, int mode, void const* act, Experts const& ex, DeviceInfo const& dev, cudaStream_t stream)
+{
+    if (p.act_dtype == W4_DTYPE_FP16)
+        return p.weight_bits == 4 ? dispatch_mode<__half, 4>(p, mode, act, ex, dev, stream)
+                                  : dispatch_mode<__half, 8>(p, mode, act, ex, dev, stream);
+    return p.weight_bits == 4 ? dispatch_mode<__nv_bfloat16, 4>(p, mode, act, ex, dev, stream)
+                              : dispatch_mode<__nv_bfloat16, 8>(p, mode, act, ex, dev, stream);
 }
 
 // Clusters of 2 * splits CTAs the current device runs side by side, by splits: fixed by how its SMs are grouped.
@@ -1070,7 +1582,7 @@ static int const* max_clusters()
     std::lock_guard<std::mutex> lock(mu);
     if (!l.known.load(std::memory_order_relaxed))
     {
-        auto kernel = gemm_kernel<__nv_bfloat16, 4, true, SPLIT_CLUSTER>;
+        auto kernel = gemm_kernel<__nv_bfloat16, 4, SCALE_ROUND, true, SPLIT_CLUSTER>;
         bool const ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin) == cudaSuccess
             && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         for (int s = 1; s <= kMaxClusterSplits; ++s)
@@ -1096,68 +1608,118 @@ static int const* max_clusters()
 
 } // namespace tc
 
-// Microseconds per 128-wide k step of a CTA pair (measured on B200): up to 96 rows the conversion's, which
-// takes most of the issue slots and, for int8 to bf16, more instructions per weight; above, the MMAs'
-// (1024 tensor cycles at 256 rows).
-static double step_us(int bm, int bits, int act_dtype)
+// Microseconds per 128-wide k step of a CTA pair (measured on B200, few rows unless said): what converting the
+// weights takes, or the MMAs (1024 tensor cycles at 256 rows, proportional to the rows above 96), or the weights' way
+// from memory for as many pairs as work at a time (6.3 TB/s).
+static double step_us(int bm, W4GemmParams const& p, int mode, double busy_pairs)
 {
-    double const conv = bits == 8 && act_dtype == W4_DTYPE_BF16 ? 0.33 : 0.25, mma = bm * (0.57 / 256);
-    return conv > mma ? conv : mma;
+    bool const w8 = p.weight_bits == 8;
+    double conv;
+    if (mode == tc::SCALE_RAW)
+        conv = w8 && p.act_dtype == W4_DTYPE_BF16 ? 0.235 : w8 ? 0.22 : 0.2;
+    else if (mode == tc::SCALE_GROUP)
+        conv = p.group_size == 64 ? 0.49 : w8 ? 0.385 : p.zeros ? 0.36 : 0.32;
+    else
+        conv = w8 && p.act_dtype == W4_DTYPE_BF16 ? 0.285 : 0.25;
+    double const mma = bm * (0.57 / 256), memory = busy_pairs * tc::kPairN * 128 * p.weight_bits / 8 / 6.3e6;
+    conv = conv > mma ? conv : mma;
+    return conv > memory ? conv : memory;
 }
 
-// The plan with the shortest estimated time: row tiles in steps of 32 and, where the tiles leave pairs idle
-// (and only up to 256 rows, where the fp32 partial tiles stay small), split factors. A launch costs 2.5 us plus
-// the waves of its work items; an item's epilogue 0.3 us per 32 rows, of which the double-buffered
-// accumulators hide all but the last. Splits that share a cluster add the exchange of the partial tiles
-// (clusters of 4 and 8 CTAs about 1 us; 6 and more than 8 wait longer for enough free SMs side by side), splits
-// through the workspace a second kernel and their traffic. Fitted to 4096 and 8192 x 1024..14336 at 16 to
-// 777 rows, each launch by itself: within 1 us of the best plan found by trying all at 14 of 16 points. Beyond
-// that, and in long runs at the power limit, it is too low (14336 x 4096 at 4096 rows 228 us, measured 302 cool
+// The plan with the shortest estimated time. A launch costs 4 us (2.2 where it leaves half of the SMs
+// to the next one) plus the waves of its work items; an item's epilogue 0.3 us per 32 rows, of which the
+// double-buffered accumulators hide all but the last. Clusters add 1.2 us for the exchange of the partial tiles
+// (2.4 above 8 CTAs), equal ranges 3.5 us and 15 % of the steps: a part's way through memory, its flag, and the copies into the shared memory of
+// the pair that adds. So ranges pay where whole tiles would leave pairs idle for longer than that. Beyond 777 rows, and
+// in long runs at the power limit, the estimate is too low (14336 x 4096 at 4096 rows 228 us, measured 302 cool
 // and 356 sustained) and says only which row tile has the fewest waves.
-TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace)
+static TcPlan search_plan(int const* rows, int experts, W4GemmParams const& p, int mode, int num_sms, size_t room)
 {
+    int const n = p.n;
     int const pairs = num_sms > 1 ? num_sms / 2 : 1;
-    int const steps = (k + 127) / 128;
-    long const tiles_n = (n + tc::kPairN - 1) / tc::kPairN;
+    int const steps = (p.k + 127) / 128;
+    int const tiles_n = (n + tc::kPairN - 1) / tc::kPairN;
     int const* const clusters = tc::max_clusters();
-    TcPlan best{};
+    TcPlan best{}, cut{}; // cut: the best with equal ranges
+    double whole = 0;     // the shortest time of whole tiles
     int m = 0; // most rows of an expert
     for (int e = 0; e < experts; ++e)
         m = m > rows[e] ? m : rows[e];
-    int const most = m >= tc::kMaxBM ? tc::kMaxBM : (m + 31) & ~31;
+    int const most = mode == tc::SCALE_GROUP ? tc::kGroupBM : m >= tc::kMaxBM ? tc::kMaxBM : (m + 31) & ~31;
     for (int bm = 32; bm <= most; bm += 32)
     {
-        long tiles = 0;
+        int tiles = 0;
         for (int e = 0; e < experts; ++e)
             tiles += tiles_n * ((rows[e] + bm - 1) / bm);
-        double const step = step_us(bm, bits, act_dtype), drain = 0.01 * bm;
+        double const drain = 0.01 * bm, again = bm <= 128 ? 0.1 : drain + 0.3;
         int splits_max = m <= 256 && tiles < pairs ? int(pairs / tiles) : 1;
-        splits_max = splits_max > 16 ? 16 : splits_max;
+        splits_max = splits_max > tc::kMaxClusterSplits ? tc::kMaxClusterSplits : splits_max;
         for (int s = 1; s <= splits_max; ++s)
         {
             int const per = (steps + s - 1) / s;
-            if ((steps + per - 1) / per != s || (s > 1 && per < 2))
-                continue; // an empty work item, or too little in each
-            bool const cluster = s > 1 && s <= tc::kMaxClusterSplits && tiles <= clusters[s];
-            if (s > 1 && !cluster && !may_use_workspace)
-                continue;
+            if ((steps + per - 1) / per != s || (s > 1 && (per < 2 || tiles > clusters[s])))
+                continue; // an empty work item, too little in each, or more clusters than run side by side
             double const waves = double((tiles * s + pairs - 1) / pairs);
-            double us = 2.5 + drain + waves * per * step + (waves - 1) * (bm <= 128 ? 0.1 : drain + 0.3);
-            if (cluster)
-                us += (s == 2 || s == 4 ? 1.0 : 3.0) + 0.008 * bm;
-            else if (s > 1)
-                us += 2.5 + double(s) * m * n * 8.0 / 6.0e6;
+            double const busy = double(tiles * s) / waves;
+            double us = (2 * tiles * s <= pairs ? 2.2 : 4.0) + drain + waves * per * step_us(bm, p, mode, busy) + (waves - 1) * again;
+            if (s > 1)
+                us += (s > 4 ? 2.4 : 1.2) + 0.008 * bm;
+            else if (!whole || us < whole)
+                whole = us;
             if (!best.bm || us < best.us)
-            {
-                best.bm = bm;
-                best.splits = s;
-                best.steps_split = per;
-                best.cluster = cluster;
-                best.us = us;
-            }
+                best = TcPlan{bm, s, per, 0, us, 0};
         }
+        // Equal ranges: as many as there are pairs, or fewer where a tile's parts would not fit a pair's shared memory.
+        int const most_parts = int(tc::rings_of(bm, p.weight_bits, mode, p.zeros != nullptr, tc::kSmemMost).bytes / (size_t(tc::kEpiWarps) * bm * 128));
+        int const total = tiles * steps, least = (steps - 1 + most_parts - 1) / most_parts; // steps of a range
+        int ranges = total / (least > 2 ? least : 2);
+        ranges = ranges < pairs ? ranges : pairs;
+        if (m > tc::kMaxRangesRows || bm > tc::kMaxRangesBM || ranges < 2 || (total % ranges == 0 && total / ranges % steps == 0) || room < tc::ranges_bytes(int(ranges), bm))
+            continue;
+        int const per = (total + ranges - 1) / ranges, parts = (steps - 1 + total / ranges - 1) / (total / ranges);
+        double const us = 7.5 + drain + 1.15 * per * step_us(bm, p, mode, double(ranges)) + double((per + steps - 2) / steps) * again
+            + 0.004 * bm * double(parts);
+        if (!cut.bm || us < cut.us)
+            cut = TcPlan{bm, 1, steps, int(ranges), us, 0};
     }
+    if (cut.bm && (!best.bm || cut.us < best.us))
+        best = cut;
+    // (up to 256 rows asked for in any case: an estimate is no promise to a caller who sizes its workspace once)
+    best.workspace = cut.bm && (cut.us < whole || m <= tc::kMaxRangesRows) ? tc::ranges_bytes(cut.ranges, cut.bm) : 0;
     return best;
+}
+
+// The search takes a few hundred nanoseconds, and a call asks for its workspace, for the kernel to take and for the plan:
+// the last plan of each thread with and without workspace is kept by what it depends on, sizes and types.
+TcPlan gemm_tc_plan(int const* rows, int experts, W4GemmParams const& p, int mode, int num_sms, size_t room)
+{
+    struct Last
+    {
+        int key[9];
+        TcPlan plan;
+    };
+    static thread_local Last last[2] = {};
+    if (experts != 1)
+        return search_plan(rows, experts, p, mode, num_sms, room);
+    Last& l = last[room != 0];
+    int const key[9] = {rows[0], p.n, p.k, p.weight_bits, p.act_dtype, p.group_size, p.zeros != nullptr, mode + 4 * num_sms,
+        current_device_info().device};
+    if (!l.plan.bm || std::memcmp(l.key, key, sizeof key) != 0)
+    {
+        l.plan = search_plan(rows, 1, p, mode, num_sms, room ? ~size_t(0) : 0);
+        std::memcpy(l.key, key, sizeof key);
+    }
+    if (l.plan.ranges && room < l.plan.workspace)
+        return search_plan(rows, 1, p, mode, num_sms, room);
+    return l.plan;
+}
+
+size_t gemm_tc_workspace(W4GemmParams const& p, bool exact)
+{
+    DeviceInfo const& dev = current_device_info();
+    TcPlan const plan = gemm_tc_plan(&p.m, 1, p, gemm_tc_mode(p, exact), dev.num_sms > 0 ? dev.num_sms : 148, ~size_t(0));
+    size_t const scaled = gemm_tc_workspace_min(p.m, p.k, p.act_scale != nullptr);
+    return plan.ranges ? tc::split_align(scaled) + plan.workspace : scaled;
 }
 
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale)
@@ -1172,15 +1734,27 @@ size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits,
     // what lets the kernel use every form of split-k; with less (but at least the minimum) it runs with the
     // forms that need none
     DeviceInfo const& dev = current_device_info();
-    int const sms = dev.num_sms > 0 ? dev.num_sms : 148;
-    int const splits = gemm_tc_plan(&m, 1, n, k, sms, bits, act_dtype, true).splits;
+    W4GemmParams p{};
+    p.n = n;
+    p.k = k;
+    p.weight_bits = bits;
+    p.act_dtype = act_dtype;
+    p.group_size = 128; // (whichever: the plan of a launch with other scales may differ, and makes do with what there is)
+    TcPlan const plan = gemm_tc_plan(&m, 1, p, tc::SCALE_ROUND, dev.num_sms > 0 ? dev.num_sms : 148, ~size_t(0));
     size_t bytes = gemm_tc_workspace_min(m, k, has_act_scale);
-    if (splits > 1)
-        bytes = tc::split_align(bytes) + tc::split_bytes(m, n, splits);
+    if (plan.workspace)
+        bytes = tc::split_align(bytes) + plan.workspace;
     return bytes;
 }
 
-int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream)
+int gemm_tc_mode(W4GemmParams const& p, bool exact)
+{
+    if (!p.group_size && !p.zeros)
+        return tc::SCALE_RAW;
+    return exact ? tc::SCALE_GROUP : tc::SCALE_ROUND;
+}
+
+int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream, bool exact)
 {
     DeviceInfo const& dev = current_device_info();
     if (dev.num_sms <= 0)
@@ -1194,12 +1768,11 @@ int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream)
         act = p.workspace;
     }
     tc::Experts const one{1, 1, {0}, {0, p.m}, {false}};
-    return p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, act, one, dev, stream)
-                                        : tc::dispatch<__nv_bfloat16>(p, act, one, dev, stream);
+    return tc::dispatch(p, gemm_tc_mode(p, exact), act, one, dev, stream);
 }
 
 int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, bool (*joins)(W4GemmParams const&, int),
-    cudaStream_t stream)
+    bool exact, cudaStream_t stream)
 {
     DeviceInfo const& dev = current_device_info();
     if (dev.num_sms <= 0)
@@ -1222,8 +1795,7 @@ int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* fi
             continue;
         if (any)
         {
-            int const rc = p.act_dtype == W4_DTYPE_FP16 ? tc::dispatch<__half>(p, p.act, ex, dev, stream)
-                                                        : tc::dispatch<__nv_bfloat16>(p, p.act, ex, dev, stream);
+            int const rc = tc::dispatch(p, gemm_tc_mode(p, exact), p.act, ex, dev, stream);
             if (rc != W4_OK)
                 return rc;
         }

@@ -1072,26 +1072,30 @@ static int dispatch_bits(Args const& a, int bits, int mb, DeviceInfo const& dev,
 
 } // namespace gemv
 
-// Microseconds of the passes of this file's kernel, as measured. Up to 8 rows: 3 us plus the weight bytes at
-// 4.1 (int4; k rounded up to panels of 4096, which a pass walks whatever they hold) or 3.6 TB/s (int8), 0.1 us
-// per 1024 k beyond the first panel (activations are reloaded), more above four rows and 15 % more for 64-wide
-// groups on int4 (weights are rounded one by one). 16 rows: int4 6.3 us plus the bytes at 2.7 TB/s, int8 3 us
-// at 3.6 TB/s, under bf16 activations 5 us at 3.1 TB/s (two nibble planes).
+// Microseconds of the passes of this file's kernel, as measured on shapes from 2048 x 2048 to 28672 x 8192. int4 up to 8
+// rows: 3 us plus the weight bytes at 4.1 TB/s (k rounded up to panels of 4096, which a pass walks whatever they hold),
+// 0.1 us per 1024 k beyond the first panel (activations are reloaded), more above four rows and 15 % more for 64-wide
+// groups (weights are rounded one by one). 16 rows, and int8: a fixed part plus the bytes of the SM with the most
+// interleaved rows (1.85 TB/s over all SMs for int4, 2.6 and 3.5 for int8 under bf16 and fp16, 3.3 and 4.0 up to 8 rows).
 static double staged_us(W4GemmParams const& p)
 {
-    bool const w4 = p.weight_bits == 4;
-    double const mb = double(p.n) * double(p.k) * p.weight_bits / 8.0 / 1.0e6;
+    bool const w4 = p.weight_bits == 4, bf16 = p.act_dtype == W4_DTYPE_BF16;
+    double const mb = double(p.n) * double(p.k) * p.weight_bits / 8.0 / 1.0e6, over = p.k > 4096 ? (p.k - 4096) / 1024.0 : 0.0;
+    double const rows = double(p.n) / (w4 ? 4 : 2), sms = 148.0, per_sm = double((long(rows) + 147) / 148);
+    double const most = mb * per_sm * sms / rows;
     double us = 0;
     int left = p.m;
     for (; left > 8; left -= left < 16 ? left : 16)
-        us += w4 ? mb / 2.7 + 6.3 : (p.act_dtype == W4_DTYPE_BF16 ? mb / 3.1 + 5.0 : mb / 3.6 + 3.0);
-    if (left > 0)
+        us += (w4 ? 3.0 + 0.54 * most : (bf16 ? 3.0 + 0.38 * most : 3.4 + 0.287 * most)) + (per_sm < 8 ? 0.2 * over : 0.0);
+    if (left > 0 && !w4)
+        us += (bf16 ? 2.2 + 0.3 * most : 2.4 + 0.25 * most) + (p.k <= 1024 ? 0.8 : 0.0) + (per_sm < 8 ? 0.2 * over : 0.0);
+    else if (left > 0)
     {
-        double const padded = w4 ? double((p.k + 4095) / 4096 * 4096) / p.k : 1.0, over = p.k > 4096 ? (p.k - 4096) / 1024.0 : 0.0;
-        us += 3.0 + mb * padded / (w4 ? 4.1 : 3.6) + (w4 ? 0.1 : 0.2) * over
-            + (left > 4 ? 0.003 * mb * (left - 4) * (left - 4) : 0.0);
+        double const padded = double((p.k + 4095) / 4096 * 4096) / p.k;
+        double const pass = 3.0 + mb * padded / 4.1 + 0.1 * over + (left > 4 ? (p.group_size == 64 ? 0.001 : 0.003) * mb * (left - 4) * (left - 4) : 0.0);
+        us += p.group_size == 64 ? 1.15 * pass : pass;
     }
-    return w4 && p.group_size == 64 ? 1.15 * us : us;
+    return us;
 }
 
 // The same of the streaming kernel: 2.9 us plus the bytes at 4.75 TB/s up to 42 MB and 5.6 TB/s beyond, and

@@ -48,27 +48,34 @@ double gemv_estimate_us(W4GemmParams const& p);
 bool allreduce_push_target(W4AllReduceParams const& r, PushTarget* t);
 
 // tcgen05 tensor-core kernel. Returns a W4Status.
-int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream);
+// `exact`: scales and zeros are applied to 32-bit sums, as the decode kernels do, not to the weights.
+int launch_gemm_tc(W4GemmParams const& p, cudaStream_t stream, bool exact = false);
 // Workspace: the minimum the kernel needs (scaled activation copy), and what also allows split-k.
 size_t gemm_tc_workspace_min(int m, int k, int has_act_scale);
+// (for the problem as it is: what the fastest plan uses)
+size_t gemm_tc_workspace(W4GemmParams const& p, bool exact);
 size_t gemm_tc_workspace_bytes(int m, int n, int k, int has_act_scale, int bits, int act_dtype);
 // Those experts of a 3-D weight tensor that joins() with their rows, in one launch for every 32 that have rows: p.m
 // is the end of the last expert's rows, expert e has rows first_row[e] .. first_row[e + 1] - 1. No pre-quant scale,
 // no workspace.
 int launch_gemm_tc_experts(W4GemmParams const& p, int num_experts, int const* first_row, bool (*joins)(W4GemmParams const&, int),
-    cudaStream_t stream);
+    bool exact, cudaStream_t stream);
 // How the tensor-core kernel runs a problem (or the experts of one, by their rows): activation rows per tile,
-// split-k factor and 128-wide k steps per work item, and the estimated duration (microseconds, from measured
+// how CTA pairs share the k range of a tile, and the estimated duration (microseconds, from measured
 // step costs); shared by the launcher, the workspace size and the choice of the kernel in w4_api.cu.
 struct TcPlan
 {
     int bm = 0;
-    int splits = 1;
-    int steps_split = 0;
-    bool cluster = false; // the splits of a tile are one cluster (otherwise they meet in the workspace)
+    int splits = 1;      // CTA pairs of a tile, one cluster (1: no split of this kind)
+    int steps_split = 0; // 128-wide k steps of each
+    int ranges = 0;      // equal ranges of the steps of all tiles, with partial tiles in the workspace (0: none)
     double us = 0;
+    size_t workspace = 0; // what equal ranges need
 };
-TcPlan gemm_tc_plan(int const* rows, int experts, int n, int k, int num_sms, int bits, int act_dtype, bool may_use_workspace);
+// Of p: n, k, the types and whether there are zeros. `room`: bytes of workspace for partial tiles.
+TcPlan gemm_tc_plan(int const* rows, int experts, W4GemmParams const& p, int mode, int num_sms, size_t room);
+// The kernel's arithmetic for a problem.
+int gemm_tc_mode(W4GemmParams const& p, bool exact);
 
 // out[m, k] = act[m, k] * scale[k], rounded to the element type (the reference's
 // apply_per_channel_scale, cpp/tensorrt_llm/kernels/preQuantScaleKernel.cu:43-95).

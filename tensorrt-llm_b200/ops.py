@@ -102,15 +102,16 @@ def moe_gemm(act, weight, scales, expert_first_row: Sequence[int], *, weight_bit
     if m == 0:
         return out
     rows = [b - a for a, b in zip(first[:-1], first[1:]) if b > a]
-    ws = None
-    if len(rows) == 1 or act_scale is not None:  # otherwise decode launches and a shared one, which need none
+    if len(rows) == 1 or act_scale is not None:
         nws = workspace_bytes_max(max(rows), n, k, group_size, weight_bits, act.dtype, act_scale is not None)
-        ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=act.device)
+    else:  # shared launches need none, but with room for 32 rows' partial tiles of all SM pairs they can cut k anywhere
+        nws = 4 << 20
+    ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=act.device)
     params = W4GemmParams(
         act=_p(act), act_scale=_p(act_scale), weight=_p(weight), scales=_p(scales), zeros=_p(zeros), bias=_p(bias),
         out=_p(out), alpha=float(alpha), m=m, n=n, k=k, group_size=group_size, weight_bits=weight_bits,
         act_dtype=_DTYPES[act.dtype], regime=W4_REGIME_AUTO, workspace=_p(ws),
-        workspace_bytes=0 if ws is None else ws.numel(),
+        workspace_bytes=ws.numel(),
         flags=_lib.W4_GEMM_WEIGHTS_STATIC if weights_static else 0)
     offsets = (ctypes.c_int * (e + 1))(*first)
     with torch.cuda.device(act.device):

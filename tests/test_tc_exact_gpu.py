@@ -1,0 +1,134 @@
+"""The tensor-core kernel with scales applied to 32-bit sums, and with the k range cut into equal ranges (needs a B200)."""
+import pytest
+import torch
+
+import tensorrt_llm_b200 as pkg
+from tensorrt_llm_b200 import quantize
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(m, n, k, bits, group, dtype, zero, bias, seed, lead=()):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    packed = torch.randint(-128, 128, lead + (k, n * bits // 8), dtype=torch.int8, generator=g, device="cuda")
+    qt = torch.quint4x2 if bits == 4 else torch.int8
+    lay = quantize.preprocess_weights_for_mixed_gemm_cuda
+    weight = torch.stack([lay(p, qt) for p in packed]) if lead else lay(packed, qt)
+    shape = lead + ((k // group, n) if group else (n,))
+    scales = (torch.rand(shape, generator=g, device="cuda") * 0.019 + 0.001).to(dtype)
+    zeros = (torch.rand(shape, generator=g, device="cuda") * 0.2 - 0.1).to(dtype) if zero else None
+    b = torch.randn(lead + (n,), generator=g, device="cuda").to(dtype) if bias else None
+    act = torch.randn((m, k), generator=g, device="cuda").to(dtype)
+    q = packed if bits == 8 else torch.stack([(packed << 4) >> 4, packed >> 4], -1).flatten(-2)
+    return act, weight, scales, zeros, b, q
+
+
+def _close(out, act, q, scales, zeros, bias, group):
+    """Within the rounding of the output, half a unit in its last place, and that of 32-bit sums: every product is exact,
+    and a sum of k terms errs by less than 2^-18 of the sum of their sizes for k up to 32768 added in chains of 64."""
+    spread = (lambda t: t.double().repeat_interleave(group, 0)) if group else (lambda t: t.double())
+    w = q.double() * spread(scales)
+    size = w.abs()
+    if zeros is not None:
+        w, size = w + spread(zeros), size + spread(zeros).abs()
+    a = act.double()
+    ref = a @ w + (0 if bias is None else bias.double())
+    half = 2.0 ** (-8 if out.dtype == torch.bfloat16 else -11)
+    return bool(((out.double() - ref).abs() <= half * ref.abs() * (1 + 2.0 ** -8) + 2.0 ** -18 * (a.abs() @ size) + 1e-7).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,bits,group,zero,bias", [
+    (1, 14336, 4096, 8, 0, False, False),     # whole tiles
+    (16, 14336, 4160, 8, 0, False, True),     # half a step at the end
+    (5, 4032, 14336, 8, 0, False, False),     # clusters, a ragged last tile
+    (16, 14336, 4096, 4, 128, True, False),
+    (13, 14400, 4224, 4, 128, False, True),
+    (16, 20480, 1024, 8, 128, True, True),
+    (7, 20512, 2048, 8, 0, True, False),      # one scale per column and zeros: one group for all k
+    (9, 8192, 28672, 4, 0, False, False),
+    (16, 8192, 28672, 4, 128, True, True),    # clusters
+    (33, 28672, 1024, 8, 64, True, False),    # two groups a step, more than one row tile
+])
+def test_decode_regime_on_the_tensor_cores(m, n, k, bits, group, zero, bias, dtype):
+    """Requested and automatic launches of the decode regime, whichever kernel runs: one result, scales on 32-bit sums."""
+    act, weight, scales, zeros, b, q = _problem(m, n, k, bits, group, dtype, zero, bias, seed=n + m)
+    kw = dict(weight_bits=bits, group_size=group, zeros=zeros, bias=b, weights_static=True)
+    for regime in (pkg.W4_REGIME_GEMV, pkg.W4_REGIME_AUTO):
+        if regime == pkg.W4_REGIME_AUTO and pkg.ops.select_regime(m, n, k, group, bits, dtype) != pkg.W4_REGIME_GEMV:
+            continue
+        out = torch.full((m, n), float("nan"), dtype=dtype, device="cuda")
+        pkg.ops.gemm_raw(act, weight, scales, out, n=n, k=k, regime=regime, **kw)
+        assert _close(out, act, q, scales, zeros, b, group), regime
+    assert pkg._lib.lib().w4_gemm_device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,bits,group", [
+    (33, 10176, 8192, 4, 128),   # a ragged last tile, parts of two row tiles
+    (64, 10240, 8128, 4, 64),    # half a step at the end
+    (100, 19968, 4096, 8, 0),    # more tiles than pairs
+    (20, 4096, 14336, 4, 128),   # a tile's parts from several pairs
+])
+def test_equal_ranges(m, n, k, bits, group):
+    """With the workspace that the library asks for, whatever it holds before: the same outputs on every launch, in a
+    replayed graph and next to a launch with a workspace of its own on another stream, and those of whole tiles up to
+    the order of 32-bit sums."""
+    dtype = torch.bfloat16
+    act, weight, scales, zeros, b, _ = _problem(m, n, k, bits, group, dtype, group != 0, True, seed=m)
+    nws = pkg.ops.workspace_bytes(m, n, k, group, bits, dtype, False, pkg.W4_REGIME_GEMM)
+    assert nws > 0
+    wss = [torch.randint(0, 256, (nws,), dtype=torch.uint8, device="cuda") for _ in range(2)]
+
+    def run(ws):
+        out = torch.full((m, n), float("nan"), dtype=dtype, device="cuda")
+        pkg.ops.gemm_raw(act, weight, scales, out, n=n, k=k, weight_bits=bits, group_size=group, zeros=zeros, bias=b,
+                         regime=pkg.W4_REGIME_GEMM, workspace=ws, weights_static=True)
+        return out
+
+    whole, first = run(None), run(wss[0])
+    assert float((first.double() - whole.double()).abs().max()) <= 2.0 ** -7 * float(whole.abs().max())
+    streams = [torch.cuda.Stream() for _ in wss]
+    torch.cuda.synchronize()
+    outs = []
+    for _ in range(4):
+        for s, ws in zip(streams, wss):
+            with torch.cuda.stream(s):
+                outs.append(run(ws))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = run(wss[0])
+    for _ in range(3):
+        replayed.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(replayed, first)
+    assert all(torch.equal(o, first) for o in outs)
+    assert pkg._lib.lib().w4_gemm_device_status() == 0
+
+
+@pytest.mark.parametrize("bits,group,rows", [
+    (4, 128, [3, 17, 0, 1, 9, 32]),
+    (4, 128, [5, 40, 16, 120]),
+    (8, 0, [2, 0, 33, 8]),
+    (8, 64, [1, 15, 7]),
+])
+def test_large_experts(bits, group, rows):
+    """Experts large enough to share launches: rows of the decode regime have its arithmetic, the others that of the
+    tensor-core kernel, whose weights are rounded."""
+    n, k, dtype = 8192, 2048, torch.bfloat16
+    first = [0]
+    for r in rows:
+        first.append(first[-1] + r)
+    act, weight, scales, zeros, b, q = _problem(first[-1], n, k, bits, group, dtype, group != 0, True, seed=len(rows),
+                                                lead=(len(rows),))
+    out = pkg.ops.moe_gemm(act, weight, scales, first, weight_bits=bits, group_size=group, zeros=zeros, bias=b, weights_static=True)
+    for e, r in enumerate(rows):
+        part = slice(first[e], first[e + 1])
+        args = act[part], q[e], scales[e], None if zeros is None else zeros[e], b[e], group
+        if r and pkg.ops.select_regime(r, n, k, group, bits, dtype) == pkg.W4_REGIME_GEMV:
+            assert _close(out[part], *args), e
+        elif r:
+            spread = (lambda t: t.double().repeat_interleave(group, 0)) if group else (lambda t: t.double())
+            w = q[e].double() * spread(scales[e]) + (0 if zeros is None else spread(zeros[e]))
+            ref = act[part].double() @ w + b[e].double()
+            assert float((out[part].double() - ref).abs().max()) <= 1e-2 * float(ref.abs().max()), e
