@@ -11,6 +11,7 @@
 // adjacent columns - the closed form of the four reference passes (row permutation inside 16/32-row
 // blocks, sub-byte transpose, column interleave in 64-k tiles, bias + in-register shuffle).
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -375,9 +376,9 @@ __global__ void __launch_bounds__(kThreads)
 // bytes of each row) and all of K: every CTA brings its rows of the strip into shared
 // memory by TMA, finds their column maxima as the 64-row boxes land, the cluster combines the maxima through
 // distributed shared memory, and the weights are quantised and laid out straight from shared memory.
-// HBM-bound: each weight is read from memory once (the two passes of the kernels below read it twice, and
-// scales were a memset, an atomic merge and a launch in between). 4096 x 14336 bf16 -> int4: 98 -> 56 us
-// per call. A thread turns one block of 32 (int4) / 16 (int8) rows x 8 columns - what four adjacent output
+// Each weight is read from memory once (the two passes of the kernels below read it twice, and
+// scales were a memset, an atomic merge and a launch in between). 4096 x 14336 bf16 -> int4: 98 -> 48.7 us
+// per call, 3.0 TB/s; what bounds it is that a cluster's phases follow one another. A thread turns one block of 32 (int4) / 16 (int8) rows x 8 columns - what four adjacent output
 // registers of each column hold - so all its stores are 16 bytes and a warp writes whole 32-byte sectors.
 // Several CTAs share an SM, so that one's arithmetic covers another's loads.
 // ------------------------------------------------------------------------------------------------
@@ -553,9 +554,35 @@ __device__ __forceinline__ void quantize8(float const (&x)[8], StripScales<W> co
     }
     else
     {
+        // The sums' low halves are the integers, made positive: two to a register, cut off there, shifted together.
+        // 19 to 20 instructions for eight weights where taking the rounding constant away, cutting off each float and
+        // packing by multiplications took 33.
+        constexpr float kUp = kRound + kHi + 1.f;
+        uint32_t u[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-            q[e] = fminf(fmaf(x[e], c.inv[e], kRound), kRound + kHi) - kRound;
+        for (int e = 0; e < 8; e += 2)
+        {
+            uint64_t y;
+            asm("{\n.reg .b64 x, i, r;\n"
+                "mov.b64 x, {%1, %2};\nmov.b64 i, {%3, %4};\nmov.b64 r, {%5, %5};\n"
+                "fma.rn.f32x2 %0, x, i, r;\n}\n"
+                : "=l"(y)
+                : "f"(x[e]), "f"(x[e + 1]), "f"(c.inv[e]), "f"(c.inv[e + 1]), "f"(kUp));
+            u[e] = uint32_t(y);
+            u[e + 1] = uint32_t(y >> 32);
+        }
+        constexpr uint32_t kMost = BITS == 8 ? 0x00ff00ffu : 0x000f000fu;
+        constexpr int HALF = 16 / BITS; // elements of half a register
+#pragma unroll
+        for (int w = 0; w < BITS / 4; ++w)
+        {
+            uint32_t r = 0;
+#pragma unroll
+            for (int e = HALF - 1; e >= 0; --e)
+                r = (r << BITS) + __vminu2(prmt(u[2 * HALF * w + e], u[2 * HALF * w + e + HALF], 0x5410u), kMost);
+            word[w] = r;
+        }
+        return;
     }
     pack_q<BITS>(q, word);
 }
@@ -580,9 +607,19 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     uint32_t rank, ranks;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
-    int const n0 = int(blockIdx.x / ranks) * S;
+    // 16-bit weights: the grid holds as many clusters as run side by side, each takes every num_clusters-th strip, and a
+    // strip's successor is fetched box by box as its own boxes are done with; a cluster for every strip waited for eight
+    // free places at a time and loaded with nothing else to do. bf16 4096 x 14336 to int4 55.1 -> 48.7 us, to int8
+    // 63 -> 59. fp32, which reads twice as much for as many stores, takes 3 % longer that way: a strip each.
+    constexpr bool PERSISTENT = sizeof(W) == 2;
+    int const num_clusters = int(gridDim.x / ranks);
     int const t0 = int(rank) * a.tiles_cta, tiles = min(a.tiles_cta, a.K / 64 - t0); // <= 0: nothing here
     int const tid = threadIdx.x, lane = tid & 31, cv = tid % NV;
+    auto fetch = [&](int strip, int i)
+    {
+        mbar_expect_tx(&full[i], TILE_BYTES);
+        tma_load_2d(slab + i * TILE_BYTES, &tm, strip * S, (t0 + i) * 64, &full[i]);
+    };
     if (tid == 0)
     {
         failed = 0;
@@ -597,186 +634,211 @@ __global__ void __launch_bounds__(kMaxStripThreads) strip_quantize_kernel(StripA
     asm volatile("griddepcontrol.wait;" ::: "memory"); // the weights, and what the outputs held before
     if (tid == 0)
         for (int i = 0; i < tiles; ++i)
-        {
-            mbar_expect_tx(&full[i], TILE_BYTES);
-            tma_load_2d(slab + i * TILE_BYTES, &tm, n0, (t0 + i) * 64, &full[i]);
-        }
+            fetch(int(blockIdx.x / ranks), i);
 
-    // ---- column maxima: a thread walks one vector of columns
-    float m[8];
+    uint32_t phase = 0;
     bool ok = true;
-    if constexpr (std::is_same<W, float>::value)
+    for (int strip = int(blockIdx.x / ranks); strip * S < a.N; strip += num_clusters, phase ^= 1)
     {
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            m[e] = 0.f;
-        for (int i = 0; i < tiles && ok; ++i)
+        int const n0 = strip * S;
+        // ---- column maxima: a thread walks one vector of columns
+        float m[8];
+        if constexpr (std::is_same<W, float>::value)
         {
-            ok = mbar_wait(&full[i], 0);
-            for (int r = tid / NV; r < 64 && ok; r += int(blockDim.x) / NV)
-            {
-                float x[8];
-                strip_load8<W>(slab + i * TILE_BYTES + r * kStripBytes, cv, (tid / NV) & 1, x);
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    m[e] = fmaxf(m[e], fabsf(x[e]));
-            }
-        }
-    }
-    else
-    {
-        StripMax<W, true> pm;
-        pm.clear();
-        for (int i = 0; i < tiles && ok; ++i)
-        {
-            ok = mbar_wait(&full[i], 0);
-            for (int r = tid / NV; r < 64 && ok; r += int(blockDim.x) / NV)
-                pm.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
-        }
-        pm.get(m);
-        bool nan = false;
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            nan |= m[e] != m[e];
-        if (nan)
-        {
-            // once more without them; the threads that quantise this CTA's rows divide
-            has_nan = 1;
-            StripMax<W, false> numbers;
-            numbers.clear();
+            for (int e = 0; e < 8; ++e)
+                m[e] = 0.f;
             for (int i = 0; i < tiles && ok; ++i)
-                for (int r = tid / NV; r < 64; r += int(blockDim.x) / NV)
-                    numbers.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
-            numbers.get(m);
-        }
-    }
-    if (!ok)
-        failed = 1;
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-#pragma unroll
-        for (int x = NV; x < 32; x *= 2)
-            m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], x));
-    if (lane < NV)
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            part[tid >> 5][lane * 8 + e] = m[e];
-    __syncthreads();
-    if (tid < S)
-    {
-        float v = part[0][tid];
-        for (int w = 1; w < int(blockDim.x) / 32; ++w)
-            v = fmaxf(v, part[w][tid]);
-        amax[tid] = v;
-    }
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (tid < S)
-    {
-        float v = 0.f;
-        for (uint32_t q = 0; q < ranks; ++q)
-        {
-            uint32_t addr;
-            float other;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&amax[tid])), "r"(q));
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(addr) : "memory");
-            v = fmaxf(v, other);
-        }
-        float const s = v * (1.f / float(1 << (BITS - 1)));
-        scale_s[tid] = s;
-        int const c = n0 + tid;
-        if (rank == 0 && c < a.N)
-        {
-            a.scales[c] = s;
-            if (a.scales_t)
             {
-                if (a.scales_dtype == W4_DTYPE_FP16)
-                    static_cast<__half*>(a.scales_t)[c] = __float2half_rn(s);
-                else
-                    static_cast<__nv_bfloat16*>(a.scales_t)[c] = __float2bfloat16_rn(s);
-            }
-        }
-    }
-    // (the barrier is also the CTA's; nobody leaves while its maxima are being read)
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (failed)
-        return;
-
-    // ---- quantise: a thread takes the E rows behind one output register of eight columns and leaves the eight
-    // finished registers in the place of the first two rows of its own input
-    int const c0 = n0 + cv * 8;
-    bool const inside = c0 < a.N; // n is a multiple of 32: a thread's eight columns are all inside or all outside
-    size_t const row_bytes = size_t(a.N) * BITS / 8;
-    constexpr uint32_t kSigned = BITS == 8 ? 0x80808080u : 0x88888888u;
-    // 16-byte place of registers 4h .. 4h + 3 of block b, register r4, column vector v
-    auto place = [&](int b, int r4, int v, int h)
-    {
-        uint8_t* row = slab + (b * GP + 2 * r4) * kStripBytes;
-        return reinterpret_cast<uint4*>(sizeof(W) == 4 ? row + v * 32 + h * 16 : row + h * kStripBytes + v * 16);
-    };
-    int const blocks = tiles * (64 / GP);
-    if (inside)
-    {
-        StripScales<W> sc;
-        sc.load(scale_s + cv * 8, has_nan != 0);
-#pragma unroll 1
-        for (int u = tid / NV; u < blocks * 4; u += int(blockDim.x) / NV)
-        {
-            int const b = u >> 2, r4 = u & 3;
-            uint8_t const* block = slab + (b * GP + 2 * r4) * kStripBytes;
-            uint32_t w[BITS / 4][E];
-#pragma unroll
-            for (int d = 0; d < E; ++d)
-            {
-                // the row behind position d of the register, as in emit_tile
-                int const p = BITS == 4 ? (d < 4 ? 2 * d : 2 * (d - 4) + 1) : (d == 1 ? 2 : (d == 2 ? 1 : d));
-                int const row = 8 * (p >> 1) + (p & 1);
-                float x[8];
-                strip_load8<W>(block + row * kStripBytes, cv, (tid / NV) & 1, x);
-                uint32_t word[BITS / 4];
-                quantize8<W, BITS>(x, sc, word);
-#pragma unroll
-                for (int h = 0; h < BITS / 4; ++h)
+                ok = mbar_wait(&full[i], phase);
+                for (int r = tid / NV; r < 64 && ok; r += int(blockDim.x) / NV)
                 {
-                    w[h][d] = word[h];
-                    if (a.unprocessed)
-                        *reinterpret_cast<uint32_t*>(a.unprocessed + (size_t(t0) * 64 + b * GP + 2 * r4 + row) * row_bytes
-                            + size_t(c0) * BITS / 8 + 4 * h)
-                            = word[h] ^ kSigned;
+                    float x[8];
+                    strip_load8<W>(slab + i * TILE_BYTES + r * kStripBytes, cv, (tid / NV) & 1, x);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        m[e] = fmaxf(m[e], fabsf(x[e]));
                 }
             }
-#pragma unroll
-            for (int h = 0; h < BITS / 4; ++h)
-                if constexpr (BITS == 4)
-                    transpose_nibbles(w[h]);
-                else
-                    transpose_bytes(w[h]);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *place(b, r4, cv, h) = make_uint4(w[4 * h / E][4 * h % E], w[4 * h / E][4 * h % E + 1], w[4 * h / E][4 * h % E + 2],
-                    w[4 * h / E][4 * h % E + 3]);
         }
-    }
-    __syncthreads();
-    // ---- store: a thread takes the four registers of a block of four columns; neighbouring blocks in one warp
-    // make whole 32-byte sectors
-    if (inside)
-    {
-        size_t const regs_per_irow = size_t(a.K / E) * IL;
-        for (int u = tid / NV; u < blocks * 2; u += int(blockDim.x) / NV)
+        else
         {
-            int const b = (u & 1) | ((u >> 2) << 1), h = (u >> 1) & 1; // (a 64-row tile has an even number of blocks)
-            uint4 r[4];
+            StripMax<W, true> pm;
+            pm.clear();
+            for (int i = 0; i < tiles && ok; ++i)
+            {
+                ok = mbar_wait(&full[i], phase);
+                if (!ok)
+                    break;
+#pragma unroll 2
+                for (int r = tid / NV; r < 64; r += int(blockDim.x) / NV)
+                    pm.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
+            }
+            pm.get(m);
+            bool nan = false;
 #pragma unroll
-            for (int r4 = 0; r4 < 4; ++r4)
-                r[r4] = *place(b, r4, cv, h);
-            int const col = c0 + 4 * h, k_tile = t0 + b / (64 / GP), vr = 4 * (b % (64 / GP));
-            uint32_t* dst = a.out + size_t(col / IL) * regs_per_irow + size_t(k_tile) * 32 + vr;
-            *reinterpret_cast<uint4*>(dst) = make_uint4(r[0].x, r[1].x, r[2].x, r[3].x);
-            *reinterpret_cast<uint4*>(dst + VT) = make_uint4(r[0].y, r[1].y, r[2].y, r[3].y);
-            dst += BITS == 4 ? 2 * VT : regs_per_irow; // int8: columns 2 and 3 are the next interleaved row
-            *reinterpret_cast<uint4*>(dst) = make_uint4(r[0].z, r[1].z, r[2].z, r[3].z);
-            *reinterpret_cast<uint4*>(dst + VT) = make_uint4(r[0].w, r[1].w, r[2].w, r[3].w);
+            for (int e = 0; e < 8; ++e)
+                nan |= m[e] != m[e];
+            if (nan)
+            {
+                // once more without them; the threads that quantise this CTA's rows divide
+                has_nan = 1;
+                StripMax<W, false> numbers;
+                numbers.clear();
+                for (int i = 0; i < tiles && ok; ++i)
+                    for (int r = tid / NV; r < 64; r += int(blockDim.x) / NV)
+                        numbers.add(reinterpret_cast<uint4 const*>(slab + i * TILE_BYTES + r * kStripBytes)[cv]);
+                numbers.get(m);
+            }
         }
+        if (!ok)
+            failed = 1;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+#pragma unroll
+            for (int x = NV; x < 32; x *= 2)
+                m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], x));
+        if (lane < NV)
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                part[tid >> 5][lane * 8 + e] = m[e];
+        __syncthreads();
+        if (tid < S)
+        {
+            float v = part[0][tid];
+            for (int w = 1; w < int(blockDim.x) / 32; ++w)
+                v = fmaxf(v, part[w][tid]);
+            amax[tid] = v;
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (tid < S)
+        {
+            float v = 0.f;
+            for (uint32_t q = 0; q < ranks; ++q)
+            {
+                uint32_t addr;
+                float other;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&amax[tid])), "r"(q));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(addr) : "memory");
+                v = fmaxf(v, other);
+            }
+            float const s = v * (1.f / float(1 << (BITS - 1)));
+            scale_s[tid] = s;
+            int const c = n0 + tid;
+            if (rank == 0 && c < a.N)
+            {
+                a.scales[c] = s;
+                if (a.scales_t)
+                {
+                    if (a.scales_dtype == W4_DTYPE_FP16)
+                        static_cast<__half*>(a.scales_t)[c] = __float2half_rn(s);
+                    else
+                        static_cast<__nv_bfloat16*>(a.scales_t)[c] = __float2bfloat16_rn(s);
+                }
+            }
+        }
+        // (the barrier is also the CTA's; nobody leaves while its maxima are being read)
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // (after a timeout the CTA stays for its cluster's barriers and does nothing more)
+        ok = failed == 0;
+        bool const number = has_nan == 0;
+        int const next = strip + num_clusters;
+
+        // ---- quantise: a thread takes the E rows behind one output register of eight columns and leaves the eight
+        // finished registers in the place of the first two rows of its own input
+        int const c0 = n0 + cv * 8;
+        bool const inside = c0 < a.N; // n is a multiple of 32: a thread's eight columns are all inside or all outside
+        size_t const row_bytes = size_t(a.N) * BITS / 8;
+        constexpr uint32_t kSigned = BITS == 8 ? 0x80808080u : 0x88888888u;
+        // 16-byte place of registers 4h .. 4h + 3 of block b, register r4, column vector v
+        auto place = [&](int b, int r4, int v, int h)
+        {
+            uint8_t* row = slab + (b * GP + 2 * r4) * kStripBytes;
+            return reinterpret_cast<uint4*>(sizeof(W) == 4 ? row + v * 32 + h * 16 : row + h * kStripBytes + v * 16);
+        };
+        // as many boxes at a time as give every thread its share
+        int const boxes = PERSISTENT ? max(1, int(blockDim.x) / NV / (4 * (64 / GP))) : max(1, tiles);
+        StripScales<W> sc;
+        sc.load(scale_s + cv * 8, !number);
+        for (int box0 = 0; box0 < tiles; box0 += boxes)
+        {
+            int const block0 = box0 * (64 / GP), block1 = min(box0 + boxes, tiles) * (64 / GP);
+            if (inside && ok)
+            {
+#pragma unroll 1
+                for (int u = block0 * 4 + tid / NV; u < block1 * 4; u += int(blockDim.x) / NV)
+                {
+                    int const b = u >> 2, r4 = u & 3;
+                    uint8_t const* block = slab + (b * GP + 2 * r4) * kStripBytes;
+                    uint32_t w[BITS / 4][E];
+#pragma unroll
+                    for (int d = 0; d < E; ++d)
+                    {
+                        // the row behind position d of the register, as in emit_tile
+                        int const p = BITS == 4 ? (d < 4 ? 2 * d : 2 * (d - 4) + 1) : (d == 1 ? 2 : (d == 2 ? 1 : d));
+                        int const row = 8 * (p >> 1) + (p & 1);
+                        float x[8];
+                        strip_load8<W>(block + row * kStripBytes, cv, (tid / NV) & 1, x);
+                        uint32_t word[BITS / 4];
+                        quantize8<W, BITS>(x, sc, word);
+#pragma unroll
+                        for (int h = 0; h < BITS / 4; ++h)
+                        {
+                            w[h][d] = word[h];
+                            if (a.unprocessed)
+                                *reinterpret_cast<uint32_t*>(a.unprocessed + (size_t(t0) * 64 + b * GP + 2 * r4 + row) * row_bytes
+                                    + size_t(c0) * BITS / 8 + 4 * h)
+                                    = word[h] ^ kSigned;
+                        }
+                    }
+#pragma unroll
+                    for (int h = 0; h < BITS / 4; ++h)
+                        if constexpr (BITS == 4)
+                            transpose_nibbles(w[h]);
+                        else
+                            transpose_bytes(w[h]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        *place(b, r4, cv, h) = make_uint4(w[4 * h / E][4 * h % E], w[4 * h / E][4 * h % E + 1], w[4 * h / E][4 * h % E + 2],
+                            w[4 * h / E][4 * h % E + 3]);
+                }
+            }
+            __syncthreads();
+            // ---- store: a thread takes the four registers of a block of four columns; neighbouring blocks in one warp
+            // make whole 32-byte sectors
+            if (inside && ok)
+            {
+                size_t const regs_per_irow = size_t(a.K / E) * IL;
+                for (int u = block0 * 2 + tid / NV; u < block1 * 2; u += int(blockDim.x) / NV)
+                {
+                    int const b = (u & 1) | ((u >> 2) << 1), h = (u >> 1) & 1; // (a 64-row tile has an even number of blocks)
+                    uint4 r[4];
+#pragma unroll
+                    for (int r4 = 0; r4 < 4; ++r4)
+                        r[r4] = *place(b, r4, cv, h);
+                    int const col = c0 + 4 * h, k_tile = t0 + b / (64 / GP), vr = 4 * (b % (64 / GP));
+                    uint32_t* dst = a.out + size_t(col / IL) * regs_per_irow + size_t(k_tile) * 32 + vr;
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(r[0].x, r[1].x, r[2].x, r[3].x);
+                    *reinterpret_cast<uint4*>(dst + VT) = make_uint4(r[0].y, r[1].y, r[2].y, r[3].y);
+                    dst += BITS == 4 ? 2 * VT : regs_per_irow; // int8: columns 2 and 3 are the next interleaved row
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(r[0].z, r[1].z, r[2].z, r[3].z);
+                    *reinterpret_cast<uint4*>(dst + VT) = make_uint4(r[0].w, r[1].w, r[2].w, r[3].w);
+                }
+            }
+            if (PERSISTENT && next * S < a.N)
+            {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // what was read and written here is behind the copies
+                __syncthreads();
+                if (tid == 0 && ok)
+                    for (int i = box0; i < min(box0 + boxes, tiles); ++i)
+                        fetch(next, i);
+            }
+        }
+        if (!PERSISTENT)
+            break;
+        if (tid == 0)
+            has_nan = 0; // (read before the last barrier, written next behind the one below)
+        __syncthreads();
     }
 }
 
@@ -830,7 +892,6 @@ int launch_strips(StripArgs a, W const* w, int cluster, cudaStream_t stream)
     int const units = a.tiles_cta * (64 / GP) * 4 * NV;
     int const threads = std::max(64, std::min(units, kMaxStripThreads)); // units: a multiple of 64
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned((a.N + S - 1) / S * cluster));
     cfg.blockDim = dim3(unsigned(threads));
     cfg.dynamicSmemBytes = size_t(a.tiles_cta) * 64 * kStripBytes;
     cfg.stream = stream;
@@ -842,6 +903,19 @@ int launch_strips(StripArgs a, W const* w, int cluster, cudaStream_t stream)
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
+    // Clusters that run side by side, asked of the runtime once per device, cluster size (1, 2, 4, 8, 16) and slab.
+    static std::atomic<int> resident[64][17][kMaxStripTiles + 1];
+    std::atomic<int>& r = resident[dev.device & 63][cluster][a.tiles_cta];
+    int most = r.load(std::memory_order_relaxed);
+    if (most <= 0)
+    {
+        cfg.gridDim = dim3(unsigned(cluster));
+        if (cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess || most <= 0)
+            return W4_ERR_CUDA;
+        r.store(most, std::memory_order_relaxed);
+    }
+    int const strips = (a.N + S - 1) / S;
+    cfg.gridDim = dim3(unsigned((strips < most || sizeof(W) == 4 ? strips : most) * cluster));
     return cudaLaunchKernelEx(&cfg, kernel, a, tm) == cudaSuccess ? W4_OK : W4_ERR_CUDA;
 }
 

@@ -1,0 +1,29 @@
+"""The one-pass device quantiser with several strips per cluster (needs a B200): byte for byte the host path."""
+import pytest
+import torch
+
+from tensorrt_llm_b200 import quantize
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("k,n,dtype", [
+    (64, 40032, torch.bfloat16),     # one box per strip, clusters of one CTA, a last strip of half its columns
+    (1024, 19264, torch.float16),    # two boxes per CTA
+    (2624, 12352, torch.bfloat16),   # CTAs with fewer boxes than the others, and with none
+    (4800, 9664, torch.bfloat16),    # half as wide strips
+    (1024, 12352, torch.float32),
+])
+def test_strips_one_after_another(k, n, dtype, bits):
+    n = n // 64 * 64 if bits == 4 else n
+    g = torch.Generator().manual_seed(k + n)
+    w = (torch.randn((k, n), generator=g) * 0.02).to(dtype)
+    w[:, 5] = 0                                  # a column without a scale
+    w[:, n - 3] *= 100                           # and large ones in the last strip
+    w[3, n // 2] = w[:, n // 2].abs().max() * 2  # exactly the largest: rounds up and is cut off
+    qt = torch.quint4x2 if bits == 4 else torch.int8
+    dev, dev_scales = quantize.symmetric_quantize_last_axis_of_batched_matrix_cuda(w.cuda(), qt)
+    host, host_scales = quantize.symmetric_quantize_last_axis_of_batched_matrix(w, qt)
+    assert torch.equal(dev.cpu().view(torch.int8).reshape(-1), host.view(torch.int8).reshape(-1))
+    assert torch.equal(dev_scales.cpu(), host_scales)
