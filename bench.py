@@ -682,8 +682,8 @@ def prep_point(pkg, device, peaks):
 
 
 def splitk_point(pkg, device):
-    """A tensor-core shape of two tiles: without a workspace its k splits share a cluster, with one there may be
-    more of them than a cluster holds. Graph-timed."""
+    """A tensor-core shape of two tiles: without a workspace its k splits share a cluster, with one the k range may be
+    cut into equal ranges. Graph-timed."""
     from tensorrt_llm_b200 import ops
     m, n, k = 64, 512, 14336
     w = torch.randint(0, 256, (k, n // 2), dtype=torch.uint8, device=device).view(torch.int8)

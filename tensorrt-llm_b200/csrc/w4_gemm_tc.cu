@@ -943,6 +943,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t const a_col = lane_ring + uint32_t(s) * kStageCols;
             // With SCALE_GROUP the halves of a step share their instructions: the roles' loops together do not fit the
             // instruction caches otherwise (2 % of a step; in the other modes 1 to 2 % the other way).
+            ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
+            if (!ok)
+                break;
+            tc_fence_after();
             constexpr int UNROLL = MODE == SCALE_GROUP ? 1 : 2;
 #pragma unroll UNROLL
             for (int h = 0; h < 2; ++h)
@@ -979,10 +983,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                     __syncwarp();
                     if (lane == 0)
                         arrive_local(w_empty0 + 8 * ws);
-                    ok = wait_bar<false>(empty0 + 8 * s, ph ^ 1, abort_flag);
-                    if (!ok)
-                        break;
-                    tc_fence_after();
                 }
                 tc_st32(a_col + 32 * h, v);
             }
