@@ -1618,7 +1618,7 @@ static double step_us(int bm, W4GemmParams const& p, int mode, double busy_pairs
     if (mode == tc::SCALE_RAW)
         conv = w8 && p.act_dtype == W4_DTYPE_BF16 ? 0.235 : w8 ? 0.22 : 0.2;
     else if (mode == tc::SCALE_GROUP)
-        conv = p.group_size == 64 ? 0.49 : w8 ? 0.385 : p.zeros ? 0.36 : 0.32;
+        conv = p.group_size == 64 ? 0.49 : w8 ? 0.42 : p.zeros ? 0.36 : 0.32;
     else
         conv = w8 && p.act_dtype == W4_DTYPE_BF16 ? 0.285 : 0.25;
     double const mma = bm * (0.57 / 256), memory = busy_pairs * tc::kPairN * 128 * p.weight_bits / 8 / 6.3e6;
@@ -1626,9 +1626,9 @@ static double step_us(int bm, W4GemmParams const& p, int mode, double busy_pairs
     return conv > memory ? conv : memory;
 }
 
-// The plan with the shortest estimated time. A launch costs 4 us (2.2 where it leaves half of the SMs
-// to the next one) plus the waves of its work items; an item's epilogue 0.3 us per 32 rows, of which the
-// double-buffered accumulators hide all but the last. Clusters add 1.2 us for the exchange of the partial tiles
+// The plan with the shortest estimated time. A launch costs 4 us (2.4 to 3 where it leaves half of the
+// SMs to the next one) plus the waves of its work items; an item's epilogue 0.3 us per 32 rows, of which the
+// double-buffered accumulators hide all but the last. Clusters add 1.7 us for the exchange of the partial tiles
 // (2.4 above 8 CTAs), equal ranges 3.5 us and 15 % of the steps: a part's way through memory, its flag, and the copies into the shared memory of
 // the pair that adds. So ranges pay where whole tiles would leave pairs idle for longer than that. Beyond 777 rows, and
 // in long runs at the power limit, the estimate is too low (14336 x 4096 at 4096 rows 228 us, measured 302 cool
@@ -1661,9 +1661,9 @@ static TcPlan search_plan(int const* rows, int experts, W4GemmParams const& p, i
                 continue; // an empty work item, too little in each, or more clusters than run side by side
             double const waves = double((tiles * s + pairs - 1) / pairs);
             double const busy = double(tiles * s) / waves;
-            double us = (2 * tiles * s <= pairs ? 2.2 : 4.0) + drain + waves * per * step_us(bm, p, mode, busy) + (waves - 1) * again;
+            double us = (2 * tiles * s <= pairs ? 2.2 + 0.006 * bm : 4.0) + drain + waves * per * step_us(bm, p, mode, busy) + (waves - 1) * again;
             if (s > 1)
-                us += (s > 4 ? 2.4 : 1.2) + 0.008 * bm;
+                us += (s > 4 ? 2.4 : 1.7) + 0.008 * bm;
             else if (!whole || us < whole)
                 whole = us;
             if (!best.bm || us < best.us)
